@@ -319,8 +319,6 @@ int ensure_background(j3g_context *c) {
   return J3G_OK;
 }
 
-constexpr int kTargetBlocks = 152 * 8;
-
 // Gridded node-component sums comps[nmeas][NC_COUNT] for the model d_model.
 int gridded_node_forward(j3g_context *c, const double *d_model) {
   const long long nn = c->nnodes();
@@ -330,22 +328,16 @@ int gridded_node_forward(j3g_context *c, const double *d_model) {
   for (int b = 0; b < nblock; ++b)
     J3G_LAUNCH(c, launch_rho_tilde(m, d_model + (size_t)b * c->ngrid(),
                                    ptr<double>(c->rhot) + (size_t)b * nn, c->stream));
-  int npb = 2048, spb = 4;
-  auto blocks = [&](int a, int b) {
-    return ((nn + a - 1) / a) * (long long)((c->nmeas + b - 1) / b);
-  };
-  while (npb > 256 && blocks(npb, spb) < kTargetBlocks) npb >>= 1;
-  while (spb > 1 && blocks(npb, spb) < kTargetBlocks) spb >>= 1;
-  // station blocks run over grid y: at most 65535 of them
-  spb = std::max(spb, (c->nmeas + 65534) / 65535);
-  const int nblk = (int)((nn + npb - 1) / npb);
+  const NodeForwardPlan p =
+      node_forward_plan(c->nx, c->ny, c->nz, c->nmeas, (1LL << 31) - 1);
+  const int nblk = p.nblk;
   const int ncomp = kind_ncomp(c->kind);
   J3G_TRY(ensure(c, c->partial, sizeof(double) * (size_t)nblk * c->nmeas * ncomp));
   J3G_TRY(ensure(c, c->comps, sizeof(double) * (size_t)c->nmeas * NC_COUNT));
   {
     TimedScope ts(c, J3G_TIMER_NODE_FORWARD);
     J3G_LAUNCH(c, launch_node_forward(c->kind, m, station_view(c), ptr<double>(c->rhot),
-                                      ptr<double>(c->partial), nblk, npb, spb, c->stream));
+                                      ptr<double>(c->partial), p, c->stream));
   }
   J3G_LAUNCH(c, launch_forward_reduce(c->kind, c->nmeas, nblk, ptr<double>(c->partial),
                                       mag_field(c), ptr<double>(c->comps), c->stream));
@@ -480,12 +472,9 @@ int adjoint_device(j3g_context *c, const double *d_model, const double *d_misfit
     J3G_LAUNCH(c, launch_comp_weights(c->kind, c->nmeas, ptr<double>(c->wraw), mag_field(c),
                                     ptr<double>(c->W), c->stream));
     const long long nn = c->nnodes();
-    const long long nodeblocks = (nn + 255) / 256;
-    long long want = (kTargetBlocks + nodeblocks - 1) / nodeblocks;
-    long long maxchunk = (c->nmeas + 15) / 16;
-    int nchunk = (int)std::max(1LL, std::min(want, maxchunk));
-    const int spc = (c->nmeas + nchunk - 1) / nchunk;
-    nchunk = (c->nmeas + spc - 1) / spc;
+    const NodeAdjointPlan plan = node_adjoint_plan(c->nx, c->ny, c->nz, nblock, c->nmeas);
+    const int spc = plan.spc;
+    int nchunk = plan.nchunk;
     // chunks of at most spc stations that never straddle a subset
     std::vector<int> starts, first_chunk;
     const int *d_starts = nullptr;
@@ -514,7 +503,7 @@ int adjoint_device(j3g_context *c, const double *d_model, const double *d_misfit
     J3G_TRY(ensure(c, c->G, sizeof(double) * (size_t)nblock * nn));
     if (nchunk > 0) {
       TimedScope ts(c, J3G_TIMER_NODE_ADJOINT);
-      J3G_LAUNCH(c, launch_node_adjoint(c->kind, m, s, ptr<double>(c->W), spc, nchunk, d_starts,
+      J3G_LAUNCH(c, launch_node_adjoint(c->kind, m, s, ptr<double>(c->W), plan, nchunk, d_starts,
                                         ptr<double>(c->Gpart), c->stream));
     }
     for (int k = 0; k < nsub; ++k) {

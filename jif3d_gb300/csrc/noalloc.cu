@@ -93,23 +93,8 @@ extern "C" int j3g_forward_noalloc(int kind, int nx, int ny, int nz, const doubl
   const long long per_block = (long long)nmeas * ncomp;
   if (left < per_block) return J3G_ERR_SCRATCH_LIMIT;
   const long long max_blocks = left / per_block;
-  int npb = 2048;
-  while ((nn + npb - 1) / npb > max_blocks) {
-    if (npb > (1 << 26)) return J3G_ERR_SCRATCH_LIMIT;
-    npb <<= 1;
-  }
-  int spb = 4;
-  auto blocks = [&](int a, int b) {
-    return ((nn + a - 1) / a) * (long long)((nmeas + b - 1) / b);
-  };
-  // smaller node blocks for parallelism, as long as their partials still fit
-  while (npb > 256 && blocks(npb, spb) < 152 * 8 &&
-         (nn + (npb >> 1) - 1) / (npb >> 1) <= max_blocks)
-    npb >>= 1;
-  while (spb > 1 && blocks(npb, spb) < 152 * 8) spb >>= 1;
-  // station blocks run over grid y: at most 65535 of them
-  spb = std::max(spb, (nmeas + 65534) / 65535);
-  const int nblk = (int)((nn + npb - 1) / npb);
+  const NodeForwardPlan plan = node_forward_plan(nx, ny, nz, nmeas, max_blocks);
+  if (plan.nblk > max_blocks) return J3G_ERR_SCRATCH_LIMIT;
 
   int device = 0;
   if (cudaGetDevice(&device) != cudaSuccess) return J3G_ERR_CUDA;
@@ -145,9 +130,9 @@ extern "C" int j3g_forward_noalloc(int kind, int nx, int ny, int nz, const doubl
   // clearing is needed: rho~ covers all nodes, the partials all (block,
   // station, component) triples and the sums all (station, component) pairs
   if (launch_rho_tilde(m, d_model, rho_t, st) != cudaSuccess) return J3G_ERR_CUDA;
-  if (launch_node_forward(kind, m, s, rho_t, partial, nblk, npb, spb, st) != cudaSuccess)
+  if (launch_node_forward(kind, m, s, rho_t, partial, plan, st) != cudaSuccess)
     return J3G_ERR_CUDA;
-  if (launch_forward_reduce(kind, nmeas, nblk, partial, mf, comps, st) != cudaSuccess)
+  if (launch_forward_reduce(kind, nmeas, plan.nblk, partial, mf, comps, st) != cudaSuccess)
     return J3G_ERR_CUDA;
   if (launch_assemble(kind, TR_NONE, 0.0, 0.0, 0.0, nmeas, comps, NC_COUNT, nullptr, 0, nullptr,
                       mf, nullptr, d_data, st) != cudaSuccess)

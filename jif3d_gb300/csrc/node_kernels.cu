@@ -1,0 +1,361 @@
+// node_kernels.cu -- the node-term forward and adjoint sums of the matrix-free
+// path (prism_kernels.h): every mesh node's corner terms, for all stations,
+// summed with the model differences or the weights.
+//
+// Work is split into node columns (fixed x and y): a thread takes one column
+// and walks its nodes, so that dx, dy and dx^2 + dy^2 are formed once per
+// column and station and the z offsets once per block and station (in shared
+// memory), instead of once per node.  The terms come from node_fixed.cuh.
+//
+// Measured (forward + adjoint of one model): joint g_z + FTG, 64 x 64 x 32
+// cells, 1024 stations 10.8 ms, from 77.1 ms with the terms on the FP64 pipe;
+// 96 x 96 x 48 cells, 2500 stations 85.5 ms from 612 ms; 12 x 10 x 6 cells, 16
+// stations 20 us from 41 us.  Bound by instruction issue: the integer (ALU)
+// and FP64 pipes are each 60 % busy, 128 registers leave four warps to a
+// scheduler.
+#include <algorithm>
+
+#include "node_fixed.cuh"
+#include "prism_kernels.h"
+
+namespace j3g {
+namespace {
+
+constexpr int kNodeThreads = 256;
+constexpr int kMaxColumn = 64;  // z offsets of a forward block held at a time
+constexpr int kAdjNodes = 8;    // nodes of a column per adjoint thread
+constexpr int kAdjStage = 16;   // stations staged at a time
+
+// The tables of node_fixed.cuh, copied to shared memory: random lookups there
+// cost a few bank conflicts, through L1 up to a cycle per lane.
+struct NodeTables {
+  uint64_t L[nodetab::kLogN];
+  uint64_t A[nodetab::kAtanN + 1];
+  uint32_t G[nodetab::kLogN];
+  __device__ __forceinline__ void load() {
+    for (int i = threadIdx.x; i < nodetab::kLogN; i += blockDim.x) {
+      L[i] = nodetab::kLogL[i];
+      G[i] = nodetab::kLogG[i];
+    }
+    for (int i = threadIdx.x; i <= nodetab::kAtanN; i += blockDim.x) A[i] = nodetab::kAtan[i];
+  }
+};
+
+struct ZOffset {
+  FxAxis a;
+  double d;
+};
+
+__device__ __forceinline__ ZOffset z_offset(double mz, double Z) {
+  ZOffset o;
+  o.d = sub(mz, Z);
+  o.a = fx_axis(o.d);
+  return o;
+}
+
+template <int MASK>
+__device__ __forceinline__ void node_eval(const FxColumn &c, double dx, double dy,
+                                          const ZOffset &z, const NodeTables &t, double *F) {
+  if (!fx_node<MASK>(c, z.a, dx, dy, z.d, t.G, t.L, t.A, F)) node_terms<MASK>(dx, dy, z.d, F);
+}
+
+// rho~(i,j,k) = sum_{a,b,c in {0,1}} (-1)^(a+b+c) rho(i-a, j-b, k-c), zero
+// outside, in the column order of the forward: [k][column].
+__global__ void __launch_bounds__(kNodeThreads)
+    k_rho_tilde(MeshView m, const double *__restrict__ rho, double *__restrict__ rt) {
+  const int ny1 = m.ny + 1, ncol = (m.nx + 1) * ny1;
+  const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= ncol * (m.nz + 1)) return;
+  const int k = n / ncol, col = n - k * ncol, i = col / ny1, j = col - i * ny1;
+  double v = 0.0;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int a = (q >> 2) & 1, b = (q >> 1) & 1, c = q & 1;
+    const int ci = i - a, cj = j - b, ck = k - c;
+    if (ci < 0 || cj < 0 || ck < 0 || ci >= m.nx || cj >= m.ny || ck >= m.nz) continue;
+    const double r = rho[((long long)ci * m.ny + cj) * m.nz + ck];
+    v = ((a + b + c) & 1) ? v - r : v + r;
+  }
+  rt[n] = v;
+}
+
+// Forward partial sums: block x covers cols columns and kper nodes of each,
+// block y spb stations; partial[x][station][component].
+template <int KIND>
+__global__ void __launch_bounds__(kNodeThreads, 2)
+    k_node_forward(MeshView m, StationView st, const double *__restrict__ rt,
+                   double *__restrict__ partial, int cols, int kper, int nkc, int spb) {
+  using T = KindTraits<KIND>;
+  constexpr int MASK = T::mask;
+  constexpr int NCMP = T::ncomp;
+  constexpr int NZ = T::twin ? 2 : 1;
+  __shared__ NodeTables tab;
+  __shared__ ZOffset zo[NZ][kMaxColumn];
+  __shared__ double red[NCMP][kNodeThreads];
+  const int ny1 = m.ny + 1, nz1 = m.nz + 1, ncol = (m.nx + 1) * ny1;
+  const long long nn = (long long)ncol * nz1;
+  const int cb = blockIdx.x / nkc, k0 = (blockIdx.x - cb * nkc) * kper;
+  const int k1 = min(nz1, k0 + kper);
+  const int c0 = cb * cols, c1 = min(ncol, c0 + cols);
+  const int s0 = blockIdx.y * spb, s1 = min(st.n, s0 + spb);
+  const int tid = threadIdx.x, nt = blockDim.x;
+  tab.load();
+  for (int s = s0; s < s1; ++s) {
+    const double mx = st.x[s], my = st.y[s], mz = st.z[s];
+    double acc[NCMP];
+#pragma unroll
+    for (int q = 0; q < NCMP; ++q) acc[q] = 0.0;
+    for (int kb = k0; kb < k1; kb += kMaxColumn) {
+      const int nk = min(kMaxColumn, k1 - kb);
+      __syncthreads();  // the offsets and sums of the last pass are read
+      for (int k = tid; k < nk; k += nt) {
+        const double Z = m.Z[kb + k];
+        zo[0][k] = z_offset(mz, Z);
+        // the second position of the vertical gradient, z_meas + 1 as the
+        // reference forms it (OMPMagneticGradImp.cpp:76-79)
+        if constexpr (T::twin) zo[NZ - 1][k] = z_offset(add(mz, 1.0), Z);
+      }
+      __syncthreads();
+      for (int col = c0 + tid; col < c1; col += nt) {
+        const int i = col / ny1, j = col - i * ny1;
+        const double dx = sub(mx, m.X[i]), dy = sub(my, m.Y[j]);
+        const FxColumn c = fx_column<MASK>(fx_axis(dx), fx_axis(dy), tab.G, tab.L);
+        const double *r = rt + (long long)kb * ncol + col;
+#pragma unroll 1
+        for (int k = 0; k < nk; ++k) {
+          double F[NZ][NC_COUNT];
+#pragma unroll
+          for (int p = 0; p < NZ; ++p) node_eval<MASK>(c, dx, dy, zo[p][k], tab, F[p]);
+          double w[T::nblock];
+#pragma unroll
+          for (int b = 0; b < T::nblock; ++b) w[b] = r[b * nn + (long long)k * ncol];
+#pragma unroll
+          for (int q = 0; q < NCMP; ++q)
+            acc[q] = fma(F[T::at(q)][T::comp(q)], w[T::block(q)], acc[q]);
+        }
+      }
+    }
+    // a warp per component sums the threads' values (13 FP64 additions a warp
+    // and component instead of a shuffle tree in every warp)
+#pragma unroll
+    for (int q = 0; q < NCMP; ++q) red[q][tid] = acc[q];
+    __syncthreads();
+    for (int q = tid >> 5; q < NCMP; q += nt >> 5) {
+      double v = 0.0;
+      for (int t = tid & 31; t < nt; t += 32) v += red[q][t];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+      if ((tid & 31) == 0) partial[((long long)blockIdx.x * st.n + s) * NCMP + q] = v;
+    }
+  }
+}
+
+// Adjoint: block x covers blockDim columns and kper nodes of each, block y a
+// chunk of stations, staged kAdjStage at a time; the sums of a thread's nodes
+// are in shared memory, so that the node loop need not be unrolled.
+template <int KIND>
+__global__ void __launch_bounds__(kNodeThreads, 2)
+    k_node_adjoint(MeshView m, StationView st, const double *__restrict__ W, int kper, int nkc,
+                   int spc, const int *__restrict__ chunk_start, double *__restrict__ Gpart) {
+  using T = KindTraits<KIND>;
+  constexpr int MASK = T::mask;
+  constexpr int NCMP = T::ncomp;
+  constexpr int NZ = T::twin ? 2 : 1;
+  // weights: node-component layout [nmeas][NC_COUNT], or [nmeas][ncomp] for
+  // the special kinds
+  constexpr int WLD = T::special ? NCMP : NC_COUNT;
+  __shared__ NodeTables tab;
+  __shared__ ZOffset zo[NZ][kAdjStage][kAdjNodes];
+  __shared__ double sx[kAdjStage], sy[kAdjStage], sw[kAdjStage][NCMP];
+  extern __shared__ double acc[];  // [nblock][kper][blockDim]
+  const int ny1 = m.ny + 1, nz1 = m.nz + 1, ncol = (m.nx + 1) * ny1;
+  const long long nn = (long long)ncol * nz1;
+  const int cb = blockIdx.x / nkc, k0 = (blockIdx.x - cb * nkc) * kper;
+  const int nk = min(kper, nz1 - k0);
+  const int tid = threadIdx.x, nt = blockDim.x;
+  const int c0 = cb * nt, col = c0 + tid;
+  const bool live = col < ncol;
+  const int i = live ? col / ny1 : 0, j = live ? col - i * ny1 : 0;
+  const double X = m.X[i], Y = m.Y[j];
+  // stations of this chunk: spc apiece, or the ranges of chunk_start (chunks
+  // that never straddle a station subset)
+  const int chunk = blockIdx.y;
+  const int s0 = chunk_start ? chunk_start[chunk] : chunk * spc;
+  const int s1 = chunk_start ? chunk_start[chunk + 1] : min(st.n, s0 + spc);
+  tab.load();
+  for (int k = 0; k < nk; ++k)
+#pragma unroll
+    for (int b = 0; b < T::nblock; ++b) acc[(b * kper + k) * nt + tid] = 0.0;
+  for (int base = s0; base < s1; base += kAdjStage) {
+    const int cnt = min(kAdjStage, s1 - base);
+    __syncthreads();
+    for (int t = tid; t < cnt; t += nt) {
+      sx[t] = st.x[base + t];
+      sy[t] = st.y[base + t];
+    }
+    for (int t = tid; t < cnt * NCMP; t += nt) {
+      const int s = t / NCMP, q = t - s * NCMP;
+      sw[s][q] = W[(long long)(base + s) * WLD + (T::special ? q : T::comp(q))];
+    }
+    for (int t = tid; t < cnt * nk; t += nt) {
+      const int s = t / nk, k = t - s * nk;
+      const double mz = st.z[base + s], Z = m.Z[k0 + k];
+      zo[0][s][k] = z_offset(mz, Z);
+      if constexpr (T::twin) zo[NZ - 1][s][k] = z_offset(add(mz, 1.0), Z);
+    }
+    __syncthreads();
+    if (!live) continue;
+#pragma unroll 1
+    for (int t = 0; t < cnt; ++t) {
+      const double dx = sub(sx[t], X), dy = sub(sy[t], Y);
+      const FxColumn c = fx_column<MASK>(fx_axis(dx), fx_axis(dy), tab.G, tab.L);
+#pragma unroll 1
+      for (int k = 0; k < nk; ++k) {
+        double F[NZ][NC_COUNT], v[T::nblock];
+#pragma unroll
+        for (int p = 0; p < NZ; ++p) node_eval<MASK>(c, dx, dy, zo[p][t][k], tab, F[p]);
+#pragma unroll
+        for (int b = 0; b < T::nblock; ++b) v[b] = acc[(b * kper + k) * nt + tid];
+#pragma unroll
+        for (int q = 0; q < NCMP; ++q)
+          v[T::block(q)] = fma(sw[t][q], F[T::at(q)][T::comp(q)], v[T::block(q)]);
+#pragma unroll
+        for (int b = 0; b < T::nblock; ++b) acc[(b * kper + k) * nt + tid] = v[b];
+      }
+    }
+  }
+  __syncthreads();
+  // out in node order: runs of nk nodes of consecutive columns
+  const int ncl = min(nt, ncol - c0);
+#pragma unroll
+  for (int b = 0; b < T::nblock; ++b) {
+    double *g = Gpart + ((long long)chunk * T::nblock + b) * nn;
+    for (int t = tid; t < ncl * nk; t += nt) {
+      const int c = t / nk, k = t - c * nk;
+      g[(long long)(c0 + c) * nz1 + k0 + k] = acc[(b * kper + k) * nt + c];
+    }
+  }
+}
+
+inline int cdiv(long long a, long long b) { return (int)((a + b - 1) / b); }
+
+int column_threads(int ncol) { return std::min(kNodeThreads, (ncol + 31) / 32 * 32); }
+
+// Blocks that fill the GPU a few times over (two resident per SM).
+constexpr long long kNodeBlocks = 152 * 2 * 3;
+
+}  // namespace
+
+NodeForwardPlan node_forward_plan(int nx, int ny, int nz, int nmeas, long long max_blocks) {
+  NodeForwardPlan p;
+  const int ncol = (nx + 1) * (ny + 1), nz1 = nz + 1;
+  p.threads = column_threads(ncol);
+  p.cols = p.threads;
+  p.nkc = 1;
+  p.kper = nz1;
+  p.spb = 8;
+  auto blocks = [&]() {
+    return (long long)cdiv(ncol, p.cols) * p.nkc * cdiv(nmeas, p.spb);
+  };
+  // few blocks: fewer stations each, then shorter pieces of the columns
+  while (p.spb > 1 && blocks() < kNodeBlocks) p.spb >>= 1;
+  while (p.kper > 1 && blocks() < kNodeBlocks) {
+    p.kper = (p.kper + 1) / 2;
+    p.nkc = cdiv(nz1, p.kper);
+  }
+  // short columns on many blocks: several columns per thread share a block's
+  // station setup and sums
+  while (p.cols < 8 * p.threads && (long long)p.kper * p.cols < 16LL * p.threads &&
+         blocks() >= 4 * kNodeBlocks)
+    p.cols += p.threads;
+  // within the caller's room for partial sums
+  if ((long long)cdiv(ncol, p.cols) * p.nkc > max_blocks) {
+    p.nkc = 1;
+    p.kper = nz1;
+    while ((long long)cdiv(ncol, p.cols) * p.nkc > max_blocks && p.cols < ncol)
+      p.cols += p.threads;
+  }
+  // station blocks run over grid y: at most 65535 of them
+  p.spb = std::max(p.spb, cdiv(nmeas, 65535));
+  p.nblk = cdiv(ncol, p.cols) * p.nkc;
+  return p;
+}
+
+template <int KIND>
+static cudaError_t adjoint_launch(dim3 grid, int threads, size_t smem, cudaStream_t st, const MeshView &m,
+                           const StationView &s, const double *W, const NodeAdjointPlan &p,
+                           const int *chunk_start, double *Gpart) {
+  if (smem > 16384) {  // three model blocks: beyond 48 KB with the tables, by opt-in
+    const cudaError_t e = cudaFuncSetAttribute(
+        k_node_adjoint<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  k_node_adjoint<KIND><<<grid, threads, smem, st>>>(m, s, W, p.kper, p.nkc, p.spc, chunk_start,
+                                                    Gpart);
+  return cudaGetLastError();
+}
+
+#define J3G_NODE_DISPATCH(kind, ...)                                             \
+  switch (kind) {                                                                 \
+    case KIND_SCALAR: { constexpr int K = KIND_SCALAR; __VA_ARGS__; } break;             \
+    case KIND_TENSOR: { constexpr int K = KIND_TENSOR; __VA_ARGS__; } break;             \
+    case KIND_MAGNETIC: { constexpr int K = KIND_MAGNETIC; __VA_ARGS__; } break;         \
+    case KIND_JOINT: { constexpr int K = KIND_JOINT; __VA_ARGS__; } break;               \
+    case KIND_MAG_GRADIENT: { constexpr int K = KIND_MAG_GRADIENT; __VA_ARGS__; } break; \
+    case KIND_MAGNETIZATION: { constexpr int K = KIND_MAGNETIZATION; __VA_ARGS__; } break; \
+    default: return cudaErrorInvalidValue;                                        \
+  }
+
+cudaError_t launch_rho_tilde(const MeshView &m, const double *rho, double *rho_t,
+                             cudaStream_t st) {
+  k_rho_tilde<<<cdiv(m.nnodes(), kNodeThreads), kNodeThreads, 0, st>>>(m, rho, rho_t);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_node_forward(int kind, const MeshView &m, const StationView &s,
+                                const double *rho_t, double *partial, const NodeForwardPlan &p,
+                                cudaStream_t st) {
+  const dim3 grid(p.nblk, cdiv(s.n, p.spb));
+  J3G_NODE_DISPATCH(kind, (k_node_forward<K><<<grid, p.threads, 0, st>>>(
+                              m, s, rho_t, partial, p.cols, p.kper, p.nkc, p.spb)));
+  return cudaGetLastError();
+}
+
+NodeAdjointPlan node_adjoint_plan(int nx, int ny, int nz, int nblock, int nmeas) {
+  NodeAdjointPlan p;
+  const int ncol = (nx + 1) * (ny + 1), nz1 = nz + 1;
+  p.threads = column_threads(ncol);
+  const int ncb = cdiv(ncol, p.threads);
+  p.nkc = cdiv(nz1, kAdjNodes);
+  p.kper = cdiv(nz1, p.nkc);
+  // Chunks of 64 stations: short enough that the rounding of a node's running
+  // sum stays small (a survey's chunks are added up afterwards), long enough
+  // that a block's setup does not count.  Surveys that leave SMs idle take
+  // shorter pieces of the columns, then shorter chunks.
+  p.spc = 64;
+  auto blocks = [&]() { return (long long)ncb * p.nkc * cdiv(nmeas, p.spc); };
+  while (p.spc > 16 && blocks() < kNodeBlocks / 2) p.spc >>= 1;
+  while (p.kper > 1 && blocks() < kNodeBlocks / 2) {
+    p.kper = (p.kper + 1) / 2;
+    p.nkc = cdiv(nz1, p.kper);
+  }
+  while (p.spc > 1 && blocks() < kNodeBlocks / 6) p.spc >>= 1;
+  // the chunks' sums within 512 MB
+  const long long room = std::max(1LL, (512LL << 20) / (8LL * nblock * ncol * nz1));
+  p.spc = std::max<long long>(p.spc, (nmeas + room - 1) / room);
+  p.nchunk = cdiv(nmeas, p.spc);
+  return p;
+}
+
+cudaError_t launch_node_adjoint(int kind, const MeshView &m, const StationView &s,
+                                const double *W, const NodeAdjointPlan &p, int nchunk,
+                                const int *chunk_start, double *Gpart, cudaStream_t st) {
+  const int ncb = cdiv((long long)(m.nx + 1) * (m.ny + 1), p.threads);
+  const dim3 grid(ncb * p.nkc, nchunk);
+  const size_t smem = sizeof(double) * (size_t)kind_nblock(kind) * p.kper * p.threads;
+  J3G_NODE_DISPATCH(kind, return adjoint_launch<K>(grid, p.threads, smem, st, m, s, W, p,
+                                                   chunk_start, Gpart));
+  return cudaGetLastError();
+}
+
+}  // namespace j3g

@@ -39,83 +39,6 @@ template <int KIND> struct Slots {
   static constexpr int off = (KIND == KIND_SCALAR || KIND == KIND_JOINT) ? 0 : 1;
 };
 
-// ---------------------------------------------------------------------------
-// rho~(i,j,k) = sum_{a,b,c in {0,1}} (-1)^(a+b+c) rho(i-a, j-b, k-c), zero outside.
-__global__ void k_rho_tilde(MeshView m, const double *__restrict__ rho, double *__restrict__ rt) {
-  const int ny1 = m.ny + 1, nz1 = m.nz + 1;
-  const int nn = (m.nx + 1) * ny1 * nz1;
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= nn) return;
-  int i, j, k;
-  decode_node(n, ny1, nz1, i, j, k);
-  double v = 0.0;
-#pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const int a = (q >> 2) & 1, b = (q >> 1) & 1, c = q & 1;
-    const int ci = i - a, cj = j - b, ck = k - c;
-    if (ci < 0 || cj < 0 || ck < 0 || ci >= m.nx || cj >= m.ny || ck >= m.nz) continue;
-    const double r = rho[((long long)ci * m.ny + cj) * m.nz + ck];
-    v = ((a + b + c) & 1) ? v - r : v + r;
-  }
-  rt[n] = v;
-}
-
-// ---------------------------------------------------------------------------
-// Forward partial sums.  Block (bx, by) covers nodes [bx*npb, (bx+1)*npb) and
-// stations [by*spb, (by+1)*spb); each thread walks npb/256 nodes per station
-// so the block reduction is amortised over several node evaluations.
-template <int KIND>
-__global__ void __launch_bounds__(kThreads)
-    k_node_forward(MeshView m, StationView st, const double *__restrict__ rt,
-                   double *__restrict__ partial, int npb, int spb) {
-  using T = KindTraits<KIND>;
-  constexpr int MASK = T::mask;
-  constexpr int NCMP = T::ncomp;
-  const int ny1 = m.ny + 1, nz1 = m.nz + 1;
-  const int nn = (m.nx + 1) * ny1 * nz1;
-  const int n0 = blockIdx.x * npb;
-  const int n1 = min(nn, n0 + npb);
-  const int s0 = blockIdx.y * spb;
-  const int s1 = min(st.n, s0 + spb);
-  __shared__ double red[kWarps][NCMP];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int s = s0; s < s1; ++s) {
-    const double mx = st.x[s], my = st.y[s], mz = st.z[s];
-    // the second position of the vertical gradient, z_meas + 1 as the
-    // reference forms it (OMPMagneticGradImp.cpp:76-79)
-    const double mz1 = T::twin ? add(mz, 1.0) : mz;
-    double acc[NCMP];
-#pragma unroll
-    for (int q = 0; q < NCMP; ++q) acc[q] = 0.0;
-    for (int n = n0 + threadIdx.x; n < n1; n += kThreads) {
-      int i, j, k;
-      decode_node(n, ny1, nz1, i, j, k);
-      double F[T::twin ? 2 : 1][NC_COUNT];
-      const double dx = sub(mx, m.X[i]), dy = sub(my, m.Y[j]);
-      node_terms<MASK>(dx, dy, sub(mz, m.Z[k]), F[0]);
-      if constexpr (T::twin) node_terms<MASK>(dx, dy, sub(mz1, m.Z[k]), F[T::twin ? 1 : 0]);
-      double w[T::nblock];
-#pragma unroll
-      for (int b = 0; b < T::nblock; ++b) w[b] = rt[(long long)b * nn + n];
-#pragma unroll
-      for (int q = 0; q < NCMP; ++q) acc[q] = fma(F[T::at(q)][T::comp(q)], w[T::block(q)], acc[q]);
-    }
-#pragma unroll
-    for (int q = 0; q < NCMP; ++q) {
-      const double v = warp_sum(acc[q]);
-      if (lane == 0) red[warp][q] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x < NCMP) {
-      double v = 0.0;
-#pragma unroll
-      for (int w = 0; w < kWarps; ++w) v += red[w][threadIdx.x];
-      partial[((long long)blockIdx.x * st.n + s) * NCMP + threadIdx.x] = v;
-    }
-    __syncthreads();
-  }
-}
-
 template <int KIND>
 __global__ void k_forward_reduce(int nmeas, int nblk, const double *__restrict__ partial,
                                  double *__restrict__ comps) {
@@ -343,68 +266,6 @@ __global__ void k_comp_weights(int kind, int nmeas, const double *__restrict__ w
   double u[NC_COUNT];
   comps_from_raw_weights(kind, w, mf, u);
   for (int c = 0; c < NC_COUNT; ++c) W[(long long)s * NC_COUNT + c] = u[c] * comp_scale(c);
-}
-
-// ---------------------------------------------------------------------------
-// Adjoint: one thread per node, stations of one chunk staged through shared
-// memory 64 at a time.
-constexpr int kStage = 64;
-
-template <int KIND>
-__global__ void __launch_bounds__(kThreads)
-    k_node_adjoint(MeshView m, StationView st, const double *__restrict__ W, int spc,
-                   const int *__restrict__ chunk_start, double *__restrict__ Gpart) {
-  using T = KindTraits<KIND>;
-  constexpr int MASK = T::mask;
-  constexpr int NCMP = T::ncomp;
-  // weights: node-component layout [nmeas][NC_COUNT], or [nmeas][ncomp] for
-  // the special kinds
-  constexpr int WLD = T::special ? NCMP : NC_COUNT;
-  const int ny1 = m.ny + 1, nz1 = m.nz + 1;
-  const int nn = (m.nx + 1) * ny1 * nz1;
-  const int n = blockIdx.x * kThreads + threadIdx.x;
-  const int chunk = blockIdx.y;
-  // stations of this chunk: spc apiece, or the ranges of chunk_start (chunks
-  // that never straddle a station subset)
-  const int s0 = chunk_start ? chunk_start[chunk] : chunk * spc;
-  const int s1 = chunk_start ? chunk_start[chunk + 1] : min(st.n, s0 + spc);
-  __shared__ double sx[kStage], sy[kStage], sz[kStage], sw[kStage][NCMP];
-  int i = 0, j = 0, k = 0;
-  if (n < nn) decode_node(n, ny1, nz1, i, j, k);
-  const double X = (n < nn) ? m.X[i] : 0.0, Y = (n < nn) ? m.Y[j] : 0.0,
-               Z = (n < nn) ? m.Z[k] : 0.0;
-  double acc[T::nblock];
-#pragma unroll
-  for (int b = 0; b < T::nblock; ++b) acc[b] = 0.0;
-  for (int base = s0; base < s1; base += kStage) {
-    const int cnt = min(kStage, s1 - base);
-    __syncthreads();
-    for (int t = threadIdx.x; t < cnt; t += kThreads) {
-      sx[t] = st.x[base + t];
-      sy[t] = st.y[base + t];
-      sz[t] = st.z[base + t];
-#pragma unroll
-      for (int q = 0; q < NCMP; ++q)
-        sw[t][q] = W[(long long)(base + t) * WLD + (T::special ? q : T::comp(q))];
-    }
-    __syncthreads();
-    if (n < nn) {
-      for (int t = 0; t < cnt; ++t) {
-        double F[T::twin ? 2 : 1][NC_COUNT];
-        const double dx = sub(sx[t], X), dy = sub(sy[t], Y);
-        node_terms<MASK>(dx, dy, sub(sz[t], Z), F[0]);
-        if constexpr (T::twin) node_terms<MASK>(dx, dy, sub(add(sz[t], 1.0), Z), F[T::twin ? 1 : 0]);
-#pragma unroll
-        for (int q = 0; q < NCMP; ++q)
-          acc[T::block(q)] = fma(sw[t][q], F[T::at(q)][T::comp(q)], acc[T::block(q)]);
-      }
-    }
-  }
-  if (n < nn) {
-#pragma unroll
-    for (int b = 0; b < T::nblock; ++b)
-      Gpart[((long long)chunk * T::nblock + b) * nn + n] = acc[b];
-  }
 }
 
 // G[n] = sum_c Gpart[c * stride + n] (stride = blocks x nodes per chunk).
@@ -693,21 +554,6 @@ inline int cdiv(long long a, long long b) { return (int)((a + b - 1) / b); }
 // the kinds with a node-component layout (node reduce)
 #define J3G_DISPATCH_ORDINARY(kind, CALL) J3G_DISPATCH4(kind, CALL, )
 
-cudaError_t launch_rho_tilde(const MeshView &m, const double *rho, double *rho_t,
-                             cudaStream_t st) {
-  const long long nn = m.nnodes();
-  k_rho_tilde<<<cdiv(nn, kThreads), kThreads, 0, st>>>(m, rho, rho_t);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_node_forward(int kind, const MeshView &m, const StationView &s,
-                                const double *rho_t, double *partial, int nblk, int npb, int spb,
-                                cudaStream_t st) {
-  dim3 grid(nblk, cdiv(s.n, spb));
-  J3G_DISPATCH(kind, (k_node_forward<K><<<grid, kThreads, 0, st>>>(m, s, rho_t, partial, npb, spb)));
-  return cudaGetLastError();
-}
-
 cudaError_t launch_forward_reduce(int kind, int nmeas, int nblk, const double *partial,
                                   const MagField &mf, double *comps, cudaStream_t st) {
   if (kind == KIND_MAG_GRADIENT) {
@@ -759,14 +605,6 @@ cudaError_t launch_backproject(int kind, int transform, double tbx, double tby, 
 cudaError_t launch_comp_weights(int kind, int nmeas, const double *w_raw, const MagField &mf,
                                 double *W, cudaStream_t st) {
   k_comp_weights<<<cdiv(nmeas, 128), 128, 0, st>>>(kind, nmeas, w_raw, mf, W);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_node_adjoint(int kind, const MeshView &m, const StationView &s,
-                                const double *W, int spc, int nchunk, const int *chunk_start,
-                                double *Gpart, cudaStream_t st) {
-  dim3 grid(cdiv(m.nnodes(), kThreads), nchunk);
-  J3G_DISPATCH(kind, (k_node_adjoint<K><<<grid, kThreads, 0, st>>>(m, s, W, spc, chunk_start, Gpart)));
   return cudaGetLastError();
 }
 

@@ -31,11 +31,19 @@ struct StationView {
 // block; magnetisation runs it once per block into rho_t + block * nnodes).
 cudaError_t launch_rho_tilde(const MeshView &m, const double *rho, double *rho_t,
                              cudaStream_t st);
+// Split of the forward's work: blocks of `cols` node columns and `kper` nodes
+// of each (nblk = column blocks x nkc pieces of the columns, at most
+// max_blocks of them where more columns per block can see to that), spb
+// stations per block.
+struct NodeForwardPlan {
+  int threads, cols, kper, nkc, spb, nblk;
+};
+NodeForwardPlan node_forward_plan(int nx, int ny, int nz, int nmeas, long long max_blocks);
 // partial: [nblk][nmeas][ncomp] virtual-component sums; rho_t holds one
 // nnodes block per model block of the kind.
 cudaError_t launch_node_forward(int kind, const MeshView &m, const StationView &s,
-                                const double *rho_t, double *partial, int nblk,
-                                int nodes_per_block, int stations_per_block, cudaStream_t st);
+                                const double *rho_t, double *partial, const NodeForwardPlan &p,
+                                cudaStream_t st);
 // comps: [nmeas][NC_COUNT] node-component sums (scaled), unused comps zero;
 // for the vertical gradient and magnetisation the raw rows [nmeas][raw].
 cudaError_t launch_forward_reduce(int kind, int nmeas, int nblk, const double *partial,
@@ -67,9 +75,13 @@ cudaError_t launch_comp_weights(int kind, int nmeas, const double *w_raw, const 
 // Gpart [nchunk][nblock][nnodes] = sum over the chunk's stations of
 // sum_q W_q * F_q, per model block.
 // chunk_start (device, nchunk + 1 values, may be null): explicit station
-// ranges of the chunks instead of stations_per_chunk apiece.
+// ranges of the chunks instead of spc apiece.
+struct NodeAdjointPlan {
+  int threads, kper, nkc, spc, nchunk;
+};
+NodeAdjointPlan node_adjoint_plan(int nx, int ny, int nz, int nblock, int nmeas);
 cudaError_t launch_node_adjoint(int kind, const MeshView &m, const StationView &s,
-                                const double *W, int stations_per_chunk, int nchunk,
+                                const double *W, const NodeAdjointPlan &p, int nchunk,
                                 const int *chunk_start, double *Gpart, cudaStream_t st);
 // grad[b * ngrid + cell] = 2 * sum_corners (-1)^shifts * sum_chunks
 // Gpart[chunk][b][node] for each model block b; G: nblock * nnodes scratch.

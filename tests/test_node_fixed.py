@@ -1,0 +1,154 @@
+"""The fixed-point node terms (csrc/node_fixed.cuh): on the host against long
+double, and the kernels built on them at the edges of their tiles against FP64
+sums with log(r + d) formed without cancellation (on deep columns the oracle's
+own rounding of r + d, d negative, is worth up to 7e-9 of the data).
+
+Host bounds, from the number formats: a logarithm at scale 2^57 carries a few
+units of truncation (2^-54) and the relative error 2^-56 of its argument,
+enlarged by r / (r + d) where a negative offset cancels; an angle 2^-56, and
+2^-48 of itself where it is small; each is rounded once to FP64.
+"""
+import os
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+
+from helpers import oracle_forward, relerr, small_survey
+from jif3d_gb300 import build as B, workloads as W
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+KINDS = [W.SCALAR, W.TENSOR, W.MAGNETIC, W.JOINT, W.MAG_GRADIENT, W.MAGNETIZATION]
+
+
+def test_terms_against_long_double(tmp_path):
+    cxx = shutil.which("g++")
+    assert cxx, "a host compiler is needed"
+    exe = str(tmp_path / "node_fixed_check")
+    src = os.path.join(HERE, "cpp", "node_fixed_check.cpp")
+    r = subprocess.run([cxx, "-O2", "-std=c++17", "-ffp-contract=off", "-I", B.CSRC, src, "-o", exe],
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    out = subprocess.run([exe], capture_output=True, text=True, timeout=600).stdout
+    rows = [line.split() for line in out.splitlines()]
+    assert len(rows) == 24
+    for name, which, n, left, *worst in rows:
+        # only the sets with cancelling, exactly zero or far-apart offsets leave any
+        assert int(left) <= {"1": 0.1, "4": 0.05, "5": 1.0, "2": 0.0}.get(which, 0.001) * int(n), \
+            (name, which, left)
+        assert all(float(w) <= 1.0 for w in worst), (name, which, worst)
+
+
+def _survey(kind, nx, ny, nz, nmeas, aligned):
+    s = small_survey(kind, nx=nx, ny=ny, nz=nz, nmeas=nmeas, seed=nx + 10 * ny + 100 * nz + kind,
+                     bg=False)
+    if kind == W.MAGNETIZATION:
+        rng = np.random.default_rng(nx)
+        s.model = rng.uniform(1, 11, 3 * s.ngrid)
+    if aligned:
+        # stations above columns, on node planes, and level with the mesh's top
+        n = s.stations.shape[0]
+        s.stations[:, 0] = s.coords(0)[np.arange(n) % (nx + 1)]
+        s.stations[::2, 1] = s.coords(1)[(np.arange(n) % (ny + 1))[::2]]
+    return s
+
+
+GRAV = 6.67428e-11
+
+
+def _prisms(s, st):
+    """Prism values of the seven components [stations][cells] (FP64)."""
+    d = [st[:, a].reshape(-1, 1, 1, 1) - s.coords(a).reshape([1] + [-1 if b == a else 1
+                                                                   for b in range(3)])
+         for a in range(3)]
+    x, y, z = d
+    xx, yy, zz = x * x, y * y, z * z
+    r = np.sqrt(xx + yy + zz)
+
+    def ln(u, rest):
+        with np.errstate(divide="ignore", invalid="ignore"):
+            return np.log(np.maximum(np.where(u < 0, rest / (r - u), u + r), 2.0 ** -52))
+    lx, ly = ln(x, yy + zz), ln(y, xx + zz)
+    F = {"gz": x * ly + y * lx + z * np.arctan2(z * r, x * y), "xx": np.arctan2(y * z, x * r),
+         "yy": np.arctan2(x * z, y * r), "zz": np.arctan2(x * y, z * r), "xy": ln(z, xx + yy),
+         "xz": ly, "yz": lx}
+    out = {}
+    for k, f in F.items():
+        for a in (1, 2, 3):
+            f = np.diff(f, axis=a)
+        out[k] = (GRAV if k in ("xx", "yy", "zz") else -GRAV) * f.reshape(f.shape[0], -1)
+    return out
+
+
+def _rows(s):
+    """Raw sensitivity rows [stations * raw][parameters]."""
+    def rows(st):
+        p = _prisms(s, st)
+        t = [p[k] for k in ("xx", "xy", "xz", "xy", "yy", "yz", "xz", "yz", "zz")]
+        b = (np.cos(s.inc) * np.cos(s.dec), np.cos(s.inc) * np.sin(s.dec), np.sin(s.inc))
+        if s.kind == W.SCALAR:
+            return [p["gz"]]
+        if s.kind == W.TENSOR:
+            return t
+        if s.kind == W.JOINT:
+            return [p["gz"]] + t
+        if s.kind == W.MAGNETIC:
+            f = s.fs / (4 * np.pi * GRAV)
+            return [f * sum(b[j] * t[3 * k + j] for j in range(3)) for k in range(3)]
+        if s.kind == W.MAGNETIZATION:
+            f = 1e9 * 4e-7 * np.pi / (4 * np.pi * GRAV)
+            return [f * np.concatenate([t[3 * k + j] for j in range(3)], axis=1) for k in range(3)]
+        f = s.fs * 1e-7 / GRAV
+        return [f * (b[0] * p["xz"] + b[1] * p["yz"] + b[2] * p["zz"])]
+    J = rows(s.stations)
+    if s.kind == W.MAG_GRADIENT:
+        J = [J[0] - rows(s.stations + [0.0, 0.0, 1.0])[0]]
+    return np.stack(J, axis=1).reshape(-1, J[0].shape[1])
+
+
+# columns (nx + 1)(ny + 1) around a warp and around a block, nodes per column
+# around the pieces of 8 and 64, stations around the stages of 16 and the
+# chunks of 64
+SHAPES = [(1, 1, 1, 1), (3, 7, 7, 15), (2, 10, 8, 16), (15, 15, 15, 17), (15, 16, 16, 64),
+          (4, 5, 63, 65), (6, 4, 64, 33), (5, 5, 130, 129)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("kind", KINDS)
+def test_kernels_at_tile_edges(ctx, kind, shape):
+    for aligned in (False, True):
+        s = _survey(kind, *shape, aligned)
+        W.setup_context(ctx, s)
+        J = _rows(s)
+        d = ctx.forward(s.model)
+        assert relerr(d, J @ s.model) <= 1e-10
+        misfit = np.random.default_rng(3).normal(size=d.size)
+        assert relerr(ctx.lqderivative(s.model, misfit), 2.0 * (misfit @ J)) <= 1e-10
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", [W.SCALAR, W.TENSOR, W.JOINT])
+def test_offsets_left_to_fp64(ctx, oracle_lib, kind):
+    """Stations level with the mesh's top on a node plane (two zero offsets), a
+    millimetre above an edge's line, and offsets beyond 2^40 m: the nodes that
+    the fixed-point terms leave out."""
+    s = _survey(kind, 6, 5, 4, 8, False)
+    s.stations[:, 2] = -20.0
+    s.stations[0] = [s.coords(0)[2] + 3.0, s.coords(1)[0] - 5.0, -1e-3]
+    s.stations[1] = [s.coords(0)[0] - 900.0, s.coords(1)[2], -1e-2]
+    s.stations[2] = [s.coords(0)[3], s.coords(1)[0] - 40.0, 0.0]
+    W.setup_context(ctx, s)
+    d, ref = ctx.forward(s.model), oracle_forward(oracle_lib, s)
+    assert np.array_equal(np.isnan(d), np.isnan(ref))  # g_z on an edge's line is 0 log 0
+    ok = ~np.isnan(ref)
+    # values against the sums without cancellation: r + d of the first two
+    # stations has no correct digits in the oracle's FP64
+    assert relerr(d[ok], (_rows(s) @ s.model)[ok]) <= 1e-10
+    far = s.subset([3])
+    far.stations = np.array([[3e12, 0.0, -1.0]])
+    W.setup_context(ctx, far)
+    # the far field's box terms are rounding in FP64 too: finite, and no larger
+    # than a few units of the node terms
+    assert np.all(np.isfinite(ctx.forward(far.model)))
