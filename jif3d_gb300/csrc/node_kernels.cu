@@ -8,11 +8,10 @@
 // memory), instead of once per node.  The terms come from node_fixed.cuh.
 //
 // Measured (forward + adjoint of one model): joint g_z + FTG, 64 x 64 x 32
-// cells, 1024 stations 10.8 ms, from 77.1 ms with the terms on the FP64 pipe;
-// 96 x 96 x 48 cells, 2500 stations 85.5 ms from 612 ms; 12 x 10 x 6 cells, 16
-// stations 20 us from 41 us.  Bound by instruction issue: the integer (ALU)
-// and FP64 pipes are each 60 % busy, 128 registers leave four warps to a
-// scheduler.
+// cells, 1024 stations 8.7 ms, from 77.1 ms with the terms on the FP64 pipe;
+// 12 x 10 x 6 cells, 16 stations 19 us from 41 us.  A joint node takes about
+// 750 instructions; the FP64, integer and multiply-add pipes are 50 to 70 %
+// busy each and the schedulers issue in 60 % of the cycles.
 #include <algorithm>
 
 #include "node_fixed.cuh"
@@ -21,26 +20,16 @@
 namespace j3g {
 namespace {
 
-constexpr int kNodeThreads = 256;
+// 128 threads at 96 registers: five blocks, 20 warps, to an SM (256 threads at
+// 128 registers: 16 warps, 1 to 7 % slower)
+constexpr int kNodeThreads = 128;
+constexpr int kNodeResident = 5;
 constexpr int kMaxColumn = 64;  // z offsets of a forward block held at a time
 constexpr int kAdjNodes = 8;    // nodes of a column per adjoint thread
 constexpr int kAdjStage = 16;   // stations staged at a time
 
-// The tables of node_fixed.cuh, copied to shared memory: random lookups there
-// cost a few bank conflicts, through L1 up to a cycle per lane.
-struct NodeTables {
-  uint64_t L[nodetab::kLogN];
-  uint64_t A[nodetab::kAtanN + 1];
-  uint32_t G[nodetab::kLogN];
-  __device__ __forceinline__ void load() {
-    for (int i = threadIdx.x; i < nodetab::kLogN; i += blockDim.x) {
-      L[i] = nodetab::kLogL[i];
-      G[i] = nodetab::kLogG[i];
-    }
-    for (int i = threadIdx.x; i <= nodetab::kAtanN; i += blockDim.x) A[i] = nodetab::kAtan[i];
-  }
-};
-
+// The tables of node_fixed.cuh are copied to shared memory: random lookups
+// there cost a few bank conflicts, through L1 up to a cycle per lane.
 struct ZOffset {
   FxAxis a;
   double d;
@@ -51,12 +40,6 @@ __device__ __forceinline__ ZOffset z_offset(double mz, double Z) {
   o.d = sub(mz, Z);
   o.a = fx_axis(o.d);
   return o;
-}
-
-template <int MASK>
-__device__ __forceinline__ void node_eval(const FxColumn &c, double dx, double dy,
-                                          const ZOffset &z, const NodeTables &t, double *F) {
-  if (!fx_node<MASK>(c, z.a, dx, dy, z.d, t.G, t.L, t.A, F)) node_terms<MASK>(dx, dy, z.d, F);
 }
 
 // rho~(i,j,k) = sum_{a,b,c in {0,1}} (-1)^(a+b+c) rho(i-a, j-b, k-c), zero
@@ -82,14 +65,16 @@ __global__ void __launch_bounds__(kNodeThreads)
 // Forward partial sums: block x covers cols columns and kper nodes of each,
 // block y spb stations; partial[x][station][component].
 template <int KIND>
-__global__ void __launch_bounds__(kNodeThreads, 2)
+__global__ void __launch_bounds__(kNodeThreads, kNodeResident)
     k_node_forward(MeshView m, StationView st, const double *__restrict__ rt,
                    double *__restrict__ partial, int cols, int kper, int nkc, int spb) {
   using T = KindTraits<KIND>;
   constexpr int MASK = T::mask;
   constexpr int NCMP = T::ncomp;
   constexpr int NZ = T::twin ? 2 : 1;
-  __shared__ NodeTables tab;
+  // component 0 is g_z: dx ln(dy + r) + dy ln(dx + r) + dz atan2(dz r, dx dy)
+  constexpr bool kGz = (MASK & (1 << NC_GZ)) != 0;
+  __shared__ FxTables tab;
   __shared__ ZOffset zo[NZ][kMaxColumn];
   __shared__ double red[NCMP][kNodeThreads];
   const int ny1 = m.ny + 1, nz1 = m.nz + 1, ncol = (m.nx + 1) * ny1;
@@ -99,7 +84,7 @@ __global__ void __launch_bounds__(kNodeThreads, 2)
   const int c0 = cb * cols, c1 = min(ncol, c0 + cols);
   const int s0 = blockIdx.y * spb, s1 = min(st.n, s0 + spb);
   const int tid = threadIdx.x, nt = blockDim.x;
-  tab.load();
+  tab.set(tid, nt);
   for (int s = s0; s < s1; ++s) {
     const double mx = st.x[s], my = st.y[s], mz = st.z[s];
     double acc[NCMP];
@@ -119,19 +104,42 @@ __global__ void __launch_bounds__(kNodeThreads, 2)
       for (int col = c0 + tid; col < c1; col += nt) {
         const int i = col / ny1, j = col - i * ny1;
         const double dx = sub(mx, m.X[i]), dy = sub(my, m.Y[j]);
-        const FxColumn c = fx_column<MASK>(fx_axis(dx), fx_axis(dy), tab.G, tab.L);
+        const FxColumn c = fx_column<MASK>(fx_axis(dx), fx_axis(dy), tab);
         const double *r = rt + (long long)kb * ncol + col;
+        double slx = 0.0, sly = 0.0;  // this column's sums of ln(dx + r), ln(dy + r)
 #pragma unroll 1
         for (int k = 0; k < nk; ++k) {
-          double F[NZ][NC_COUNT];
-#pragma unroll
-          for (int p = 0; p < NZ; ++p) node_eval<MASK>(c, dx, dy, zo[p][k], tab, F[p]);
           double w[T::nblock];
 #pragma unroll
           for (int b = 0; b < T::nblock; ++b) w[b] = r[b * nn + (long long)k * ncol];
 #pragma unroll
-          for (int q = 0; q < NCMP; ++q)
-            acc[q] = fma(F[T::at(q)][T::comp(q)], w[T::block(q)], acc[q]);
+          for (int p = 0; p < NZ; ++p) {
+            const ZOffset &z = zo[p][k];
+            double F[NC_COUNT];
+            if (fx_node<MASK>(c, z.a, tab, F)) {
+              if constexpr (kGz) {
+                slx = fma(F[NC_YZ], w[0], slx);
+                sly = fma(F[NC_XZ], w[0], sly);
+                F[NC_GZ] *= z.d;
+              }
+#pragma unroll
+              for (int q = 0; q < NCMP; ++q)
+                if (T::at(q) == p && !(kGz && (T::comp(q) == NC_XZ || T::comp(q) == NC_YZ)))
+                  acc[q] = fma(F[T::comp(q)], w[T::block(q)], acc[q]);
+            } else {
+              node_terms<MASK>(dx, dy, z.d, F);
+#pragma unroll
+              for (int q = 0; q < NCMP; ++q)
+                if (T::at(q) == p) acc[q] = fma(F[T::comp(q)], w[T::block(q)], acc[q]);
+            }
+          }
+        }
+        if constexpr (kGz) {  // dx and dy belong to the column
+          acc[0] = fma(dx, sly, fma(dy, slx, acc[0]));
+          if constexpr (NCMP > 1) {
+            acc[NC_XZ] += sly;
+            acc[NC_YZ] += slx;
+          }
         }
       }
     }
@@ -154,7 +162,7 @@ __global__ void __launch_bounds__(kNodeThreads, 2)
 // chunk of stations, staged kAdjStage at a time; the sums of a thread's nodes
 // are in shared memory, so that the node loop need not be unrolled.
 template <int KIND>
-__global__ void __launch_bounds__(kNodeThreads, 2)
+__global__ void __launch_bounds__(kNodeThreads, kNodeResident)
     k_node_adjoint(MeshView m, StationView st, const double *__restrict__ W, int kper, int nkc,
                    int spc, const int *__restrict__ chunk_start, double *__restrict__ Gpart) {
   using T = KindTraits<KIND>;
@@ -164,9 +172,16 @@ __global__ void __launch_bounds__(kNodeThreads, 2)
   // weights: node-component layout [nmeas][NC_COUNT], or [nmeas][ncomp] for
   // the special kinds
   constexpr int WLD = T::special ? NCMP : NC_COUNT;
-  __shared__ NodeTables tab;
+  __shared__ FxTables tab;
   __shared__ ZOffset zo[NZ][kAdjStage][kAdjNodes];
   __shared__ double sx[kAdjStage], sy[kAdjStage], sw[kAdjStage][NCMP];
+  // g_z weight times dz (component 0 is g_z, see the forward)
+  constexpr bool kGz = (MASK & (1 << NC_GZ)) != 0;
+  __shared__ double swz[kGz ? kAdjStage : 1][kAdjNodes];
+  // g_z alone: a station's three products are added up before they meet the
+  // running sum, so that it is rounded once per station (the other kinds'
+  // rounding is less than that of the terms they had in FP64)
+  constexpr bool kSumFirst = KIND == KIND_SCALAR;
   extern __shared__ double acc[];  // [nblock][kper][blockDim]
   const int ny1 = m.ny + 1, nz1 = m.nz + 1, ncol = (m.nx + 1) * ny1;
   const long long nn = (long long)ncol * nz1;
@@ -182,7 +197,7 @@ __global__ void __launch_bounds__(kNodeThreads, 2)
   const int chunk = blockIdx.y;
   const int s0 = chunk_start ? chunk_start[chunk] : chunk * spc;
   const int s1 = chunk_start ? chunk_start[chunk + 1] : min(st.n, s0 + spc);
-  tab.load();
+  tab.set(tid, nt);
   for (int k = 0; k < nk; ++k)
 #pragma unroll
     for (int b = 0; b < T::nblock; ++b) acc[(b * kper + k) * nt + tid] = 0.0;
@@ -200,7 +215,9 @@ __global__ void __launch_bounds__(kNodeThreads, 2)
     for (int t = tid; t < cnt * nk; t += nt) {
       const int s = t / nk, k = t - s * nk;
       const double mz = st.z[base + s], Z = m.Z[k0 + k];
-      zo[0][s][k] = z_offset(mz, Z);
+      const ZOffset o = z_offset(mz, Z);
+      zo[0][s][k] = o;
+      if constexpr (kGz) swz[s][k] = W[(long long)(base + s) * WLD + NC_GZ] * o.d;
       if constexpr (T::twin) zo[NZ - 1][s][k] = z_offset(add(mz, 1.0), Z);
     }
     __syncthreads();
@@ -208,19 +225,44 @@ __global__ void __launch_bounds__(kNodeThreads, 2)
 #pragma unroll 1
     for (int t = 0; t < cnt; ++t) {
       const double dx = sub(sx[t], X), dy = sub(sy[t], Y);
-      const FxColumn c = fx_column<MASK>(fx_axis(dx), fx_axis(dy), tab.G, tab.L);
+      const FxColumn c = fx_column<MASK>(fx_axis(dx), fx_axis(dy), tab);
+      // g_z's logarithms go with those of Uxz and Uyz
+      double wlx = 0.0, wly = 0.0;
+      if constexpr (kGz) {
+        wlx = sw[t][0] * dy;
+        wly = sw[t][0] * dx;
+        if constexpr (NCMP > 1) {
+          wlx += sw[t][NC_YZ];
+          wly += sw[t][NC_XZ];
+        }
+      }
 #pragma unroll 1
       for (int k = 0; k < nk; ++k) {
-        double F[NZ][NC_COUNT], v[T::nblock];
+        double v[T::nblock];
 #pragma unroll
-        for (int p = 0; p < NZ; ++p) node_eval<MASK>(c, dx, dy, zo[p][t][k], tab, F[p]);
+        for (int b = 0; b < T::nblock; ++b) v[b] = kSumFirst ? 0.0 : acc[(b * kper + k) * nt + tid];
 #pragma unroll
-        for (int b = 0; b < T::nblock; ++b) v[b] = acc[(b * kper + k) * nt + tid];
+        for (int p = 0; p < NZ; ++p) {
+          const ZOffset &z = zo[p][t][k];
+          double F[NC_COUNT];
+          if (fx_node<MASK>(c, z.a, tab, F)) {
+            if constexpr (kGz)
+              v[0] = fma(swz[t][k], F[NC_GZ], fma(wly, F[NC_XZ], fma(wlx, F[NC_YZ], v[0])));
 #pragma unroll
-        for (int q = 0; q < NCMP; ++q)
-          v[T::block(q)] = fma(sw[t][q], F[T::at(q)][T::comp(q)], v[T::block(q)]);
+            for (int q = 0; q < NCMP; ++q)
+              if (T::at(q) == p && !(kGz && (q == 0 || T::comp(q) == NC_XZ || T::comp(q) == NC_YZ)))
+                v[T::block(q)] = fma(sw[t][q], F[T::comp(q)], v[T::block(q)]);
+          } else {
+            node_terms<MASK>(dx, dy, z.d, F);
 #pragma unroll
-        for (int b = 0; b < T::nblock; ++b) acc[(b * kper + k) * nt + tid] = v[b];
+            for (int q = 0; q < NCMP; ++q)
+              if (T::at(q) == p)
+                v[T::block(q)] = fma(sw[t][q], F[T::comp(q)], v[T::block(q)]);
+          }
+        }
+#pragma unroll
+        for (int b = 0; b < T::nblock; ++b)
+          acc[(b * kper + k) * nt + tid] = kSumFirst ? acc[(b * kper + k) * nt + tid] + v[b] : v[b];
       }
     }
   }
@@ -241,8 +283,8 @@ inline int cdiv(long long a, long long b) { return (int)((a + b - 1) / b); }
 
 int column_threads(int ncol) { return std::min(kNodeThreads, (ncol + 31) / 32 * 32); }
 
-// Blocks that fill the GPU a few times over (two resident per SM).
-constexpr long long kNodeBlocks = 152 * 2 * 3;
+// Blocks that fill the GPU a few times over.
+constexpr long long kNodeBlocks = 152 * kNodeResident * 3;
 
 }  // namespace
 
