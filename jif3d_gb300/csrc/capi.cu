@@ -70,7 +70,7 @@ struct j3g_context {
   long long st_rows = 0;       // nmeas * stored rows per station
   long long st_ld = 0;         // cells padded to a multiple of 64
   long long st_ldT = 0;        // rows padded to a multiple of 64 (transposed copy)
-  DevBuf J32, Jhi, Jlo, JThi, JTlo, rowscale, Jrowsum;
+  DevBuf J32, Jhi, Jlo, JThi, JTlo, rowscale, Jrowsum, rowmax;
   DevBuf x32, sums, part, Bhi, Blo, P, wst, wrawb, rawb, gerr, mscale, mmean, swork, sexp;
 
   // tensor-core product plans (j3g_set_autotune): key direction, rows, padded
@@ -347,7 +347,7 @@ int gridded_node_forward(j3g_context *c, const double *d_model) {
 // Station chunk for row generation, bounded by ~1 GiB of row scratch.
 int row_chunk(j3g_context *c, long long ld) {
   const long long per = (long long)c->raw() * ld * 8 +
-                        (c->node_exact ? (long long)kind_ncomp(c->kind) * c->nnodes() * 8 : 0);
+                        (c->node_exact ? (long long)node_terms_stored(c->kind) * c->nnodes() * 8 : 0);
   long long ch = (1LL << 30) / (per > 0 ? per : 1);
   if (ch < 1) ch = 1;
   if (ch > c->nmeas) ch = c->nmeas;
@@ -366,7 +366,7 @@ int gridded_rows_forward(j3g_context *c, const double *d_model, double *h_sens) 
   const int chunk = row_chunk(c, ld);
   J3G_TRY(ensure(c, c->rows, sizeof(double) * (size_t)chunk * raw * ld));
   if (c->node_exact)
-    J3G_TRY(ensure(c, c->F, sizeof(double) * (size_t)chunk * kind_ncomp(c->kind) * c->nnodes()));
+    J3G_TRY(ensure(c, c->F, 8 * (size_t)chunk * node_terms_stored(c->kind) * c->nnodes()));
   J3G_TRY(ensure(c, c->rowsum, sizeof(double) * (size_t)c->nmeas * raw));
   MeshView m = mesh_view(c);
   StationView s = station_view(c);
@@ -374,9 +374,14 @@ int gridded_rows_forward(j3g_context *c, const double *d_model, double *h_sens) 
   for (int s0 = 0; s0 < c->nmeas; s0 += chunk) {
     const int ns = std::min(chunk, c->nmeas - s0);
     if (ngrid > 0) {
-      J3G_LAUNCH(c, launch_sens_rows(c->kind, c->node_exact, m, s, s0, ns, mf, ptr<double>(c->F),
-                                   ptr<double>(c->rows), ld, c->stream));
-      if (c->node_exact) ++c->launches;  // node terms + cell combine
+      if (c->node_exact) {
+        J3G_LAUNCH(c, launch_node_rows(c->kind, m, s, s0, ns, mf, ptr<double>(c->F),
+                                       ptr<double>(c->rows), ld, c->stream));
+        ++c->launches;  // node terms + cell rows
+      } else {
+        J3G_LAUNCH(c, launch_direct_rows(c->kind, m, s, s0, ns, mf, ptr<double>(c->rows), ld,
+                                         c->stream));
+      }
       J3G_LAUNCH(c, launch_rows_dot(raw, ns, ncolg, ptr<double>(c->rows), ld, d_model,
                                   ptr<double>(c->rowsum) + (size_t)s0 * raw, c->stream));
     } else {
@@ -524,8 +529,8 @@ int adjoint_device(j3g_context *c, const double *d_model, const double *d_misfit
       J3G_CUDA(c, cudaMemsetAsync(gk, 0, sizeof(double) * (size_t)ncolg, c->stream));
       for (int s0 = off[k]; s0 < off[k + 1]; s0 += chunk) {
         const int ns = std::min(chunk, off[k + 1] - s0);
-        J3G_LAUNCH(c, launch_sens_rows(c->kind, false, m, s, s0, ns, mf, nullptr,
-                                     ptr<double>(c->rows), ncolg, c->stream));
+        J3G_LAUNCH(c, launch_direct_rows(c->kind, m, s, s0, ns, mf, ptr<double>(c->rows), ncolg,
+                                         c->stream));
         J3G_LAUNCH(c, launch_rows_tdot(ns * raw, ncolg, ptr<double>(c->rows), ncolg,
                                      ptr<double>(c->wraw) + (size_t)s0 * raw, gk, c->stream));
       }
@@ -556,21 +561,21 @@ void free_buf(DevBuf &b) {
   b.cap = 0;
 }
 
+void drop_memory(j3g_context *c) {
+  for (DevBuf *b : {&c->J32, &c->Jhi, &c->Jlo, &c->JThi, &c->JTlo, &c->rowscale, &c->Jrowsum,
+                    &c->rowmax})
+    free_buf(*b);
+}
+
 void drop_stored(j3g_context *c) {
   if (!c || c->storage == 0) return;
   cudaStreamSynchronize(c->stream);
-  free_buf(c->J32);
-  free_buf(c->Jhi);
-  free_buf(c->Jlo);
-  free_buf(c->JThi);
-  free_buf(c->JTlo);
-  free_buf(c->rowscale);
-  free_buf(c->Jrowsum);
+  drop_memory(c);
   c->storage = 0;
 }
 
 long long round64(long long v) { return (v + 63) / 64 * 64; }
-int nstored(const j3g_context *c) { return stored_rows_per_station(c->kind); }
+int nstored(const j3g_context *c) { return stored_rows(c->kind); }
 
 int build_stored(j3g_context *c, int storage) {
   J3G_TRY(check_ready(c));
@@ -580,66 +585,74 @@ int build_stored(j3g_context *c, int storage) {
     return fail(c, J3G_ERR_UNSUPPORTED,
                 "device sensitivity needs corner coordinates that are running sums of the sizes");
   if (c->ngrid() == 0 || c->nmeas == 0) return fail(c, J3G_ERR_ARG, "empty mesh or survey");
-  drop_stored(c);
+  // a matrix that is rebuilt keeps its memory where it fits
+  if (c->storage != 0) J3G_CUDA(c, cudaStreamSynchronize(c->stream));
+  c->storage = 0;
+  const bool pair = storage == J3G_STORE_F16X2;
+  for (DevBuf *b : {&c->Jhi, &c->Jlo, &c->JThi, &c->JTlo})
+    if (!pair) free_buf(*b);
+  if (pair) free_buf(c->J32);
   J3G_TRY(ensure_background(c));
   const long long K = c->ngrid_cols(), ldK = round64(K);
   const int NS = nstored(c);
   const long long R = (long long)c->nmeas * NS, ldR = round64(R);
-  const size_t need = storage == J3G_STORE_FP32
-                          ? (size_t)R * ldK * 4
-                          : (size_t)(tiled_rows(R) * ldK + tiled_rows(K) * ldR) * 4;
-  size_t fr = 0, tot = 0;
+  const size_t bj = 2 * (size_t)tiled_rows(R) * ldK, bjt = 2 * (size_t)tiled_rows(K) * ldR;
+  const size_t b32 = sizeof(float) * (size_t)R * ldK;
+  size_t fr = 0, tot = 0, held = 0, need = pair ? 2 * (bj + bjt) : b32;
   J3G_CUDA(c, cudaMemGetInfo(&fr, &tot));
-  if (need + (size_t)(1ull << 31) > fr)
+  for (const DevBuf *b : {&c->J32, &c->Jhi, &c->Jlo, &c->JThi, &c->JTlo}) held += b->cap;
+  if (need + (size_t)(1ull << 31) > fr + held) {
+    drop_memory(c);
     return fail(c, J3G_ERR_NOMEM, "sensitivity of " + std::to_string(need) + " bytes does not fit");
+  }
   c->st_rows = R;
   c->st_ld = ldK;
   c->st_ldT = ldR;
-  // station chunks bounded by ~1 GiB of FP64 rows + node scratch
-  const long long per = (long long)NS * K * 8 + (long long)kind_ncomp(c->kind) * c->nnodes() * 8;
-  int chunk = (int)std::max(1LL, std::min<long long>(c->nmeas, (1LL << 30) / per));
-  chunk = std::min(chunk, 65535);
-  J3G_TRY(ensure(c, c->F, sizeof(double) * (size_t)chunk * kind_ncomp(c->kind) * c->nnodes()));
+  // station chunks bounded by ~1 GiB of node terms and FP64 rows, in eights so
+  // that the transpose is written in whole 16-byte pieces
+  const long long per = 8 * ((pair ? (long long)NS * K : 0) +
+                             (long long)node_terms_stored(c->kind) * c->nnodes());
+  long long chunk = std::max(1LL, (1LL << 30) / per);
+  if (chunk > 8) chunk = chunk / 8 * 8;
+  chunk = std::min<long long>({chunk, c->nmeas, 65535});
+  J3G_TRY(ensure(c, c->F, 8 * (size_t)chunk * node_terms_stored(c->kind) * c->nnodes()));
   MeshView m = mesh_view(c);
   StationView s = station_view(c);
   const MagField mf = mag_field(c);
-  if (storage == J3G_STORE_FP32) {
-    J3G_TRY(ensure(c, c->J32, sizeof(float) * (size_t)R * ldK));
-    J3G_CUDA(c, cudaMemsetAsync(c->J32.p, 0, sizeof(float) * (size_t)R * ldK, c->stream));
-    for (int s0 = 0; s0 < c->nmeas; s0 += chunk) {
-      const int ns = std::min(chunk, c->nmeas - s0);
-      J3G_LAUNCH(c, launch_stored_rows(c->kind, m, s, s0, ns, mf, ptr<double>(c->F), nullptr,
-                                       ptr<float>(c->J32) + (size_t)s0 * NS * ldK, ldK,
-                                       c->stream));
+  if (!pair) {
+    J3G_TRY(ensure(c, c->J32, b32));
+    if (ldK > K)  // padding columns
+      J3G_CUDA(c, cudaMemset2DAsync(ptr<float>(c->J32) + K, sizeof(float) * ldK, 0,
+                                    sizeof(float) * (ldK - K), R, c->stream));
+    for (int s0 = 0; s0 < c->nmeas; s0 += (int)chunk) {
+      const int ns = std::min((int)chunk, c->nmeas - s0);
+      J3G_LAUNCH(c, launch_stored_rows32(c->kind, m, s, s0, ns, mf, ptr<double>(c->F),
+                                         ptr<float>(c->J32) + (size_t)s0 * NS * ldK, ldK,
+                                         c->stream));
       ++c->launches;
     }
   } else {
-    // tiled layout; the padding rows of the last row block stay zero
-    const size_t bj = 2 * (size_t)tiled_rows(R) * ldK, bjt = 2 * (size_t)tiled_rows(K) * ldR;
     J3G_TRY(ensure(c, c->Jhi, bj));
     J3G_TRY(ensure(c, c->Jlo, bj));
     J3G_TRY(ensure(c, c->JThi, bjt));
     J3G_TRY(ensure(c, c->JTlo, bjt));
-    J3G_CUDA(c, cudaMemsetAsync(c->Jhi.p, 0, bj, c->stream));
-    J3G_CUDA(c, cudaMemsetAsync(c->Jlo.p, 0, bj, c->stream));
-    J3G_CUDA(c, cudaMemsetAsync(c->JThi.p, 0, bjt, c->stream));
-    J3G_CUDA(c, cudaMemsetAsync(c->JTlo.p, 0, bjt, c->stream));
     J3G_TRY(ensure(c, c->rowscale, sizeof(float) * (size_t)R));
     J3G_TRY(ensure(c, c->Jrowsum, sizeof(double) * (size_t)R));
+    J3G_TRY(ensure(c, c->rowmax, 2 * sizeof(unsigned) * (size_t)R));
     J3G_TRY(ensure(c, c->rows, sizeof(double) * (size_t)chunk * NS * K));
     J3G_TRY(ensure(c, c->gerr, sizeof(int)));
     J3G_CUDA(c, cudaMemsetAsync(c->gerr.p, 0, sizeof(int), c->stream));
-    for (int s0 = 0; s0 < c->nmeas; s0 += chunk) {
-      const int ns = std::min(chunk, c->nmeas - s0);
-      J3G_LAUNCH(c, launch_stored_rows(c->kind, m, s, s0, ns, mf, ptr<double>(c->F),
-                                       ptr<double>(c->rows), nullptr, K, c->stream));
-      ++c->launches;
-      J3G_LAUNCH(c, launch_split_rows(ptr<double>(c->rows), K, K, ns * NS, c->Jhi.p, c->Jlo.p,
-                                      ldK, ptr<float>(c->rowscale), ptr<double>(c->Jrowsum),
-                                      (long long)s0 * NS, c->stream));
+    J3G_CUDA(c, cudaMemsetAsync(c->rowmax.p, 0, 2 * sizeof(unsigned) * (size_t)R, c->stream));
+    const StoredPair p{c->Jhi.p, c->Jlo.p, c->JThi.p, c->JTlo.p, ldK, ldR,
+                       ptr<float>(c->rowscale), ptr<double>(c->Jrowsum)};
+    J3G_LAUNCH(c, launch_zero_padding(p, R, K, c->stream));
+    for (int s0 = 0; s0 < c->nmeas; s0 += (int)chunk) {
+      const int ns = std::min((int)chunk, c->nmeas - s0);
+      J3G_LAUNCH(c, launch_stored_pair(c->kind, m, s, s0, ns, mf, ptr<double>(c->F),
+                                       ptr<double>(c->rows), K,
+                                       ptr<unsigned>(c->rowmax), p, c->stream));
+      c->launches += 3;  // node terms, cell rows, row sums, split
     }
-    J3G_LAUNCH(c, launch_transpose16(c->Jhi.p, ldK, R, K, c->JThi.p, ldR, c->stream));
-    J3G_LAUNCH(c, launch_transpose16(c->Jlo.p, ldK, R, K, c->JTlo.p, ldR, c->stream));
   }
   J3G_CUDA(c, cudaStreamSynchronize(c->stream));
   c->storage = storage;
@@ -1105,7 +1118,7 @@ int j3g_destroy(j3g_context *c) {
                     &c->G, &c->F, &c->rows, &c->rowsum, &c->probe, &c->J32, &c->Jhi,
                     &c->Jlo, &c->JThi, &c->JTlo, &c->rowscale, &c->x32, &c->sums, &c->part,
                     &c->Bhi, &c->Blo, &c->P, &c->wst, &c->wrawb, &c->rawb, &c->gerr,
-                    &c->mscale, &c->Jrowsum, &c->mmean, &c->swork, &c->sexp, &c->chunks, &c->rmaps,
+                    &c->mscale, &c->Jrowsum, &c->rowmax, &c->mmean, &c->swork, &c->sexp, &c->chunks, &c->rmaps,
                     &c->rcoarse, &c->rfine};
   for (DevBuf *b : bufs)
     if (b->p) cudaFree(b->p);

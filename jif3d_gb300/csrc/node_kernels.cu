@@ -14,34 +14,18 @@
 // busy each and the schedulers issue in 60 % of the cycles.
 #include <algorithm>
 
-#include "node_fixed.cuh"
+#include "node_column.cuh"
 #include "prism_kernels.h"
 
 namespace j3g {
 namespace {
 
-// 128 threads at 96 registers: five blocks, 20 warps, to an SM (256 threads at
-// 128 registers: 16 warps, 1 to 7 % slower)
-constexpr int kNodeThreads = 128;
-constexpr int kNodeResident = 5;
 constexpr int kMaxColumn = 64;  // z offsets of a forward block held at a time
 constexpr int kAdjNodes = 8;    // nodes of a column per adjoint thread
 constexpr int kAdjStage = 16;   // stations staged at a time
 
 // The tables of node_fixed.cuh are copied to shared memory: random lookups
 // there cost a few bank conflicts, through L1 up to a cycle per lane.
-struct ZOffset {
-  FxAxis a;
-  double d;
-};
-
-__device__ __forceinline__ ZOffset z_offset(double mz, double Z) {
-  ZOffset o;
-  o.d = sub(mz, Z);
-  o.a = fx_axis(o.d);
-  return o;
-}
-
 // rho~(i,j,k) = sum_{a,b,c in {0,1}} (-1)^(a+b+c) rho(i-a, j-b, k-c), zero
 // outside, in the column order of the forward: [k][column].
 __global__ void __launch_bounds__(kNodeThreads)

@@ -318,28 +318,7 @@ __global__ void k_background_grad(int kind, int nmeas, int nbg, const double *__
 }
 
 // ---------------------------------------------------------------------------
-// Sensitivity rows.
-template <int KIND>
-__global__ void __launch_bounds__(kThreads)
-    k_node_eval(MeshView m, StationView st, int s0, double *__restrict__ F) {
-  using T = KindTraits<KIND>;
-  constexpr int MASK = T::mask;
-  constexpr int NCMP = T::ncomp;
-  const int ny1 = m.ny + 1, nz1 = m.nz + 1;
-  const int nn = (m.nx + 1) * ny1 * nz1;
-  const int n = blockIdx.x * kThreads + threadIdx.x;
-  const int sl = blockIdx.y;
-  if (n >= nn) return;
-  int i, j, k;
-  decode_node(n, ny1, nz1, i, j, k);
-  const int s = s0 + sl;
-  double v[T::twin ? 2 : 1][NC_COUNT];
-  const double dx = sub(st.x[s], m.X[i]), dy = sub(st.y[s], m.Y[j]);
-  node_terms<MASK>(dx, dy, sub(st.z[s], m.Z[k]), v[0]);
-  if constexpr (T::twin) node_terms<MASK>(dx, dy, sub(add(st.z[s], 1.0), m.Z[k]), v[T::twin ? 1 : 0]);
-#pragma unroll
-  for (int q = 0; q < NCMP; ++q) F[((long long)sl * NCMP + q) * nn + n] = v[T::at(q)][T::comp(q)];
-}
+// Sensitivity rows of meshes whose corners are given one by one.
 
 // Raw rows of one cell from its virtual-component box values u[q]:
 // the ordinary kinds through raw_from_comps, the vertical gradient through
@@ -369,95 +348,6 @@ __device__ __forceinline__ void store_cell_rows(const double *u, const MagField 
     raw_from_comps(KIND, c, mf, raw);
 #pragma unroll
     for (int r = 0; r < T::raw; ++r) rows[(long long)r * ld + cell] = (OutT)raw[r];
-  }
-}
-
-template <int KIND>
-__global__ void __launch_bounds__(kThreads)
-    k_cell_rows(MeshView m, const double *__restrict__ F, MagField mf, double *__restrict__ rows,
-                long long ld) {
-  using T = KindTraits<KIND>;
-  constexpr int NCMP = T::ncomp;
-  const long long cell = (long long)blockIdx.x * kThreads + threadIdx.x;
-  const int sl = blockIdx.y;
-  if (cell >= m.ngrid()) return;
-  const int k = cell % m.nz;
-  const long long t = cell / m.nz;
-  const int j = t % m.ny;
-  const int i = t / m.ny;
-  const int ny1 = m.ny + 1, nz1 = m.nz + 1;
-  const int nn = (m.nx + 1) * ny1 * nz1;
-  double u[kMaxVc];
-#pragma unroll
-  for (int q = 0; q < NCMP; ++q) {
-    const double *f = F + ((long long)sl * NCMP + q) * nn;
-    double v[8];
-#pragma unroll
-    for (int c = 0; c < 8; ++c)
-      v[c] = f[((i + ((c >> 2) & 1)) * ny1 + (j + ((c >> 1) & 1))) * nz1 + (k + (c & 1))];
-    u[q] = combine8(T::comp(q), v);
-  }
-  store_cell_rows<KIND>(u, mf, m.ngrid(), cell, rows + (long long)sl * T::raw * ld, ld);
-}
-
-// Stored rows for the device-resident sensitivity: the node components of the
-// kind (scalar 1, tensor 6, joint 7) or the raw magnetic rows (3 of Bx By Bz;
-// 1 of the vertical gradient; 3 over the three magnetisation blocks, columns
-// block * ngrid + cell), one row per (station, stored component), written as
-// OutT (double or float).
-template <int KIND> struct StoredRows {
-  static constexpr int n = stored_rows(KIND);
-};
-
-template <int KIND, class OutT>
-__global__ void __launch_bounds__(kThreads)
-    k_cell_stored(MeshView m, const double *__restrict__ F, MagField mf, OutT *__restrict__ rows,
-                  long long ld) {
-  constexpr int NCMP = KindTraits<KIND>::ncomp;
-  constexpr int OFF = Slots<KIND>::off;
-  constexpr int NS = StoredRows<KIND>::n;
-  const long long cell = (long long)blockIdx.x * kThreads + threadIdx.x;
-  const int sl = blockIdx.y;
-  if (cell >= m.ngrid()) return;
-  const int k = cell % m.nz;
-  const long long t = cell / m.nz;
-  const int j = t % m.ny;
-  const int i = t / m.ny;
-  const int ny1 = m.ny + 1, nz1 = m.nz + 1;
-  const int nn = (m.nx + 1) * ny1 * nz1;
-  if constexpr (KindTraits<KIND>::special) {
-    // the raw rows, as k_cell_rows forms them
-    double u[kMaxVc];
-#pragma unroll
-    for (int q = 0; q < NCMP; ++q) {
-      const double *f = F + ((long long)sl * NCMP + q) * nn;
-      double v[8];
-#pragma unroll
-      for (int c = 0; c < 8; ++c)
-        v[c] = f[((i + ((c >> 2) & 1)) * ny1 + (j + ((c >> 1) & 1))) * nz1 + (k + (c & 1))];
-      u[q] = combine8(KindTraits<KIND>::comp(q), v);
-    }
-    store_cell_rows<KIND, OutT>(u, mf, m.ngrid(), cell, rows + (long long)sl * NS * ld, ld);
-  } else {
-    double u[NC_COUNT];
-#pragma unroll
-    for (int q = 0; q < NCMP; ++q) {
-      const double *f = F + ((long long)sl * NCMP + q) * nn;
-      double v[8];
-#pragma unroll
-      for (int c = 0; c < 8; ++c)
-        v[c] = f[((i + ((c >> 2) & 1)) * ny1 + (j + ((c >> 1) & 1))) * nz1 + (k + (c & 1))];
-      u[q + OFF] = combine8(q + OFF, v);
-    }
-    if (KIND == KIND_MAGNETIC) {
-      double raw[10];
-      raw_from_comps(KIND, u, mf, raw);
-#pragma unroll
-      for (int r = 0; r < 3; ++r) rows[((long long)sl * NS + r) * ld + cell] = (OutT)raw[r];
-    } else {
-#pragma unroll
-      for (int q = 0; q < NCMP; ++q) rows[((long long)sl * NS + q) * ld + cell] = (OutT)u[q + OFF];
-    }
   }
 }
 
@@ -627,37 +517,10 @@ cudaError_t launch_background_grad(int kind, int nmeas, int nbg, const double *w
   return cudaGetLastError();
 }
 
-cudaError_t launch_sens_rows(int kind, bool node_exact, const MeshView &m, const StationView &s,
-                             int s0, int ns, const MagField &mf, double *F, double *rows,
-                             long long ld, cudaStream_t st) {
-  if (node_exact) {
-    dim3 g1(cdiv(m.nnodes(), kThreads), ns);
-    dim3 g2(cdiv(m.ngrid(), kThreads), ns);
-    J3G_DISPATCH(kind, (k_node_eval<K><<<g1, kThreads, 0, st>>>(m, s, s0, F),
-                        k_cell_rows<K><<<g2, kThreads, 0, st>>>(m, F, mf, rows, ld)));
-  } else {
-    dim3 g2(cdiv(m.ngrid(), kThreads), ns);
-    J3G_DISPATCH(kind, (k_cell_direct<K><<<g2, kThreads, 0, st>>>(m, s, s0, mf, rows, ld)));
-  }
-  return cudaGetLastError();
-}
-
-int stored_rows_per_station(int kind) {
-  return stored_rows(kind);
-}
-
-cudaError_t launch_stored_rows(int kind, const MeshView &m, const StationView &s, int s0, int ns,
-                               const MagField &mf, double *F, double *rows64, float *rows32,
-                               long long ld, cudaStream_t st) {
-  dim3 g1(cdiv(m.nnodes(), kThreads), ns);
-  dim3 g2(cdiv(m.ngrid(), kThreads), ns);
-  if (rows64) {
-    J3G_DISPATCH(kind, (k_node_eval<K><<<g1, kThreads, 0, st>>>(m, s, s0, F),
-                        k_cell_stored<K, double><<<g2, kThreads, 0, st>>>(m, F, mf, rows64, ld)));
-  } else {
-    J3G_DISPATCH(kind, (k_node_eval<K><<<g1, kThreads, 0, st>>>(m, s, s0, F),
-                        k_cell_stored<K, float><<<g2, kThreads, 0, st>>>(m, F, mf, rows32, ld)));
-  }
+cudaError_t launch_direct_rows(int kind, const MeshView &m, const StationView &s, int s0, int ns,
+                               const MagField &mf, double *rows, long long ld, cudaStream_t st) {
+  const dim3 grid(cdiv(m.ngrid(), kThreads), ns);
+  J3G_DISPATCH(kind, (k_cell_direct<K><<<grid, kThreads, 0, st>>>(m, s, s0, mf, rows, ld)));
   return cudaGetLastError();
 }
 

@@ -91,22 +91,40 @@ cudaError_t launch_adjoint_combine(const MeshView &m, int nchunk, int nblock, co
 cudaError_t launch_background_grad(int kind, int nmeas, int nbg, const double *w_raw,
                                    const double *bgsens, double *grad_bg, cudaStream_t st);
 
-// Sensitivity rows (reference per-cell order).  rows[(sl*raw + r) * ld + cell]
-// for stations s0 .. s0+ns-1 (sl = s - s0); magnetisation rows carry the three
-// blocks at columns b * ngrid + cell.  node_exact selects the node-term
-// path (F scratch of ns * ncomp * nnodes doubles), otherwise eight corner
-// evaluations per cell.
-cudaError_t launch_sens_rows(int kind, bool node_exact, const MeshView &m,
-                             const StationView &s, int s0, int ns, const MagField &mf,
-                             double *F, double *rows, long long ld, cudaStream_t st);
-// Rows of the device-resident sensitivity for stations s0..s0+ns-1: per
-// station the kind's node components (scalar 1, tensor 6 = xx yy zz xy xz yz,
-// joint 7 = gz + tensor) or, for magnetics, the 3 raw rows Bx By Bz.  Written
-// as double (rows64) or float (rows32), row (sl*nstored + q) at stride ld.
-int stored_rows_per_station(int kind);
-cudaError_t launch_stored_rows(int kind, const MeshView &m, const StationView &s, int s0, int ns,
-                               const MagField &mf, double *F, double *rows64, float *rows32,
-                               long long ld, cudaStream_t st);
+// Raw sensitivity rows by eight corner evaluations per cell (corners that are
+// not node terms): rows[(sl*raw + r) * ld + cell] for stations s0 .. s0+ns-1
+// (sl = s - s0); magnetisation rows carry the three blocks at columns
+// b * ngrid + cell.
+cudaError_t launch_direct_rows(int kind, const MeshView &m, const StationView &s, int s0, int ns,
+                               const MagField &mf, double *rows, long long ld, cudaStream_t st);
+// The same from the node terms, kept in F: ns * node_terms_stored(kind) *
+// nnodes doubles.
+int node_terms_stored(int kind);
+cudaError_t launch_node_rows(int kind, const MeshView &m, const StationView &s, int s0, int ns,
+                             const MagField &mf, double *F, double *rows, long long ld,
+                             cudaStream_t st);
+// Rows of the device-resident sensitivity for the same stations: per station
+// the kind's node components (scalar 1, tensor 6 = xx yy zz xy xz yz, joint 7 =
+// gz + tensor) or, for the magnetic kinds, the raw rows.  As floats at stride ld:
+cudaError_t launch_stored_rows32(int kind, const MeshView &m, const StationView &s, int s0, int ns,
+                                 const MagField &mf, double *F, float *rows, long long ld,
+                                 cudaStream_t st);
+// or as the fp16 pair (stored.h): row = scale * (hi + lo) with a power-of-two
+// scale, max|hi| in (2^13, 2^14], hi / lo with ld columns and the transpose thi /
+// tlo with ldt columns, both tiled, and the FP64 row sums J 1.  rows: scratch of
+// ns * stored rows * K doubles; rowmax: two zeroed words per row of the whole
+// matrix (largest high word, any NaN).  Columns beyond K are written as zero, the
+// rest of the padding by launch_zero_padding.
+struct StoredPair {
+  void *hi, *lo, *thi, *tlo;
+  long long ld, ldt;
+  float *rowscale;
+  double *rowsum;
+};
+cudaError_t launch_stored_pair(int kind, const MeshView &m, const StationView &s, int s0, int ns,
+                               const MagField &mf, double *F, double *rows, long long K,
+                               unsigned *rowmax, const StoredPair &p, cudaStream_t st);
+cudaError_t launch_zero_padding(const StoredPair &p, long long R, long long K, cudaStream_t st);
 
 // d[(s0+sl)*raw + r] = sum_cell rows[(sl*raw + r)*ld + cell] * rho[cell]
 cudaError_t launch_rows_dot(int raw, int ns, long long ngrid, const double *rows, long long ld,

@@ -93,57 +93,6 @@ __device__ __forceinline__ double block_max_abs(const T &get, long long n, doubl
   return r;
 }
 
-// One block per row: power-of-two row scale and fp16 hi / lo split of an FP64
-// row (padding columns zero).  scale[row0 + r] receives the scale and, when
-// given, rowsum[row0 + r] the FP64 sum of the row (J 1, used to add back the
-// mean of a centred model).
-__global__ void k_split_rows(const double *__restrict__ rows, long long ld_in, long long ncol,
-                             __half *__restrict__ hi, __half *__restrict__ lo, long long ld_out,
-                             float *__restrict__ scale, double *__restrict__ rowsum,
-                             long long row0) {
-  const long long r = blockIdx.x;
-  const double *p = rows + r * ld_in;
-  __shared__ double red[kT / 32];
-  const double sc = pow2_scale(block_max_abs([&](long long c) { return p[c]; }, ncol, red));
-  if (threadIdx.x == 0) scale[row0 + r] = (float)sc;
-  if (rowsum) {
-    double acc = 0.0;
-    for (long long c = threadIdx.x; c < ncol; c += kT) acc += p[c];
-    acc = block_sum_d<kT>(acc, red);
-    if (threadIdx.x == 0) rowsum[row0 + r] = acc;
-  }
-  const double inv = 1.0 / sc;
-  for (long long c = threadIdx.x; c < ld_out; c += kT) {
-    __half hv, lv;
-    split_half(c < ncol ? p[c] * inv : 0.0, hv, lv);
-    const long long o = tiled_index(row0 + r, c, ld_out);
-    hi[o] = hv;
-    lo[o] = lv;
-  }
-}
-
-// 32x32 blocked transpose of a 16-bit matrix, (r, c) -> (c, r), both in the
-// tiled layout (a 32-wide block never straddles a 64-column tile).
-__global__ void k_transpose16(const uint16_t *__restrict__ in, long long ld_in, long long rows,
-                              long long cols, uint16_t *__restrict__ out, long long ld_out) {
-  __shared__ uint16_t tile[32][34];
-  const long long c0 = (long long)blockIdx.x * 32;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8 threads
-  // row blocks loop over grid y (at most 65535 blocks)
-  for (long long r0 = (long long)blockIdx.y * 32; r0 < ld_out; r0 += (long long)gridDim.y * 32) {
-    __syncthreads();  // the previous block's tile has been written out
-    for (int k = ty; k < 32; k += 8) {
-      const long long r = r0 + k, c = c0 + tx;
-      tile[k][tx] = (r < rows && c < cols) ? in[tiled_index(r, c, ld_in)] : (uint16_t)0;
-    }
-    __syncthreads();
-    for (int k = ty; k < 32; k += 8) {
-      const long long c = c0 + k, r = r0 + tx;
-      if (c < cols && r < ld_out) out[tiled_index(c, r, ld_out)] = tile[tx][k];
-    }
-  }
-}
-
 // Splitting an FP64 matrix [nrow][ld_src] (the adjoint's scaled residual
 // rows) into fp16 hi / lo rows [nrow_pad][ld_dst], in three grid-wide passes
 // so that a few hundred long rows still fill the GPU:
@@ -1064,23 +1013,6 @@ inline int grid_for(long long n) {
 }
 
 }  // namespace
-
-cudaError_t launch_split_rows(const double *rows, long long ld_in, long long ncol, int nrows,
-                              void *hi, void *lo, long long ld_out, float *scale, double *rowsum,
-                              long long row0, cudaStream_t st) {
-  if (nrows == 0) return cudaSuccess;
-  k_split_rows<<<nrows, kT, 0, st>>>(rows, ld_in, ncol, static_cast<__half *>(hi),
-                                     static_cast<__half *>(lo), ld_out, scale, rowsum, row0);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_transpose16(const void *in, long long ld_in, long long rows, long long cols,
-                               void *out, long long ld_out, cudaStream_t st) {
-  dim3 grid(cdiv(cols, 32), std::min(cdiv(ld_out, 32), 65535));
-  k_transpose16<<<grid, 256, 0, st>>>(static_cast<const uint16_t *>(in), ld_in, rows, cols,
-                                      static_cast<uint16_t *>(out), ld_out);
-  return cudaGetLastError();
-}
 
 int split_matrix_launches(long long ld_dst) { return ld_dst <= kSmallRow ? 1 : 3; }
 

@@ -18,18 +18,6 @@ __host__ __device__ inline long long tiled_index(long long r, long long c, long 
 }
 inline long long tiled_rows(long long rows) { return (rows + 127) / 128 * 128; }
 
-// fp16 hi / lo split of FP64 rows with a power-of-two row scale
-// (scale[row0 + r]): row = scale * (hi + lo), max|hi| in (2^13, 2^14];
-// hi / lo in the tiled layout with ld_out columns (padding columns zero).
-// rowsum (optional) receives the FP64 row sums J 1.
-cudaError_t launch_split_rows(const double *rows, long long ld_in, long long ncol, int nrows,
-                              void *hi, void *lo, long long ld_out, float *scale, double *rowsum,
-                              long long row0, cudaStream_t st);
-// out(c, r) = in(r, c) for r < rows (zero for rows <= r < ld_out), c < cols;
-// 16-bit elements, both matrices in the tiled layout (in: ld_in columns,
-// out: ld_out columns).
-cudaError_t launch_transpose16(const void *in, long long ld_in, long long rows, long long cols,
-                               void *out, long long ld_out, cudaStream_t st);
 // FP64 [nrow][ld_src] (column c times colscale[c] when given) -> fp16 hi / lo
 // [nrow_pad][ld_dst] with a power-of-two scale per row into rowscale[r]; rows
 // beyond nrow and columns beyond ncol are zero.  work:

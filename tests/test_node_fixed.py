@@ -152,3 +152,28 @@ def test_offsets_left_to_fp64(ctx, oracle_lib, kind):
     # the far field's box terms are rounding in FP64 too: finite, and no larger
     # than a few units of the node terms
     assert np.all(np.isfinite(ctx.forward(far.model)))
+
+
+# rows of one station a multiple of 64, of 16, odd; fewer cells than a tile, not
+# a multiple of it; one station, and more than a chunk of eight
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("shape", [(3, 2, 1, 1), (5, 5, 5, 8), (7, 9, 11, 33), (16, 4, 8, 130)])
+def test_stored_pair_at_tile_edges(ctx, kind, shape):
+    """The fp16 pair and its transpose, built in one pass: J m of unit models and
+    J^T r of unit residuals give the matrix back, column by column and row by
+    row, within the 2^-21 of its entries' rows that hi + lo keep."""
+    from jif3d_gb300 import capi
+    s = _survey(kind, *shape, False)
+    W.setup_context(ctx, s)
+    J = _rows(s)
+    ctx.build_sensitivity(capi.STORE_F16X2)
+    rng = np.random.default_rng(5)
+    cols = rng.choice(s.nparm, min(s.nparm, 40), replace=False)
+    d = ctx.batched_forward(np.eye(s.nparm)[cols])
+    bound = 2.0 ** -21 * np.abs(J).max(axis=1)
+    # a unit model is centred on its mean, which is added back with J 1
+    assert np.all(np.abs(d - J[:, cols].T) <= 2 * bound[None, :])
+    rows = rng.choice(J.shape[0], min(J.shape[0], 40), replace=False)
+    g = ctx.batched_lqderivative(None, np.eye(J.shape[0])[rows])
+    assert np.all(np.abs(g - 2.0 * J[rows]) <= 2 * 2 * bound[rows, None])
