@@ -675,11 +675,11 @@ int stored_forward_f32(j3g_context *c, const double *d_model, double *d_data, do
   tfa_dir(c, tbx, tby, tbz);
   J3G_TRY(ensure(c, c->x32, sizeof(float) * (size_t)ldK));
   J3G_TRY(ensure(c, c->sums, sizeof(double) * (size_t)R));
-  J3G_LAUNCH(c, launch_to_f32(d_model, K, ldK, ptr<float>(c->x32), c->stream));
+  J3G_LAUNCH(c, launch_to_f32(d_model, K, 1, K, ldK, ptr<float>(c->x32), c->stream));
   {
     TimedScope ts(c, J3G_TIMER_STREAM_FORWARD);
-    J3G_LAUNCH(c, launch_gemv_f32(ptr<float>(c->J32), ldK, (int)R, ptr<float>(c->x32),
-                                  ptr<double>(c->sums), c->stream));
+    J3G_LAUNCH(c, launch_gemv_f32(ptr<float>(c->J32), ldK, (int)R, 1, ptr<float>(c->x32),
+                                  ptr<double>(c->sums), R, c->stream));
   }
   const int nbg = c->nbg_active();
   J3G_LAUNCH(c, launch_stored_assemble(c->kind, c->transform, tbx, tby, tbz, c->nmeas, 1,
@@ -721,8 +721,8 @@ int stored_adjoint_f32(j3g_context *c, const double *d_model, const double *d_mi
                                       ptr<double>(c->wrawb), ptr<double>(c->wst), R, c->stream));
   {
     TimedScope ts(c, J3G_TIMER_STREAM_ADJOINT);
-    J3G_LAUNCH(c, launch_gemv_t_f32(ptr<float>(c->J32), ldK, (int)R, ptr<double>(c->wst),
-                                    ptr<double>(c->part), K, 2.0, d_grad, c->stream));
+    J3G_LAUNCH(c, launch_gemv_t_f32(ptr<float>(c->J32), ldK, (int)R, 1, ptr<double>(c->wst), R,
+                                    ptr<double>(c->part), K, 2.0, d_grad, c->nparm(), c->stream));
   }
   ++c->launches;  // column-block sums + chunk reduction
   if (nbg)
@@ -891,11 +891,14 @@ int batched_forward_pass(j3g_context *c, int nmod, const double *d_models, doubl
   const int nbg = c->nbg_active();
   J3G_TRY(ensure(c, c->sums, sizeof(double) * (size_t)nmod * R));
   if (c->storage == J3G_STORE_FP32) {
-    for (int n = 0; n < nmod; ++n) {
-      J3G_TRY(ensure(c, c->x32, sizeof(float) * (size_t)ldK));
-      J3G_LAUNCH(c, launch_to_f32(d_models + (size_t)n * np, K, ldK, ptr<float>(c->x32), c->stream));
-      J3G_LAUNCH(c, launch_gemv_f32(ptr<float>(c->J32), ldK, (int)R, ptr<float>(c->x32),
-                                    ptr<double>(c->sums) + (size_t)n * R, c->stream));
+    // kStreamModels models per pass over J
+    J3G_TRY(ensure(c, c->x32, sizeof(float) * (size_t)std::min(nmod, kStreamModels) * ldK));
+    for (int n = 0; n < nmod; n += kStreamModels) {
+      const int nm = std::min(kStreamModels, nmod - n);
+      J3G_LAUNCH(c, launch_to_f32(d_models + (size_t)n * np, np, nm, K, ldK, ptr<float>(c->x32),
+                                  c->stream));
+      J3G_LAUNCH(c, launch_gemv_f32(ptr<float>(c->J32), ldK, (int)R, nm, ptr<float>(c->x32),
+                                    ptr<double>(c->sums) + (size_t)n * R, R, c->stream));
     }
   } else {
     const int tile = gemm_n_tile(nmod);
@@ -988,11 +991,14 @@ int batched_adjoint_pass(j3g_context *c, int nmod, const double *d_models,
                                         R, c->stream));
   }
   if (c->storage == J3G_STORE_FP32) {
-    J3G_TRY(ensure(c, c->part, sizeof(double) * (size_t)gemv_t_chunks((int)R) * ldK));
-    for (int n = 0; n < nmod; ++n) {
+    J3G_TRY(ensure(c, c->part, sizeof(double) * (size_t)std::min(nmod, kStreamModels) *
+                                   gemv_t_chunks((int)R) * ldK));
+    for (int n = 0; n < nmod; n += kStreamModels) {
       J3G_LAUNCH(c, launch_gemv_t_f32(ptr<float>(c->J32), ldK, (int)R,
-                                      ptr<double>(c->wst) + (size_t)n * R, ptr<double>(c->part), K,
-                                      2.0, d_grads + (size_t)n * np, c->stream));
+                                      std::min(kStreamModels, nmod - n),
+                                      ptr<double>(c->wst) + (size_t)n * R, R,
+                                      ptr<double>(c->part), K, 2.0, d_grads + (size_t)n * np, np,
+                                      c->stream));
       ++c->launches;
     }
   } else {

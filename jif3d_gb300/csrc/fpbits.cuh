@@ -43,6 +43,17 @@ __device__ __forceinline__ float f64_to_f32_ftz(double v) {
   return __uint_as_float(s | ((e2 - 896u) << 23) | (uint32_t)((m >> 29) & 0x7fffffu));
 }
 
+// Exact widening of a float that is rarely zero or subnormal (f32_to_f64 takes
+// those): the exponent and fraction move down three bits and the bias is added,
+// once more for infinities and NaNs.
+__device__ __forceinline__ double f32_to_f64(float f);
+__device__ __forceinline__ double widen_f32(float f) {
+  const uint32_t u = __float_as_uint(f), a = u & 0x7fffffffu;
+  if (a < 0x800000u) return f32_to_f64(f);
+  const uint32_t hi = (a >> 3) + (a >= 0x7f800000u ? 0x70000000u : 0x38000000u);
+  return __hiloint2double((int)(hi | (u & 0x80000000u)), (int)(u << 29));
+}
+
 // Exact widening of a float (including subnormals) to a double.
 __device__ __forceinline__ double f32_to_f64(float f) {
   const uint32_t u = __float_as_uint(f);

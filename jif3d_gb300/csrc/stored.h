@@ -28,16 +28,21 @@ int split_matrix_launches(long long ld_dst);
 cudaError_t launch_split_matrix(const double *src, long long ld_src, int nrow, long long ncol,
                                 const float *colscale, void *hi, void *lo, long long ld_dst,
                                 int nrow_pad, float *rowscale, double *work, cudaStream_t st);
-cudaError_t launch_to_f32(const double *src, long long n, long long npad, float *dst,
-                          cudaStream_t st);
-// d[r] = sum_c J[r][c] x[c] (FP32 J, FP32 x, FP64 result), ld multiple of 4.
-cudaError_t launch_gemv_f32(const float *J, long long ld, int nrows, const float *x, double *out,
-                            cudaStream_t st);
-// out[c] = factor * sum_r J[r][c] w[r]; part needs gemv_t_chunks(nrows) * ld doubles.
+cudaError_t launch_to_f32(const double *src, long long ld_src, int nrow, long long n,
+                          long long npad, float *dst, cudaStream_t st);
+// Models per pass over J of the FP32 products: the registers of the sums of
+// four models leave two blocks to an SM, still enough loads in flight.
+constexpr int kStreamModels = 4;
+// d[m][r] = sum_c J[r][c] x[m][c] for 1 .. kStreamModels models (FP32 J, FP32 x
+// [model][ld], FP64 result [model][ld_out]), ld multiple of 4.
+cudaError_t launch_gemv_f32(const float *J, long long ld, int nrows, int nmod, const float *x,
+                            double *out, long long ld_out, cudaStream_t st);
+// out[m][c] = factor * sum_r J[r][c] w[m][r] for 1 .. kStreamModels models; part
+// needs nmod * gemv_t_chunks(nrows) * ld doubles.
 int gemv_t_chunks(int nrows);
-cudaError_t launch_gemv_t_f32(const float *J, long long ld, int nrows, const double *w,
-                              double *part, long long ncol, double factor, double *out,
-                              cudaStream_t st);
+cudaError_t launch_gemv_t_f32(const float *J, long long ld, int nrows, int nmod, const double *w,
+                              long long ldw, double *part, long long ncol, double factor,
+                              double *out, long long ld_out, cudaStream_t st);
 // out[n][r] = factor * rowscale[r] * modscale[n] * sum_s 2^sexp[n][s] P[s][n][r]
 // (P float, out double; modscale and sexp optional, sexp [nmod][nsplit])
 // + modmean[n] * rowsum[r] when modmean is given (adds back a centred mean).

@@ -579,3 +579,24 @@ def test_autotuned_products(ctx, oracle_lib):
     for i in (0, 299):
         check_groups(s, d1[i], oracle_forward(oracle_lib, s, models[i]))
         assert relerr(g1[i], oracle_lqderivative(oracle_lib, s, mis[i], models[i])) <= TOL
+
+
+@pytest.mark.parametrize("shape", [(9, 8, 6), (16, 16, 15), (16, 16, 16), (17, 16, 16),
+                                   (32, 16, 16)])
+@pytest.mark.parametrize("nmeas", [1, 3, 37])
+def test_fp32_batches_share_a_pass(ctx, shape, nmeas):
+    """FP32 storage, 1 to 6 models (four to a pass over J): bit for bit the
+    models one at a time, at cell counts around whole chains of 16 x 256
+    products and row counts around the four rows of a block and the 128 rows of
+    a chunk."""
+    s = small_survey(W.JOINT, nx=shape[0], ny=shape[1], nz=shape[2], nmeas=nmeas, seed=11)
+    W.setup_context(ctx, s)
+    ctx.build_sensitivity(capi.STORE_FP32)
+    rng = np.random.default_rng(7)
+    models = s.model[None, :] * (1 + 0.1 * rng.normal(size=(6, s.nparm)))
+    mis = rng.normal(size=(6, nmeas * s.dpm))
+    one = [ctx.batched_forward(m[None, :])[0] for m in models]
+    grad = [ctx.batched_lqderivative(models[k:k + 1], mis[k:k + 1])[0] for k in range(6)]
+    for n in range(2, 7):
+        assert np.array_equal(ctx.batched_forward(models[:n]), np.array(one[:n]))
+        assert np.array_equal(ctx.batched_lqderivative(models[:n], mis[:n]), np.array(grad[:n]))
