@@ -46,7 +46,11 @@ struct j3g_context {
   // geometry (host copies)
   int nx = 0, ny = 0, nz = 0;
   bool mesh_set = false;
-  bool node_exact = true;
+  bool node_exact = true;  // every corner is a running sum of the cell sizes
+  bool node_path = true;   // the node kernels serve the mesh: exact, or through planes
+  int np[3] = {1, 1, 1};   // node planes of the axes (exact: nx + 1, ny + 1, nz + 1)
+  DevBuf dplanes, dplane_maps;
+  NodePlanes planes{};
   std::vector<double> X, Y, Z, xs, ys, zs;
   double xw = 0, yw = 0, zw = 0;
   std::vector<double> bg;
@@ -257,6 +261,22 @@ MeshView mesh_view(j3g_context *c) {
   return m;
 }
 
+// The node grid: the mesh's own nodes, or its planes.
+MeshView node_view(j3g_context *c) {
+  MeshView m = mesh_view(c);
+  if (c->node_exact) return m;
+  m.nx = c->np[0] - 1;
+  m.ny = c->np[1] - 1;
+  m.nz = c->np[2] - 1;
+  m.X = ptr<double>(c->dplanes);
+  m.Y = m.X + c->np[0];
+  m.Z = m.Y + c->np[1];
+  return m;
+}
+const NodePlanes *node_planes(const j3g_context *c) {
+  return c->node_exact ? nullptr : &c->planes;
+}
+
 StationView station_view(j3g_context *c) {
   StationView s;
   s.n = c->nmeas;
@@ -321,15 +341,15 @@ int ensure_background(j3g_context *c) {
 
 // Gridded node-component sums comps[nmeas][NC_COUNT] for the model d_model.
 int gridded_node_forward(j3g_context *c, const double *d_model) {
-  const long long nn = c->nnodes();
+  const MeshView m = node_view(c);
+  const long long nn = m.nnodes();
   const int nblock = kind_nblock(c->kind);
   J3G_TRY(ensure(c, c->rhot, sizeof(double) * nn * nblock));
-  MeshView m = mesh_view(c);
   for (int b = 0; b < nblock; ++b)
-    J3G_LAUNCH(c, launch_rho_tilde(m, d_model + (size_t)b * c->ngrid(),
+    J3G_LAUNCH(c, launch_rho_tilde(mesh_view(c), m, node_planes(c), d_model + (size_t)b * c->ngrid(),
                                    ptr<double>(c->rhot) + (size_t)b * nn, c->stream));
   const NodeForwardPlan p =
-      node_forward_plan(c->nx, c->ny, c->nz, c->nmeas, (1LL << 31) - 1);
+      node_forward_plan(m.nx, m.ny, m.nz, c->nmeas, (1LL << 31) - 1);
   const int nblk = p.nblk;
   const int ncomp = kind_ncomp(c->kind);
   J3G_TRY(ensure(c, c->partial, sizeof(double) * (size_t)nblk * c->nmeas * ncomp));
@@ -419,7 +439,7 @@ int forward_device(j3g_context *c, const double *d_model, double *d_data, double
   const double *bgsens = nbg ? ptr<double>(c->bgsens) : nullptr;
   // node sums per station: node components, or raw rows for the special kinds
   const int comps_ld = kind_special(c->kind) ? c->raw() : NC_COUNT;
-  if (h_sens || (!c->node_exact && c->ngrid() > 0)) {
+  if (h_sens || (!c->node_path && c->ngrid() > 0)) {
     J3G_TRY(gridded_rows_forward(c, d_model, h_sens));
     J3G_LAUNCH(c, launch_assemble(c->kind, c->transform, tbx, tby, tbz, c->nmeas,
                                 ptr<double>(c->rowsum), c->raw(), bgsens, nbg, bgval,
@@ -472,12 +492,14 @@ int adjoint_device(j3g_context *c, const double *d_model, const double *d_misfit
                                  ptr<double>(c->wraw), c->stream));
   MeshView m = mesh_view(c);
   StationView s = station_view(c);
-  if (ngrid > 0 && c->node_exact) {
+  if (ngrid > 0 && c->node_path) {
+    const MeshView nodes = node_view(c);
     J3G_TRY(ensure(c, c->W, sizeof(double) * (size_t)c->nmeas * std::max<int>(NC_COUNT, kMaxVc)));
     J3G_LAUNCH(c, launch_comp_weights(c->kind, c->nmeas, ptr<double>(c->wraw), mag_field(c),
                                     ptr<double>(c->W), c->stream));
-    const long long nn = c->nnodes();
-    const NodeAdjointPlan plan = node_adjoint_plan(c->nx, c->ny, c->nz, nblock, c->nmeas);
+    const long long nn = nodes.nnodes();
+    const NodeAdjointPlan plan =
+        node_adjoint_plan(nodes.nx, nodes.ny, nodes.nz, nblock, c->nmeas);
     const int spc = plan.spc;
     int nchunk = plan.nchunk;
     // chunks of at most spc stations that never straddle a subset
@@ -508,12 +530,12 @@ int adjoint_device(j3g_context *c, const double *d_model, const double *d_misfit
     J3G_TRY(ensure(c, c->G, sizeof(double) * (size_t)nblock * nn));
     if (nchunk > 0) {
       TimedScope ts(c, J3G_TIMER_NODE_ADJOINT);
-      J3G_LAUNCH(c, launch_node_adjoint(c->kind, m, s, ptr<double>(c->W), plan, nchunk, d_starts,
+      J3G_LAUNCH(c, launch_node_adjoint(c->kind, nodes, s, ptr<double>(c->W), plan, nchunk, d_starts,
                                         ptr<double>(c->Gpart), c->stream));
     }
     for (int k = 0; k < nsub; ++k) {
       const int c0 = first_chunk[k], nk = first_chunk[k + 1] - c0;
-      J3G_LAUNCH(c, launch_adjoint_combine(m, nk, nblock,
+      J3G_LAUNCH(c, launch_adjoint_combine(m, nodes, node_planes(c), nk, nblock,
                                            ptr<double>(c->Gpart) + (size_t)c0 * nblock * nn,
                                            ptr<double>(c->G), d_grad + (size_t)k * nparm,
                                            c->stream));
@@ -547,6 +569,62 @@ int adjoint_device(j3g_context *c, const double *d_model, const double *d_misfit
                                            ptr<double>(c->bgsens) + (size_t)off[k] * raw * nbg,
                                            gk + ngrid, c->stream));
   }
+  return J3G_OK;
+}
+
+// The node planes of a mesh whose corners are given one by one (NodePlanes):
+// the upper corner of cell i (corner + size, as the reference forms it) shares
+// the plane of the next cell's lower corner where the two are equal bit for bit.
+// Meshes of more than kMaxPlaneNodes plane nodes keep the eight-corner kernel.
+constexpr long long kMaxPlaneNodes = 1LL << 28;
+int set_planes(j3g_context *c) {
+  const int n[3] = {c->nx, c->ny, c->nz};
+  for (int a = 0; a < 3; ++a) c->np[a] = n[a] + 1;
+  c->node_path = c->node_exact;
+  if (c->node_exact || c->ngrid() == 0) return J3G_OK;
+  const std::vector<double> *corner[3] = {&c->X, &c->Y, &c->Z}, *size[3] = {&c->xs, &c->ys, &c->zs};
+  std::vector<double> coord;
+  std::vector<int> lower_of[3], upper_of[3], lower[3], upper[3], maps;
+  for (int a = 0; a < 3; ++a) {
+    auto plane = [&](double v, int lo, int up) {
+      coord.push_back(v);
+      lower_of[a].push_back(lo);
+      upper_of[a].push_back(up);
+      return (int)lower_of[a].size() - 1;
+    };
+    for (int i = 0; i < n[a]; ++i) {
+      const double lo = (*corner[a])[i];
+      if (i > 0 && (*corner[a])[i - 1] + (*size[a])[i - 1] == lo) {
+        lower[a].push_back(upper[a].back());
+        lower_of[a][lower[a].back()] = i;
+      } else {
+        lower[a].push_back(plane(lo, i, -1));
+      }
+      upper[a].push_back(plane(lo + (*size[a])[i], -1, i));
+    }
+    c->np[a] = (int)lower_of[a].size();
+  }
+  if ((long long)c->np[0] * c->np[1] * c->np[2] > kMaxPlaneNodes) return J3G_OK;
+  size_t off[4][3];
+  const std::vector<int> *part[4] = {lower_of, upper_of, lower, upper};
+  for (int p = 0; p < 4; ++p)
+    for (int a = 0; a < 3; ++a) {
+      off[p][a] = maps.size();
+      maps.insert(maps.end(), part[p][a].begin(), part[p][a].end());
+    }
+  J3G_TRY(upload(c, c->dplanes, coord));
+  J3G_TRY(ensure(c, c->dplane_maps, sizeof(int) * maps.size()));
+  J3G_CUDA(c, cudaMemcpyAsync(c->dplane_maps.p, maps.data(), sizeof(int) * maps.size(),
+                              cudaMemcpyHostToDevice, c->stream));
+  J3G_CUDA(c, cudaStreamSynchronize(c->stream));  // the host tables are locals
+  const int *d = ptr<int>(c->dplane_maps);
+  for (int a = 0; a < 3; ++a) {
+    c->planes.lower_of[a] = d + off[0][a];
+    c->planes.upper_of[a] = d + off[1][a];
+    c->planes.lower[a] = d + off[2][a];
+    c->planes.upper[a] = d + off[3][a];
+  }
+  c->node_path = true;
   return J3G_OK;
 }
 
@@ -1118,7 +1196,7 @@ int j3g_destroy(j3g_context *c) {
   if (!c) return J3G_OK;
   cudaSetDevice(c->device);
   cudaStreamSynchronize(c->stream);
-  DevBuf *bufs[] = {&c->dX, &c->dY, &c->dZ, &c->dxs, &c->dys, &c->dzs, &c->dbg, &c->dsx,
+  DevBuf *bufs[] = {&c->dplanes, &c->dplane_maps, &c->dX, &c->dY, &c->dZ, &c->dxs, &c->dys, &c->dzs, &c->dbg, &c->dsx,
                     &c->dsy, &c->dsz, &c->model, &c->data, &c->misfit, &c->grad, &c->rhot,
                     &c->partial, &c->comps, &c->bgsens, &c->rawd, &c->wraw, &c->W, &c->Gpart,
                     &c->G, &c->F, &c->rows, &c->rowsum, &c->probe, &c->J32, &c->Jhi,
@@ -1200,6 +1278,7 @@ int j3g_set_mesh(j3g_context *c, int nx, int ny, int nz, const double *xc, const
   J3G_TRY(upload(c, c->dxs, c->xs));
   J3G_TRY(upload(c, c->dys, c->ys));
   J3G_TRY(upload(c, c->dzs, c->zs));
+  J3G_TRY(set_planes(c));
   J3G_CUDA(c, cudaStreamSynchronize(c->stream));
   c->mesh_set = true;
   c->refine_set = false;  // the walks belong to the old mesh

@@ -129,7 +129,7 @@ extern "C" int j3g_forward_noalloc(int kind, int nx, int ny, int nz, const doubl
   // every scratch value read below is written first in the same call, so no
   // clearing is needed: rho~ covers all nodes, the partials all (block,
   // station, component) triples and the sums all (station, component) pairs
-  if (launch_rho_tilde(m, d_model, rho_t, st) != cudaSuccess) return J3G_ERR_CUDA;
+  if (launch_rho_tilde(m, m, nullptr, d_model, rho_t, st) != cudaSuccess) return J3G_ERR_CUDA;
   if (launch_node_forward(kind, m, s, rho_t, partial, plan, st) != cudaSuccess)
     return J3G_ERR_CUDA;
   if (launch_forward_reduce(kind, nmeas, plan.nblk, partial, mf, comps, st) != cudaSuccess)

@@ -26,21 +26,29 @@ constexpr int kAdjStage = 16;   // stations staged at a time
 
 // The tables of node_fixed.cuh are copied to shared memory: random lookups
 // there cost a few bank conflicts, through L1 up to a cycle per lane.
-// rho~(i,j,k) = sum_{a,b,c in {0,1}} (-1)^(a+b+c) rho(i-a, j-b, k-c), zero
-// outside, in the column order of the forward: [k][column].
+// rho~ of a node: the signed sum of the cells that it is a corner of, zero
+// outside, (-1)^(number of axes along which it is the upper corner), in the
+// column order of the forward: [k][column].  PLANES: the node planes of an axis
+// are given by p (cells whose lower and upper corner planes are apart), else
+// plane i is the lower corner of cell i and the upper corner of cell i - 1.
+template <bool PLANES>
 __global__ void __launch_bounds__(kNodeThreads)
-    k_rho_tilde(MeshView m, const double *__restrict__ rho, double *__restrict__ rt) {
-  const int ny1 = m.ny + 1, ncol = (m.nx + 1) * ny1;
+    k_rho_tilde(MeshView m, MeshView nodes, NodePlanes p, const double *__restrict__ rho,
+                double *__restrict__ rt) {
+  const int ny1 = nodes.ny + 1, ncol = (nodes.nx + 1) * ny1;
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= ncol * (m.nz + 1)) return;
+  if (n >= ncol * (nodes.nz + 1)) return;
   const int k = n / ncol, col = n - k * ncol, i = col / ny1, j = col - i * ny1;
+  const int ci[2] = {PLANES ? p.lower_of[0][i] : i, PLANES ? p.upper_of[0][i] : i - 1};
+  const int cj[2] = {PLANES ? p.lower_of[1][j] : j, PLANES ? p.upper_of[1][j] : j - 1};
+  const int ck[2] = {PLANES ? p.lower_of[2][k] : k, PLANES ? p.upper_of[2][k] : k - 1};
   double v = 0.0;
 #pragma unroll
   for (int q = 0; q < 8; ++q) {
     const int a = (q >> 2) & 1, b = (q >> 1) & 1, c = q & 1;
-    const int ci = i - a, cj = j - b, ck = k - c;
-    if (ci < 0 || cj < 0 || ck < 0 || ci >= m.nx || cj >= m.ny || ck >= m.nz) continue;
-    const double r = rho[((long long)ci * m.ny + cj) * m.nz + ck];
+    if (ci[a] < 0 || cj[b] < 0 || ck[c] < 0 || ci[a] >= m.nx || cj[b] >= m.ny || ck[c] >= m.nz)
+      continue;
+    const double r = rho[((long long)ci[a] * m.ny + cj[b]) * m.nz + ck[c]];
     v = ((a + b + c) & 1) ? v - r : v + r;
   }
   rt[n] = v;
@@ -332,9 +340,13 @@ static cudaError_t adjoint_launch(dim3 grid, int threads, size_t smem, cudaStrea
     default: return cudaErrorInvalidValue;                                        \
   }
 
-cudaError_t launch_rho_tilde(const MeshView &m, const double *rho, double *rho_t,
-                             cudaStream_t st) {
-  k_rho_tilde<<<cdiv(m.nnodes(), kNodeThreads), kNodeThreads, 0, st>>>(m, rho, rho_t);
+cudaError_t launch_rho_tilde(const MeshView &m, const MeshView &nodes, const NodePlanes *planes,
+                             const double *rho, double *rho_t, cudaStream_t st) {
+  const int blocks = cdiv(nodes.nnodes(), kNodeThreads);
+  if (planes)
+    k_rho_tilde<true><<<blocks, kNodeThreads, 0, st>>>(m, nodes, *planes, rho, rho_t);
+  else
+    k_rho_tilde<false><<<blocks, kNodeThreads, 0, st>>>(m, nodes, NodePlanes{}, rho, rho_t);
   return cudaGetLastError();
 }
 

@@ -278,21 +278,25 @@ __global__ void k_sum_chunks(int nn, int nchunk, long long stride,
   G[n] = v;
 }
 
-// grad(cell) = 2 * sum_{a,b,c} (-1)^(a+b+c) G(i+a, j+b, k+c)
-__global__ void k_adjoint_combine(MeshView m, const double *__restrict__ G,
-                                  double *__restrict__ grad) {
+// grad(cell) = 2 * sum_{a,b,c} (-1)^(a+b+c) G(corner a, b, c of the cell)
+template <bool PLANES>
+__global__ void k_adjoint_combine(MeshView m, MeshView nodes, NodePlanes p,
+                                  const double *__restrict__ G, double *__restrict__ grad) {
   const long long cell = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (cell >= m.ngrid()) return;
   const int k = cell % m.nz;
   const long long t = cell / m.nz;
   const int j = t % m.ny;
   const int i = t / m.ny;
-  const int ny1 = m.ny + 1, nz1 = m.nz + 1;
+  const int ny1 = nodes.ny + 1, nz1 = nodes.nz + 1;
+  const int ni[2] = {PLANES ? p.lower[0][i] : i, PLANES ? p.upper[0][i] : i + 1};
+  const int nj[2] = {PLANES ? p.lower[1][j] : j, PLANES ? p.upper[1][j] : j + 1};
+  const int nk[2] = {PLANES ? p.lower[2][k] : k, PLANES ? p.upper[2][k] : k + 1};
   double v = 0.0;
 #pragma unroll
   for (int q = 0; q < 8; ++q) {
     const int a = (q >> 2) & 1, b = (q >> 1) & 1, c = q & 1;
-    const double g = G[((long long)(i + a) * ny1 + (j + b)) * nz1 + (k + c)];
+    const double g = G[((long long)ni[a] * ny1 + nj[b]) * nz1 + nk[c]];
     v = ((a + b + c) & 1) ? v - g : v + g;
   }
   grad[cell] = 2.0 * v;
@@ -498,14 +502,20 @@ cudaError_t launch_comp_weights(int kind, int nmeas, const double *w_raw, const 
   return cudaGetLastError();
 }
 
-cudaError_t launch_adjoint_combine(const MeshView &m, int nchunk, int nblock, const double *Gpart,
-                                   double *G, double *grad, cudaStream_t st) {
-  const long long nn = m.nnodes();
+cudaError_t launch_adjoint_combine(const MeshView &m, const MeshView &nodes,
+                                   const NodePlanes *planes, int nchunk, int nblock,
+                                   const double *Gpart, double *G, double *grad, cudaStream_t st) {
+  const long long nn = nodes.nnodes();
+  const int blocks = cdiv(m.ngrid(), kThreads);
   for (int b = 0; b < nblock; ++b) {
     k_sum_chunks<<<cdiv(nn, kThreads), kThreads, 0, st>>>((int)nn, nchunk, nblock * nn,
                                                            Gpart + b * nn, G + b * nn);
-    k_adjoint_combine<<<cdiv(m.ngrid(), kThreads), kThreads, 0, st>>>(m, G + b * nn,
-                                                                      grad + b * m.ngrid());
+    if (planes)
+      k_adjoint_combine<true><<<blocks, kThreads, 0, st>>>(m, nodes, *planes, G + b * nn,
+                                                           grad + b * m.ngrid());
+    else
+      k_adjoint_combine<false><<<blocks, kThreads, 0, st>>>(m, nodes, NodePlanes{}, G + b * nn,
+                                                            grad + b * m.ngrid());
   }
   return cudaGetLastError();
 }

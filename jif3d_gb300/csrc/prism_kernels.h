@@ -25,12 +25,23 @@ struct StationView {
   const double *x, *y, *z;
 };
 
+// The node planes of a mesh whose corners are not all running sums of the
+// cell sizes: along each axis the distinct corner coordinates, lower and upper
+// corners of neighbouring cells apart where they differ (2 n planes at most).
+// lower_of / upper_of: the cell that a plane is the lower / upper corner of, or
+// -1; lower / upper: the planes of a cell.  The node kernels work on the planes
+// as on any node grid (a MeshView of them).
+struct NodePlanes {
+  const int *lower_of[3], *upper_of[3], *lower[3], *upper[3];
+};
+
 // Forward, node formulation:  per station and component
 //   U_c(s) = scale_c * sum_nodes F_c(s, node) * rho~(node)
 // rho~ = third mixed backward difference of the zero-padded model (one model
 // block; magnetisation runs it once per block into rho_t + block * nnodes).
-cudaError_t launch_rho_tilde(const MeshView &m, const double *rho, double *rho_t,
-                             cudaStream_t st);
+// nodes: the node grid, m itself or that of its planes.
+cudaError_t launch_rho_tilde(const MeshView &m, const MeshView &nodes, const NodePlanes *planes,
+                             const double *rho, double *rho_t, cudaStream_t st);
 // Split of the forward's work: blocks of `cols` node columns and `kper` nodes
 // of each (nblk = column blocks x nkc pieces of the columns, at most
 // max_blocks of them where more columns per block can see to that), spb
@@ -85,8 +96,9 @@ cudaError_t launch_node_adjoint(int kind, const MeshView &m, const StationView &
                                 const int *chunk_start, double *Gpart, cudaStream_t st);
 // grad[b * ngrid + cell] = 2 * sum_corners (-1)^shifts * sum_chunks
 // Gpart[chunk][b][node] for each model block b; G: nblock * nnodes scratch.
-cudaError_t launch_adjoint_combine(const MeshView &m, int nchunk, int nblock, const double *Gpart,
-                                   double *G, double *grad, cudaStream_t st);
+cudaError_t launch_adjoint_combine(const MeshView &m, const MeshView &nodes,
+                                   const NodePlanes *planes, int nchunk, int nblock,
+                                   const double *Gpart, double *G, double *grad, cudaStream_t st);
 // grad[ngrid + j] = 2 * sum_s sum_r w_raw[s][r] * bgsens[s][r][j]
 cudaError_t launch_background_grad(int kind, int nmeas, int nbg, const double *w_raw,
                                    const double *bgsens, double *grad_bg, cudaStream_t st);

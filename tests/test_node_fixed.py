@@ -177,3 +177,40 @@ def test_stored_pair_at_tile_edges(ctx, kind, shape):
     rows = rng.choice(J.shape[0], min(J.shape[0], 40), replace=False)
     g = ctx.batched_lqderivative(None, np.eye(J.shape[0])[rows])
     assert np.all(np.abs(g - 2.0 * J[rows]) <= 2 * 2 * bound[rows, None])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", [W.SCALAR, W.TENSOR, W.MAGNETIC, W.MAG_GRADIENT, W.MAGNETIZATION])
+@pytest.mark.parametrize("apart", ["none", "some", "all"])
+def test_planes_of_given_corners(ctx, oracle_lib, kind, apart):
+    """Corners given one by one, lower and upper corners of neighbouring cells
+    apart on no axis, on some planes, or on every plane (by a rounding step, by
+    a gap and by an overlap): forward, gradient, and the gradients of station
+    subsets against the oracle's eight corners per cell."""
+    import torch
+    s = _survey(kind, 6, 5, 4, 9, False)
+    co = [s.coords(a) for a in range(3)]
+    rng = np.random.default_rng(17)
+    for a in range(3):
+        inner = co[a][1:-1]
+        shift = np.array([1e-9, 0.3, -0.2])[np.arange(inner.size) % 3]
+        take = {"none": np.zeros(inner.size), "all": np.ones(inner.size),
+                "some": rng.integers(0, 2, inner.size)}[apart]
+        inner += take * shift
+    size = (s.xsize, s.ysize, s.zsize)
+    W.setup_context(ctx, s)
+    ctx.set_mesh(*co, *size)
+    p = oracle_lib.Problem(*co, *size, s.stations, kind=kind, inc=s.inc, dec=s.dec, fs=s.fs)
+    d = ctx.forward(s.model)
+    assert relerr(d, p.forward(s.model)) <= 1e-10
+    misfit = rng.normal(size=d.size)
+    assert relerr(ctx.lqderivative(s.model, misfit), p.lqderivative(s.model, misfit)) <= 1e-10
+    # subsets [0, 3) and [3, 9): their gradients add up to that of all stations
+    like = dict(dtype=torch.float64, device="cuda")
+    m, r = torch.tensor(s.model, **like), torch.tensor(misfit, **like)
+    g = torch.zeros(2, s.nparm, **like)
+    torch.cuda.synchronize()
+    ctx.subsets_lqderivative_device([np.arange(3), np.arange(3, 9)], m.data_ptr(), r.data_ptr(),
+                                    g.data_ptr())
+    ctx.synchronize()
+    assert relerr(g.sum(0).cpu().numpy(), p.lqderivative(s.model, misfit)) <= 1e-10
