@@ -66,7 +66,7 @@ struct j3g_context {
   // device copies of the geometry
   DevBuf dX, dY, dZ, dxs, dys, dzs, dbg, dsx, dsy, dsz;
   // scratch
-  DevBuf model, data, misfit, grad, rhot, partial, comps, bgsens, rawd, wraw, W, Gpart, G, F,
+  DevBuf model, data, misfit, grad, rhot, partial, bgsens, rawd, wraw, W, Gpart, F,
       rows, rowsum, probe;
 
   // device-resident sensitivity (j3g_build_sensitivity)
@@ -339,28 +339,27 @@ int ensure_background(j3g_context *c) {
   return J3G_OK;
 }
 
-// Gridded node-component sums comps[nmeas][NC_COUNT] for the model d_model.
-int gridded_node_forward(j3g_context *c, const double *d_model) {
+// The data by node sums: model differences, partial sums, data.
+int node_forward(j3g_context *c, const double *d_model, double *d_data, double *raw_out,
+                 const double *bgsens, const double *bgval) {
   const MeshView m = node_view(c);
-  const long long nn = m.nnodes();
   const int nblock = kind_nblock(c->kind);
-  J3G_TRY(ensure(c, c->rhot, sizeof(double) * nn * nblock));
-  for (int b = 0; b < nblock; ++b)
-    J3G_LAUNCH(c, launch_rho_tilde(mesh_view(c), m, node_planes(c), d_model + (size_t)b * c->ngrid(),
-                                   ptr<double>(c->rhot) + (size_t)b * nn, c->stream));
+  J3G_TRY(ensure(c, c->rhot, sizeof(double) * m.nnodes() * nblock));
   const NodeForwardPlan p =
       node_forward_plan(m.nx, m.ny, m.nz, c->nmeas, (1LL << 31) - 1);
-  const int nblk = p.nblk;
-  const int ncomp = kind_ncomp(c->kind);
-  J3G_TRY(ensure(c, c->partial, sizeof(double) * (size_t)nblk * c->nmeas * ncomp));
-  J3G_TRY(ensure(c, c->comps, sizeof(double) * (size_t)c->nmeas * NC_COUNT));
+  J3G_TRY(ensure(c, c->partial, sizeof(double) * (size_t)p.nblk * c->nmeas * kind_ncomp(c->kind)));
+  J3G_LAUNCH(c, launch_rho_tilde(mesh_view(c), m, node_planes(c), nblock, d_model,
+                                 ptr<double>(c->rhot), c->stream));
   {
     TimedScope ts(c, J3G_TIMER_NODE_FORWARD);
     J3G_LAUNCH(c, launch_node_forward(c->kind, m, station_view(c), ptr<double>(c->rhot),
                                       ptr<double>(c->partial), p, c->stream));
   }
-  J3G_LAUNCH(c, launch_forward_reduce(c->kind, c->nmeas, nblk, ptr<double>(c->partial),
-                                      mag_field(c), ptr<double>(c->comps), c->stream));
+  double tbx, tby, tbz;
+  tfa_dir(c, tbx, tby, tbz);
+  J3G_LAUNCH(c, launch_forward_finish(c->kind, c->transform, tbx, tby, tbz, c->nmeas, p.nblk,
+                                      ptr<double>(c->partial), bgsens, c->nbg_active(), bgval,
+                                      mag_field(c), raw_out, d_data, c->stream));
   return J3G_OK;
 }
 
@@ -437,24 +436,18 @@ int forward_device(j3g_context *c, const double *d_model, double *d_data, double
   const int nbg = c->nbg_active();
   const double *bgval = d_model + c->ngrid();
   const double *bgsens = nbg ? ptr<double>(c->bgsens) : nullptr;
-  // node sums per station: node components, or raw rows for the special kinds
-  const int comps_ld = kind_special(c->kind) ? c->raw() : NC_COUNT;
-  if (h_sens || (!c->node_path && c->ngrid() > 0)) {
+  if (c->ngrid() > 0 && c->node_path && !h_sens)
+    return node_forward(c, d_model, d_data, raw_out, bgsens, bgval);
+  // the gridded part from explicit sensitivities, or none
+  if (h_sens || c->ngrid() > 0) {
     J3G_TRY(gridded_rows_forward(c, d_model, h_sens));
-    J3G_LAUNCH(c, launch_assemble(c->kind, c->transform, tbx, tby, tbz, c->nmeas,
-                                ptr<double>(c->rowsum), c->raw(), bgsens, nbg, bgval,
-                                mag_field(c), raw_out, d_data, c->stream));
   } else {
-    if (c->ngrid() > 0) {
-      J3G_TRY(gridded_node_forward(c, d_model));
-    } else {
-      J3G_TRY(ensure(c, c->comps, sizeof(double) * (size_t)c->nmeas * NC_COUNT));
-      J3G_CUDA(c, cudaMemsetAsync(c->comps.p, 0, sizeof(double) * c->nmeas * NC_COUNT, c->stream));
-    }
-    J3G_LAUNCH(c, launch_assemble(c->kind, c->transform, tbx, tby, tbz, c->nmeas,
-                                ptr<double>(c->comps), comps_ld, bgsens, nbg, bgval, mag_field(c),
-                                raw_out, d_data, c->stream));
+    J3G_TRY(ensure(c, c->rowsum, sizeof(double) * (size_t)c->nmeas * c->raw()));
+    J3G_CUDA(c, cudaMemsetAsync(c->rowsum.p, 0, sizeof(double) * c->nmeas * c->raw(), c->stream));
   }
+  J3G_LAUNCH(c, launch_assemble(c->kind, c->transform, tbx, tby, tbz, c->nmeas,
+                                ptr<double>(c->rowsum), bgsens, nbg, bgval, raw_out, d_data,
+                                c->stream));
   return J3G_OK;
 }
 
@@ -488,60 +481,63 @@ int adjoint_device(j3g_context *c, const double *d_model, const double *d_misfit
     rawd = ptr<double>(c->rawd);
   }
   J3G_TRY(ensure(c, c->wraw, sizeof(double) * (size_t)c->nmeas * raw));
-  J3G_LAUNCH(c, launch_backproject(c->kind, c->transform, tbx, tby, tbz, c->nmeas, d_misfit, rawd,
-                                 ptr<double>(c->wraw), c->stream));
   MeshView m = mesh_view(c);
   StationView s = station_view(c);
   if (ngrid > 0 && c->node_path) {
     const MeshView nodes = node_view(c);
     J3G_TRY(ensure(c, c->W, sizeof(double) * (size_t)c->nmeas * std::max<int>(NC_COUNT, kMaxVc)));
-    J3G_LAUNCH(c, launch_comp_weights(c->kind, c->nmeas, ptr<double>(c->wraw), mag_field(c),
-                                    ptr<double>(c->W), c->stream));
+    J3G_LAUNCH(c, launch_node_weights(c->kind, c->transform, tbx, tby, tbz, c->nmeas, d_misfit,
+                                      rawd, mag_field(c), ptr<double>(c->wraw), ptr<double>(c->W),
+                                      c->stream));
     const long long nn = nodes.nnodes();
     const NodeAdjointPlan plan =
         node_adjoint_plan(nodes.nx, nodes.ny, nodes.nz, nblock, c->nmeas);
     const int spc = plan.spc;
     int nchunk = plan.nchunk;
-    // chunks of at most spc stations that never straddle a subset
-    std::vector<int> starts, first_chunk;
-    const int *d_starts = nullptr;
+    // chunks of at most spc stations that never straddle a subset, and each
+    // subset's first chunk
+    std::vector<int> table;
+    const int *d_starts = nullptr, *d_first = nullptr;
+    int most = nchunk;  // chunks of a subset
     if (sub) {
+      std::vector<int> first;
+      most = 0;
       for (int k = 0; k < nsub; ++k) {
-        first_chunk.push_back((int)starts.size());
-        for (int a = off[k]; a < off[k + 1]; a += spc) starts.push_back(a);
+        first.push_back((int)table.size());
+        for (int a = off[k]; a < off[k + 1]; a += spc) table.push_back(a);
+        most = std::max(most, (int)table.size() - first.back());
       }
-      first_chunk.push_back((int)starts.size());
-      starts.push_back(c->nmeas);
-      nchunk = (int)starts.size() - 1;
+      nchunk = (int)table.size();
+      first.push_back(nchunk);
+      table.push_back(c->nmeas);
+      table.insert(table.end(), first.begin(), first.end());
       // uploaded only when the subsets' chunk layout changes: a repeated call
       // on the same subsets queues kernels only (and can be graph-captured)
-      if (starts != c->chunks_h) {
-        J3G_TRY(ensure(c, c->chunks, sizeof(int) * starts.size()));
-        J3G_CUDA(c, cudaMemcpyAsync(c->chunks.p, starts.data(), sizeof(int) * starts.size(),
+      if (table != c->chunks_h) {
+        J3G_TRY(ensure(c, c->chunks, sizeof(int) * table.size()));
+        J3G_CUDA(c, cudaMemcpyAsync(c->chunks.p, table.data(), sizeof(int) * table.size(),
                                     cudaMemcpyHostToDevice, c->stream));
         J3G_CUDA(c, cudaStreamSynchronize(c->stream));  // the host table is a local
-        c->chunks_h = starts;
+        c->chunks_h = table;
       }
       d_starts = ptr<int>(c->chunks);
-    } else {
-      first_chunk = {0, nchunk};
+      d_first = d_starts + nchunk + 1;
     }
     J3G_TRY(ensure(c, c->Gpart, sizeof(double) * (size_t)std::max(nchunk, 1) * nblock * nn));
-    J3G_TRY(ensure(c, c->G, sizeof(double) * (size_t)nblock * nn));
     if (nchunk > 0) {
       TimedScope ts(c, J3G_TIMER_NODE_ADJOINT);
       J3G_LAUNCH(c, launch_node_adjoint(c->kind, nodes, s, ptr<double>(c->W), plan, nchunk, d_starts,
                                         ptr<double>(c->Gpart), c->stream));
     }
-    for (int k = 0; k < nsub; ++k) {
-      const int c0 = first_chunk[k], nk = first_chunk[k + 1] - c0;
-      J3G_LAUNCH(c, launch_adjoint_combine(m, nodes, node_planes(c), nk, nblock,
-                                           ptr<double>(c->Gpart) + (size_t)c0 * nblock * nn,
-                                           ptr<double>(c->G), d_grad + (size_t)k * nparm,
-                                           c->stream));
-      c->launches += 2 * nblock - 1;  // chunk sum + cell combine per block
-    }
-  } else if (ngrid > 0) {
+    int queued = 0;
+    J3G_CUDA(c, launch_adjoint_finish(m, nodes, node_planes(c), nblock, nsub, d_first, most, nparm,
+                                      ptr<double>(c->Gpart), d_grad, c->stream, &queued));
+    c->launches += queued;
+  } else {
+    J3G_LAUNCH(c, launch_backproject(c->kind, c->transform, tbx, tby, tbz, c->nmeas, d_misfit, rawd,
+                                     ptr<double>(c->wraw), c->stream));
+  }
+  if (ngrid > 0 && !c->node_path) {
     // eight-corner rows, accumulated chunk by chunk within each subset
     const int chunk = row_chunk(c, ncolg);
     J3G_TRY(ensure(c, c->rows, sizeof(double) * (size_t)chunk * raw * ncolg));
@@ -1198,8 +1194,8 @@ int j3g_destroy(j3g_context *c) {
   cudaStreamSynchronize(c->stream);
   DevBuf *bufs[] = {&c->dplanes, &c->dplane_maps, &c->dX, &c->dY, &c->dZ, &c->dxs, &c->dys, &c->dzs, &c->dbg, &c->dsx,
                     &c->dsy, &c->dsz, &c->model, &c->data, &c->misfit, &c->grad, &c->rhot,
-                    &c->partial, &c->comps, &c->bgsens, &c->rawd, &c->wraw, &c->W, &c->Gpart,
-                    &c->G, &c->F, &c->rows, &c->rowsum, &c->probe, &c->J32, &c->Jhi,
+                    &c->partial, &c->bgsens, &c->rawd, &c->wraw, &c->W, &c->Gpart,
+                    &c->F, &c->rows, &c->rowsum, &c->probe, &c->J32, &c->Jhi,
                     &c->Jlo, &c->JThi, &c->JTlo, &c->rowscale, &c->x32, &c->sums, &c->part,
                     &c->Bhi, &c->Blo, &c->P, &c->wst, &c->wrawb, &c->rawb, &c->gerr,
                     &c->mscale, &c->Jrowsum, &c->rowmax, &c->mmean, &c->swork, &c->sexp, &c->chunks, &c->rmaps,

@@ -129,13 +129,11 @@ extern "C" int j3g_forward_noalloc(int kind, int nx, int ny, int nz, const doubl
   // every scratch value read below is written first in the same call, so no
   // clearing is needed: rho~ covers all nodes, the partials all (block,
   // station, component) triples and the sums all (station, component) pairs
-  if (launch_rho_tilde(m, m, nullptr, d_model, rho_t, st) != cudaSuccess) return J3G_ERR_CUDA;
+  if (launch_rho_tilde(m, m, nullptr, 1, d_model, rho_t, st) != cudaSuccess) return J3G_ERR_CUDA;
   if (launch_node_forward(kind, m, s, rho_t, partial, plan, st) != cudaSuccess)
     return J3G_ERR_CUDA;
-  if (launch_forward_reduce(kind, nmeas, plan.nblk, partial, mf, comps, st) != cudaSuccess)
-    return J3G_ERR_CUDA;
-  if (launch_assemble(kind, TR_NONE, 0.0, 0.0, 0.0, nmeas, comps, NC_COUNT, nullptr, 0, nullptr,
-                      mf, nullptr, d_data, st) != cudaSuccess)
+  if (launch_forward_finish(kind, TR_NONE, 0.0, 0.0, 0.0, nmeas, plan.nblk, partial, nullptr, 0,
+                            nullptr, mf, nullptr, d_data, st) != cudaSuccess)
     return J3G_ERR_CUDA;
   return J3G_OK;
 }

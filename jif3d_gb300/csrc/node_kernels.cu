@@ -14,6 +14,7 @@
 // busy each and the schedulers issue in 60 % of the cycles.
 #include <algorithm>
 
+#include "chained.cuh"
 #include "node_column.cuh"
 #include "prism_kernels.h"
 
@@ -35,9 +36,13 @@ template <bool PLANES>
 __global__ void __launch_bounds__(kNodeThreads)
     k_rho_tilde(MeshView m, MeshView nodes, NodePlanes p, const double *__restrict__ rho,
                 double *__restrict__ rt) {
+  chain_begin();
+  chain_wait();
   const int ny1 = nodes.ny + 1, ncol = (nodes.nx + 1) * ny1;
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= ncol * (nodes.nz + 1)) return;
+  rho += blockIdx.y * m.ngrid();
+  rt += blockIdx.y * nodes.nnodes();
   const int k = n / ncol, col = n - k * ncol, i = col / ny1, j = col - i * ny1;
   const int ci[2] = {PLANES ? p.lower_of[0][i] : i, PLANES ? p.upper_of[0][i] : i - 1};
   const int cj[2] = {PLANES ? p.lower_of[1][j] : j, PLANES ? p.upper_of[1][j] : j - 1};
@@ -76,7 +81,9 @@ __global__ void __launch_bounds__(kNodeThreads, kNodeResident)
   const int c0 = cb * cols, c1 = min(ncol, c0 + cols);
   const int s0 = blockIdx.y * spb, s1 = min(st.n, s0 + spb);
   const int tid = threadIdx.x, nt = blockDim.x;
-  tab.set(tid, nt);
+  chain_begin();
+  tab.set(tid, nt);  // constant, so before the wait
+  chain_wait();
   for (int s = s0; s < s1; ++s) {
     const double mx = st.x[s], my = st.y[s], mz = st.z[s];
     double acc[NCMP];
@@ -183,13 +190,15 @@ __global__ void __launch_bounds__(kNodeThreads, kNodeResident)
   const int c0 = cb * nt, col = c0 + tid;
   const bool live = col < ncol;
   const int i = live ? col / ny1 : 0, j = live ? col - i * ny1 : 0;
+  chain_begin();
+  tab.set(tid, nt);  // constant, so before the wait
+  chain_wait();
   const double X = m.X[i], Y = m.Y[j];
   // stations of this chunk: spc apiece, or the ranges of chunk_start (chunks
   // that never straddle a station subset)
   const int chunk = blockIdx.y;
   const int s0 = chunk_start ? chunk_start[chunk] : chunk * spc;
   const int s1 = chunk_start ? chunk_start[chunk + 1] : min(st.n, s0 + spc);
-  tab.set(tid, nt);
   for (int k = 0; k < nk; ++k)
 #pragma unroll
     for (int b = 0; b < T::nblock; ++b) acc[(b * kper + k) * nt + tid] = 0.0;
@@ -275,8 +284,8 @@ inline int cdiv(long long a, long long b) { return (int)((a + b - 1) / b); }
 
 int column_threads(int ncol) { return std::min(kNodeThreads, (ncol + 31) / 32 * 32); }
 
-// Blocks that fill the GPU a few times over.
-constexpr long long kNodeBlocks = 152 * kNodeResident * 3;
+// Blocks that the GPU holds at a time.
+constexpr double kNodeSlots = 152.0 * kNodeResident;
 
 }  // namespace
 
@@ -285,22 +294,32 @@ NodeForwardPlan node_forward_plan(int nx, int ny, int nz, int nmeas, long long m
   const int ncol = (nx + 1) * (ny + 1), nz1 = nz + 1;
   p.threads = column_threads(ncol);
   p.cols = p.threads;
-  p.nkc = 1;
-  p.kper = nz1;
-  p.spb = 8;
+  // The split with the least of (blocks / slots) * busy + 0.45 * alone, in the
+  // time of one node: busy what a block of spb stations and kper nodes costs the
+  // SMs, alone how long it takes, its tables' latency included, which is what
+  // the first and last blocks add.  Fitted to sweeps over eight meshes of 605 to
+  // 52,000 nodes with 16 to 1200 stations, where it is within 5 % of the best
+  // split (fixed thresholds on the number of blocks lost up to a quarter there).
+  double best = 0.0;
+  for (int spb = 8; spb > 0; spb >>= 1)
+    for (int n = 1; n <= std::min(nz1, 64); ++n) {
+      const int kper = cdiv(nz1, n), nkc = cdiv(nz1, kper);
+      const double blocks = (double)cdiv(ncol, p.cols) * nkc * cdiv(nmeas, spb);
+      const double cost = blocks / kNodeSlots * (1.5 + spb * (1.5 + kper)) +
+                          0.45 * (10.0 + spb * (3.0 + kper));
+      if (best != 0.0 && cost >= best) continue;
+      best = cost;
+      p.spb = spb;
+      p.kper = kper;
+      p.nkc = nkc;
+    }
   auto blocks = [&]() {
     return (long long)cdiv(ncol, p.cols) * p.nkc * cdiv(nmeas, p.spb);
   };
-  // few blocks: fewer stations each, then shorter pieces of the columns
-  while (p.spb > 1 && blocks() < kNodeBlocks) p.spb >>= 1;
-  while (p.kper > 1 && blocks() < kNodeBlocks) {
-    p.kper = (p.kper + 1) / 2;
-    p.nkc = cdiv(nz1, p.kper);
-  }
   // short columns on many blocks: several columns per thread share a block's
   // station setup and sums
   while (p.cols < 8 * p.threads && (long long)p.kper * p.cols < 16LL * p.threads &&
-         blocks() >= 4 * kNodeBlocks)
+         blocks() >= 12 * kNodeSlots)
     p.cols += p.threads;
   // within the caller's room for partial sums
   if ((long long)cdiv(ncol, p.cols) * p.nkc > max_blocks) {
@@ -324,9 +343,8 @@ static cudaError_t adjoint_launch(dim3 grid, int threads, size_t smem, cudaStrea
         k_node_adjoint<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  k_node_adjoint<KIND><<<grid, threads, smem, st>>>(m, s, W, p.kper, p.nkc, p.spc, chunk_start,
-                                                    Gpart);
-  return cudaGetLastError();
+  return launch_chained(k_node_adjoint<KIND>, grid, threads, smem, st, m, s, W, p.kper, p.nkc,
+                        p.spc, chunk_start, Gpart);
 }
 
 #define J3G_NODE_DISPATCH(kind, ...)                                             \
@@ -341,22 +359,20 @@ static cudaError_t adjoint_launch(dim3 grid, int threads, size_t smem, cudaStrea
   }
 
 cudaError_t launch_rho_tilde(const MeshView &m, const MeshView &nodes, const NodePlanes *planes,
-                             const double *rho, double *rho_t, cudaStream_t st) {
-  const int blocks = cdiv(nodes.nnodes(), kNodeThreads);
-  if (planes)
-    k_rho_tilde<true><<<blocks, kNodeThreads, 0, st>>>(m, nodes, *planes, rho, rho_t);
-  else
-    k_rho_tilde<false><<<blocks, kNodeThreads, 0, st>>>(m, nodes, NodePlanes{}, rho, rho_t);
-  return cudaGetLastError();
+                             int nblock, const double *rho, double *rho_t, cudaStream_t st) {
+  const dim3 grid(cdiv(nodes.nnodes(), kNodeThreads), nblock);
+  return planes ? launch_chained(k_rho_tilde<true>, grid, kNodeThreads, 0, st, m, nodes, *planes,
+                                 rho, rho_t)
+                : launch_chained(k_rho_tilde<false>, grid, kNodeThreads, 0, st, m, nodes,
+                                 NodePlanes{}, rho, rho_t);
 }
 
 cudaError_t launch_node_forward(int kind, const MeshView &m, const StationView &s,
                                 const double *rho_t, double *partial, const NodeForwardPlan &p,
                                 cudaStream_t st) {
   const dim3 grid(p.nblk, cdiv(s.n, p.spb));
-  J3G_NODE_DISPATCH(kind, (k_node_forward<K><<<grid, p.threads, 0, st>>>(
-                              m, s, rho_t, partial, p.cols, p.kper, p.nkc, p.spb)));
-  return cudaGetLastError();
+  J3G_NODE_DISPATCH(kind, return launch_chained(k_node_forward<K>, grid, p.threads, 0, st, m, s,
+                                                rho_t, partial, p.cols, p.kper, p.nkc, p.spb));
 }
 
 NodeAdjointPlan node_adjoint_plan(int nx, int ny, int nz, int nblock, int nmeas) {
@@ -366,20 +382,36 @@ NodeAdjointPlan node_adjoint_plan(int nx, int ny, int nz, int nblock, int nmeas)
   const int ncb = cdiv(ncol, p.threads);
   p.nkc = cdiv(nz1, kAdjNodes);
   p.kper = cdiv(nz1, p.nkc);
-  // Chunks of 64 stations: short enough that the rounding of a node's running
-  // sum stays small (a survey's chunks are added up afterwards), long enough
-  // that a block's setup does not count.  Surveys that leave SMs idle take
-  // shorter pieces of the columns, then shorter chunks.
-  p.spc = 64;
-  auto blocks = [&]() { return (long long)ncb * p.nkc * cdiv(nmeas, p.spc); };
-  while (p.spc > 16 && blocks() < kNodeBlocks / 2) p.spc >>= 1;
-  while (p.kper > 1 && blocks() < kNodeBlocks / 2) {
-    p.kper = (p.kper + 1) / 2;
-    p.nkc = cdiv(nz1, p.kper);
+  // Chunks of 16 stations: a block's setup costs about four of its nodes, a
+  // few per cent of its time, and six rounds of blocks or more end together (64
+  // stations to a block: the last round's blocks ran on alone, magnetics on
+  // 48 x 48 x 24 cells and 1024 stations 2.19 ms to 1.86).  The same for every
+  // survey with blocks enough, so that a station subset alone and within a batch
+  // is summed in the same order.
+  p.spc = 16;
+  // fewer blocks than four rounds: the split with the least of
+  // (rounds + 0.9) * time of a block, as for the forward
+  const int resident = std::min<long long>(
+      kNodeResident, (227 << 10) / ((25 << 10) + 8LL * nblock * p.kper * p.threads));
+  if ((double)ncb * p.nkc * cdiv(nmeas, p.spc) < 4.0 * 152 * resident) {
+    double best = 0.0;
+    for (int spc : {16, 8, 6, 4, 3, 2, 1})
+      for (int n = cdiv(nz1, kAdjNodes); n <= std::min(nz1, 64); ++n) {
+        const int kper = cdiv(nz1, n), nkc = cdiv(nz1, kper);
+        if (kper > kAdjNodes) continue;
+        const int fit = std::min<long long>(
+            kNodeResident, (227 << 10) / ((25 << 10) + 8LL * nblock * kper * p.threads));
+        const double rounds = (double)ncb * nkc * cdiv(nmeas, spc) / (152.0 * fit);
+        const double cost = (rounds + 0.9) * (6.0 + spc * (1.5 + kper));
+        if (best != 0.0 && cost >= best) continue;
+        best = cost;
+        p.spc = spc;
+        p.kper = kper;
+        p.nkc = nkc;
+      }
   }
-  while (p.spc > 1 && blocks() < kNodeBlocks / 6) p.spc >>= 1;
-  // the chunks' sums within 512 MB
-  const long long room = std::max(1LL, (512LL << 20) / (8LL * nblock * ncol * nz1));
+  // the chunks' sums within 1 GB
+  const long long room = std::max(1LL, (1LL << 30) / (8LL * nblock * ncol * nz1));
   p.spc = std::max<long long>(p.spc, (nmeas + room - 1) / room);
   p.nchunk = cdiv(nmeas, p.spc);
   return p;

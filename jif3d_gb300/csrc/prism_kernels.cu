@@ -14,6 +14,7 @@
 // stations in one launch and the reduction with the model on the device.
 //
 // All reductions have a fixed order, so results repeat bit for bit.
+#include "chained.cuh"
 #include "prism_kernels.h"
 
 namespace j3g {
@@ -22,58 +23,10 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 
-__device__ __forceinline__ void decode_node(int n, int ny1, int nz1, int &i, int &j, int &k) {
-  k = n % nz1;
-  const int t = n / nz1;
-  j = t % ny1;
-  i = t / ny1;
-}
-
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
   return v;
-}
-
-template <int KIND> struct Slots {
-  static constexpr int off = (KIND == KIND_SCALAR || KIND == KIND_JOINT) ? 0 : 1;
-};
-
-template <int KIND>
-__global__ void k_forward_reduce(int nmeas, int nblk, const double *__restrict__ partial,
-                                 double *__restrict__ comps) {
-  constexpr int NCMP = KindTraits<KIND>::ncomp;
-  constexpr int OFF = Slots<KIND>::off;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nmeas * NC_COUNT) return;
-  const int s = t / NC_COUNT, c = t % NC_COUNT;
-  const int q = c - OFF;
-  double v = 0.0;
-  if (q >= 0 && q < NCMP && (KindTraits<KIND>::mask & (1 << c))) {
-    for (int b = 0; b < nblk; ++b) v += partial[((long long)b * nmeas + s) * NCMP + q];
-    v *= comp_scale(c);
-  }
-  comps[t] = v;
-}
-
-// The special kinds: virtual components straight to raw rows[nmeas][raw].
-template <int KIND>
-__global__ void k_forward_reduce_raw(int nmeas, int nblk, const double *__restrict__ partial,
-                                     MagField mf, double *__restrict__ rawrows) {
-  using T = KindTraits<KIND>;
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nmeas) return;
-  double v[kMaxVc];
-#pragma unroll
-  for (int q = 0; q < T::ncomp; ++q) {
-    double a = 0.0;
-    for (int b = 0; b < nblk; ++b) a += partial[((long long)b * nmeas + s) * T::ncomp + q];
-    v[q] = a * comp_scale(T::comp(q));
-  }
-  double raw[3];
-  raw_from_vc(KIND, v, mf, raw);
-#pragma unroll
-  for (int r = 0; r < T::raw; ++r) rawrows[(long long)s * T::raw + r] = raw[r];
 }
 
 // ---------------------------------------------------------------------------
@@ -166,69 +119,114 @@ __global__ void __launch_bounds__(256) k_background(StationView st, int nbg,
 }
 
 // ---------------------------------------------------------------------------
-__device__ double apply_transform(int transform, const double *raw, double bx, double by,
-                                  double bz) {
-  switch (transform) {
-    case TR_FTG_INVARIANT:  // Gravity/GravityTransforms.h:33-37
+template <int RAW>
+__device__ __forceinline__ double apply_transform(int transform, const double *raw, double bx,
+                                                  double by, double bz) {
+  if constexpr (RAW >= 9) {
+    if (transform == TR_FTG_INVARIANT)  // Gravity/GravityTransforms.h:33-37
       return sub(sub(sub(add(add(mul(raw[0], raw[4]), mul(raw[4], raw[8])), mul(raw[0], raw[8])),
                          mul(raw[3], raw[1])),
                      mul(raw[7], raw[5])),
                  mul(raw[2], raw[6]));
-    case TR_TOTAL_FIELD:  // Magnetics/MagneticTransforms.h:27-30
-      return sqrt(add(add(mul(raw[0], raw[0]), mul(raw[1], raw[1])), mul(raw[2], raw[2])));
-    case TR_TFA:  // Magnetics/MagneticTransforms.h:122-129
-      return add(add(mul(bx, raw[0]), mul(by, raw[1])), mul(bz, raw[2]));
-    default:
-      return raw[0];
   }
+  if constexpr (RAW >= 3) {
+    if (transform == TR_TOTAL_FIELD)  // Magnetics/MagneticTransforms.h:27-30
+      return sqrt(add(add(mul(raw[0], raw[0]), mul(raw[1], raw[1])), mul(raw[2], raw[2])));
+    if (transform == TR_TFA)  // Magnetics/MagneticTransforms.h:122-129
+      return add(add(mul(bx, raw[0]), mul(by, raw[1])), mul(bz, raw[2]));
+  }
+  return raw[0];
 }
 
-__global__ void k_assemble(int kind, int transform, double tbx, double tby, double tbz,
-                           int nmeas, const double *__restrict__ comps, int comps_ld,
-                           const double *__restrict__ bgsens, int nbg,
-                           const double *__restrict__ bgval, MagField mf,
-                           double *__restrict__ raw_out, double *__restrict__ data_out) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nmeas) return;
-  const int raw = kind_raw(kind);
-  double r[10];
-  if (comps_ld == NC_COUNT) {
-    double u[NC_COUNT];
-    for (int c = 0; c < NC_COUNT; ++c) u[c] = comps[(long long)s * NC_COUNT + c];
-    raw_from_comps(kind, u, mf, r);
-  } else {  // comps already hold raw gridded rows
-    for (int c = 0; c < raw; ++c) r[c] = comps[(long long)s * comps_ld + c];
-  }
-  for (int c = 0; c < raw; ++c) {
+// A station's raw rows plus background, and their transform, out.
+template <int RAW>
+__device__ __forceinline__ void finish_station(int transform, double tbx, double tby, double tbz,
+                                               int s, double *r, const double *__restrict__ bgsens,
+                                               int nbg, const double *__restrict__ bgval,
+                                               double *__restrict__ raw_out,
+                                               double *__restrict__ data_out) {
+#pragma unroll
+  for (int c = 0; c < RAW; ++c) {
     double bg = 0.0;
     for (int j = 0; j < nbg; ++j)
-      bg = add(bg, mul(bgsens[((long long)s * raw + c) * nbg + j], bgval[j]));
+      bg = add(bg, mul(bgsens[((long long)s * RAW + c) * nbg + j], bgval[j]));
     r[c] = add(r[c], bg);
-    if (raw_out) raw_out[(long long)s * raw + c] = r[c];
+    if (raw_out) raw_out[(long long)s * RAW + c] = r[c];
   }
   if (transform == TR_NONE) {
-    for (int c = 0; c < raw; ++c) data_out[(long long)s * raw + c] = r[c];
+#pragma unroll
+    for (int c = 0; c < RAW; ++c) data_out[(long long)s * RAW + c] = r[c];
   } else {
-    data_out[s] = apply_transform(transform, r, tbx, tby, tbz);
+    data_out[s] = apply_transform<RAW>(transform, r, tbx, tby, tbz);
   }
 }
 
-// w_raw = misfit * dT/draw (GravityTransforms.h:72-93, MagneticTransforms.h:65-75,136-145);
-// without a transform the misfit is the raw weight.
-__global__ void k_backproject(int kind, int transform, double tbx, double tby, double tbz,
-                              int nmeas, const double *__restrict__ misfit,
-                              const double *__restrict__ rawd, double *__restrict__ w_raw) {
+template <int RAW>
+__global__ void k_assemble(int transform, double tbx, double tby, double tbz, int nmeas,
+                           const double *__restrict__ rows, const double *__restrict__ bgsens,
+                           int nbg, const double *__restrict__ bgval, double *__restrict__ raw_out,
+                           double *__restrict__ data_out) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nmeas) return;
-  const int raw = kind_raw(kind);
+  double r[RAW];
+#pragma unroll
+  for (int c = 0; c < RAW; ++c) r[c] = rows[(long long)s * RAW + c];
+  finish_station<RAW>(transform, tbx, tby, tbz, s, r, bgsens, nbg, bgval, raw_out, data_out);
+}
+
+// The end of a node-path forward: a station's partial sums added up in block
+// order (16 lanes to a station, one per component), then its raw rows,
+// background and transform as in k_assemble.  One launch instead of two, and
+// the sums' loads side by side: magnetisation over 14 blocks 15.3 + 3.6 -> 5 us.
+constexpr int kFinishStations = kThreads / 16;
+template <int KIND>
+__global__ void __launch_bounds__(kThreads)
+    k_forward_finish(int transform, double tbx, double tby, double tbz, int nmeas, int nblk,
+                     const double *__restrict__ partial, const double *__restrict__ bgsens,
+                     int nbg, const double *__restrict__ bgval, MagField mf,
+                     double *__restrict__ raw_out, double *__restrict__ data_out) {
+  using T = KindTraits<KIND>;
+  __shared__ double sum[kFinishStations][T::ncomp];
+  chain_begin();
+  chain_wait();
+  const int li = threadIdx.x / 16, q = threadIdx.x % 16;
+  const int s = blockIdx.x * kFinishStations + li;
+  if (s < nmeas && q < T::ncomp) {
+    const double *p = partial + (long long)s * T::ncomp + q;
+    const long long step = (long long)nmeas * T::ncomp;
+    double v = 0.0;
+#pragma unroll 8
+    for (int b = 0; b < nblk; ++b) v += p[b * step];
+    sum[li][q] = v * comp_scale(T::comp(q));
+  }
+  __syncwarp();  // a station's lanes are in one warp
+  if (s >= nmeas || q != 0) return;
+  double r[T::raw];
+  if constexpr (T::special) {
+    raw_from_vc(KIND, sum[li], mf, r);
+  } else {
+    double u[NC_COUNT];
+#pragma unroll
+    for (int c = 0; c < T::ncomp; ++c) u[T::comp(c)] = sum[li][c];
+    raw_from_comps(KIND, u, mf, r);
+  }
+  finish_station<T::raw>(transform, tbx, tby, tbz, s, r, bgsens, nbg, bgval, raw_out, data_out);
+}
+
+// w = misfit * dT/draw (GravityTransforms.h:72-93, MagneticTransforms.h:65-75,136-145);
+// without a transform the misfit is the raw weight.
+template <int RAW>
+__device__ __forceinline__ void backproject(int transform, double tbx, double tby, double tbz,
+                                            const double *__restrict__ misfit,
+                                            const double *__restrict__ rawd, int s, double *w) {
   if (transform == TR_NONE) {
-    for (int c = 0; c < raw; ++c) w_raw[(long long)s * raw + c] = misfit[(long long)s * raw + c];
+#pragma unroll
+    for (int c = 0; c < RAW; ++c) w[c] = misfit[(long long)s * RAW + c];
     return;
   }
   const double m = misfit[s];
-  const double *d = rawd + (long long)s * raw;
-  double *w = w_raw + (long long)s * raw;
-  if (transform == TR_FTG_INVARIANT) {
+  const double *d = rawd + (long long)s * RAW;
+  if constexpr (RAW == 9) {  // the FTG invariant
     w[0] = mul(m, add(d[4], d[8]));
     w[1] = mul(m, -d[3]);
     w[2] = mul(m, -d[6]);
@@ -238,72 +236,157 @@ __global__ void k_backproject(int kind, int transform, double tbx, double tby, d
     w[6] = mul(m, -d[2]);
     w[7] = mul(m, -d[5]);
     w[8] = mul(m, add(d[0], d[4]));
-  } else if (transform == TR_TOTAL_FIELD) {
-    const double t = sqrt(add(add(mul(d[0], d[0]), mul(d[1], d[1])), mul(d[2], d[2])));
-    for (int c = 0; c < 3; ++c) w[c] = mul(m, d[c] / t);
-  } else {  // TFA
-    w[0] = mul(m, tbx);
-    w[1] = mul(m, tby);
-    w[2] = mul(m, tbz);
+  }
+  if constexpr (RAW == 3) {
+    if (transform == TR_TOTAL_FIELD) {
+      const double t = sqrt(add(add(mul(d[0], d[0]), mul(d[1], d[1])), mul(d[2], d[2])));
+#pragma unroll
+      for (int c = 0; c < 3; ++c) w[c] = mul(m, d[c] / t);
+    } else {  // TFA
+      w[0] = mul(m, tbx);
+      w[1] = mul(m, tby);
+      w[2] = mul(m, tbz);
+    }
   }
 }
 
-__global__ void k_comp_weights(int kind, int nmeas, const double *__restrict__ w_raw, MagField mf,
-                               double *__restrict__ W) {
+template <int RAW>
+__global__ void k_backproject(int transform, double tbx, double tby, double tbz, int nmeas,
+                              const double *__restrict__ misfit, const double *__restrict__ rawd,
+                              double *__restrict__ w_raw) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nmeas) return;
-  const int raw = kind_raw(kind);
-  double w[10];
-  for (int c = 0; c < raw; ++c) w[c] = w_raw[(long long)s * raw + c];
-  if (kind_special(kind)) {  // virtual-component weights [nmeas][ncomp]
-    const int nv = kind_ncomp(kind);
-    double u[kMaxVc];
-    vc_from_raw_weights(kind, w, mf, u);
-    for (int q = 0; q < nv; ++q)
-      W[(long long)s * nv + q] = u[q] * comp_scale(vc_comp(kind, q));
-    return;
+  double w[RAW];
+  backproject<RAW>(transform, tbx, tby, tbz, misfit, rawd, s, w);
+#pragma unroll
+  for (int c = 0; c < RAW; ++c) w_raw[(long long)s * RAW + c] = w[c];
+}
+
+// The weights of a node-path adjoint: k_backproject's raw weights (kept for the
+// background) and from them the weights of the node components, W
+// [nmeas][NC_COUNT], or [nmeas][ncomp] for the special kinds.
+template <int KIND>
+__global__ void __launch_bounds__(128)
+    k_node_weights(int transform, double tbx, double tby, double tbz, int nmeas,
+                   const double *__restrict__ misfit, const double *__restrict__ rawd, MagField mf,
+                   double *__restrict__ w_raw, double *__restrict__ W) {
+  using T = KindTraits<KIND>;
+  chain_begin();
+  chain_wait();
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= nmeas) return;
+  double w[T::raw];
+  backproject<T::raw>(transform, tbx, tby, tbz, misfit, rawd, s, w);
+#pragma unroll
+  for (int c = 0; c < T::raw; ++c) w_raw[(long long)s * T::raw + c] = w[c];
+  if constexpr (T::special) {
+    double u[T::ncomp];
+    vc_from_raw_weights(KIND, w, mf, u);
+#pragma unroll
+    for (int q = 0; q < T::ncomp; ++q)
+      W[(long long)s * T::ncomp + q] = u[q] * comp_scale(T::comp(q));
+  } else {
+    double u[NC_COUNT];
+    comps_from_raw_weights(KIND, w, mf, u);
+#pragma unroll
+    for (int c = 0; c < NC_COUNT; ++c) W[(long long)s * NC_COUNT + c] = u[c] * comp_scale(c);
   }
-  double u[NC_COUNT];
-  comps_from_raw_weights(kind, w, mf, u);
-  for (int c = 0; c < NC_COUNT; ++c) W[(long long)s * NC_COUNT + c] = u[c] * comp_scale(c);
 }
 
-// G[n] = sum_c Gpart[c * stride + n] (stride = blocks x nodes per chunk).
-__global__ void k_sum_chunks(int nn, int nchunk, long long stride,
-                             const double *__restrict__ Gpart, double *__restrict__ G) {
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= nn) return;
+// Chunks of the station subset blockIdx.z (all of them without a table).
+__device__ __forceinline__ int subset_chunks(const int *first_chunk, int sub, int nchunk,
+                                             int &first) {
+  first = first_chunk ? first_chunk[sub] : 0;
+  return first_chunk ? first_chunk[sub + 1] - first : nchunk;
+}
+
+// Groups of `group` chunks added up in place, each into its first chunk (block
+// y one group of every subset z): chunks in order, a few loads in flight.
+__global__ void __launch_bounds__(kThreads)
+    k_sum_groups(long long len, const int *__restrict__ first_chunk, int sub0, int nchunk,
+                 int group, double *__restrict__ Gpart) {
+  chain_begin();
+  chain_wait();
+  const long long n = (long long)blockIdx.x * kThreads + threadIdx.x;
+  int first;
+  const int nk = subset_chunks(first_chunk, sub0 + blockIdx.z, nchunk, first);
+  const int c0 = blockIdx.y * group, c1 = min(nk, c0 + group);
+  if (n >= len || c1 - c0 < 2) return;
+  double *g = Gpart + (first + c0) * len + n;
   double v = 0.0;
-  for (int c = 0; c < nchunk; ++c) v += Gpart[(long long)c * stride + n];
-  G[n] = v;
+#pragma unroll 8
+  for (int c = 0; c < c1 - c0; ++c) v += g[c * len];
+  *g = v;
 }
 
-// grad(cell) = 2 * sum_{a,b,c} (-1)^(a+b+c) G(corner a, b, c of the cell)
+// grad(cell) = 2 * sum_{a,b,c} (-1)^(a+b+c) G(corner a, b, c of the cell), G
+// the sum of the chunks (or of the first of every `group`).  A block sums the
+// nodes of a tile of cells into shared memory and combines them from there;
+// block y is the model block, z the station subset.  The chunk sums through
+// memory and a combine kernel of their own took two launches per model block
+// and subset, 4 to 5 us each.
+constexpr int kTileX = 2, kTileY = 4, kTileZ = 16;  // cells of a block: 1.99 node sums per cell
 template <bool PLANES>
-__global__ void k_adjoint_combine(MeshView m, MeshView nodes, NodePlanes p,
-                                  const double *__restrict__ G, double *__restrict__ grad) {
-  const long long cell = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (cell >= m.ngrid()) return;
-  const int k = cell % m.nz;
-  const long long t = cell / m.nz;
-  const int j = t % m.ny;
-  const int i = t / m.ny;
+__global__ void __launch_bounds__(kThreads)
+    k_adjoint_finish(MeshView m, MeshView nodes, NodePlanes p, const int *__restrict__ first_chunk,
+                     int sub0, int nchunk, int group, long long ld,
+                     const double *__restrict__ Gpart, double *__restrict__ grad) {
+  // the cells of a tile lie on up to twice as many planes
+  __shared__ double g[PLANES ? 8 * kTileX * kTileY * kTileZ
+                             : (kTileX + 1) * (kTileY + 1) * (kTileZ + 1)];
+  constexpr int kTile[3] = {kTileX, kTileY, kTileZ};
+  chain_begin();
+  const int size[3] = {m.nx, m.ny, m.nz};
+  int t = blockIdx.x, c0[3], nc[3], n0[3], nn[3];
+#pragma unroll
+  for (int a = 2; a >= 0; --a) {
+    const int tiles = (size[a] + kTile[a] - 1) / kTile[a];
+    c0[a] = t % tiles * kTile[a];
+    t /= tiles;
+    nc[a] = min(kTile[a], size[a] - c0[a]);
+    n0[a] = PLANES ? p.lower[a][c0[a]] : c0[a];
+    nn[a] = (PLANES ? p.upper[a][c0[a] + nc[a] - 1] : c0[a] + nc[a]) - n0[a] + 1;
+  }
+  chain_wait();
+  int first;
+  const int nk = subset_chunks(first_chunk, sub0 + blockIdx.z, nchunk, first);
+  const long long all = nodes.nnodes(), len = all * gridDim.y;
+  const double *part = Gpart + first * len + blockIdx.y * all;
   const int ny1 = nodes.ny + 1, nz1 = nodes.nz + 1;
-  const int ni[2] = {PLANES ? p.lower[0][i] : i, PLANES ? p.upper[0][i] : i + 1};
-  const int nj[2] = {PLANES ? p.lower[1][j] : j, PLANES ? p.upper[1][j] : j + 1};
-  const int nk[2] = {PLANES ? p.lower[2][k] : k, PLANES ? p.upper[2][k] : k + 1};
+  for (int n = threadIdx.x; n < nn[0] * nn[1] * nn[2]; n += kThreads) {
+    const int k = n % nn[2], ij = n / nn[2], j = ij % nn[1], i = ij / nn[1];
+    const double *q = part + ((long long)(n0[0] + i) * ny1 + n0[1] + j) * nz1 + n0[2] + k;
+    double v = 0.0;
+#pragma unroll 8
+    for (int c = 0; c < nk; c += group) v += q[c * len];
+    g[n] = v;
+  }
+  __syncthreads();
+  const int k = threadIdx.x % kTileZ, j = threadIdx.x / kTileZ % kTileY,
+            i = threadIdx.x / (kTileZ * kTileY);
+  if (i >= nc[0] || j >= nc[1] || k >= nc[2]) return;
+  const int cell[3] = {i, j, k};
+  int corner[3][2];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    corner[a][0] = PLANES ? p.lower[a][c0[a] + cell[a]] - n0[a] : cell[a];
+    corner[a][1] = PLANES ? p.upper[a][c0[a] + cell[a]] - n0[a] : cell[a] + 1;
+  }
   double v = 0.0;
 #pragma unroll
   for (int q = 0; q < 8; ++q) {
     const int a = (q >> 2) & 1, b = (q >> 1) & 1, c = q & 1;
-    const double g = G[((long long)ni[a] * ny1 + nj[b]) * nz1 + nk[c]];
-    v = ((a + b + c) & 1) ? v - g : v + g;
+    const double x = g[(corner[0][a] * nn[1] + corner[1][b]) * nn[2] + corner[2][c]];
+    v = ((a + b + c) & 1) ? v - x : v + x;
   }
-  grad[cell] = 2.0 * v;
+  grad[(sub0 + blockIdx.z) * ld + blockIdx.y * m.ngrid() +
+       ((long long)(c0[0] + i) * m.ny + c0[1] + j) * m.nz + c0[2] + k] = 2.0 * v;
 }
 
 __global__ void k_background_grad(int kind, int nmeas, int nbg, const double *__restrict__ w_raw,
                                   const double *__restrict__ bgsens, double *__restrict__ gbg) {
+  chain_begin();
+  chain_wait();
   const int j = blockIdx.x;
   const int raw = kind_raw(kind);
   double acc = 0.0;
@@ -431,38 +514,26 @@ inline int cdiv(long long a, long long b) { return (int)((a + b - 1) / b); }
 
 // ---------------------------------------------------------------------------
 // Launchers
-#define J3G_DISPATCH4(kind, CALL, OTHER)                                     \
-  switch (kind) {                                                            \
-    case KIND_SCALAR: { constexpr int K = KIND_SCALAR; CALL; } break;        \
-    case KIND_TENSOR: { constexpr int K = KIND_TENSOR; CALL; } break;        \
-    case KIND_MAGNETIC: { constexpr int K = KIND_MAGNETIC; CALL; } break;    \
-    case KIND_JOINT: { constexpr int K = KIND_JOINT; CALL; } break;          \
-    OTHER                                                                    \
-    default: return cudaErrorInvalidValue;                                   \
+#define J3G_DISPATCH(kind, CALL)                                                  \
+  switch (kind) {                                                                 \
+    case KIND_SCALAR: { constexpr int K = KIND_SCALAR; CALL; } break;             \
+    case KIND_TENSOR: { constexpr int K = KIND_TENSOR; CALL; } break;             \
+    case KIND_MAGNETIC: { constexpr int K = KIND_MAGNETIC; CALL; } break;         \
+    case KIND_JOINT: { constexpr int K = KIND_JOINT; CALL; } break;               \
+    case KIND_MAG_GRADIENT: { constexpr int K = KIND_MAG_GRADIENT; CALL; } break; \
+    case KIND_MAGNETIZATION: { constexpr int K = KIND_MAGNETIZATION; CALL; } break; \
+    default: return cudaErrorInvalidValue;                                        \
   }
-// every kind
-#define J3G_DISPATCH(kind, CALL)                                                       \
-  J3G_DISPATCH4(kind, CALL,                                                            \
-                case KIND_MAG_GRADIENT: { constexpr int K = KIND_MAG_GRADIENT; CALL; } break; \
-                case KIND_MAGNETIZATION: { constexpr int K = KIND_MAGNETIZATION; CALL; } break;)
-// the kinds with a node-component layout (node reduce)
-#define J3G_DISPATCH_ORDINARY(kind, CALL) J3G_DISPATCH4(kind, CALL, )
 
-cudaError_t launch_forward_reduce(int kind, int nmeas, int nblk, const double *partial,
-                                  const MagField &mf, double *comps, cudaStream_t st) {
-  if (kind == KIND_MAG_GRADIENT) {
-    k_forward_reduce_raw<KIND_MAG_GRADIENT><<<cdiv(nmeas, kThreads), kThreads, 0, st>>>(
-        nmeas, nblk, partial, mf, comps);
-    return cudaGetLastError();
-  }
-  if (kind == KIND_MAGNETIZATION) {
-    k_forward_reduce_raw<KIND_MAGNETIZATION><<<cdiv(nmeas, kThreads), kThreads, 0, st>>>(
-        nmeas, nblk, partial, mf, comps);
-    return cudaGetLastError();
-  }
-  const int n = nmeas * NC_COUNT;
-  J3G_DISPATCH_ORDINARY(kind, (k_forward_reduce<K><<<cdiv(n, kThreads), kThreads, 0, st>>>(nmeas, nblk, partial, comps)));
-  return cudaGetLastError();
+cudaError_t launch_forward_finish(int kind, int transform, double tbx, double tby, double tbz,
+                                  int nmeas, int nblk, const double *partial,
+                                  const double *bgsens, int nbg, const double *bgval,
+                                  const MagField &mf, double *raw_out, double *data_out,
+                                  cudaStream_t st) {
+  J3G_DISPATCH(kind, return launch_chained(k_forward_finish<K>, dim3(cdiv(nmeas, kFinishStations)),
+                                           kThreads, 0, st, transform, tbx, tby, tbz, nmeas, nblk,
+                                           partial, bgsens, nbg, bgval, mf, raw_out, data_out));
+  return cudaSuccess;
 }
 
 cudaError_t launch_background(int kind, const MeshView &m, const StationView &s, int nbg,
@@ -479,52 +550,71 @@ cudaError_t launch_background(int kind, const MeshView &m, const StationView &s,
 }
 
 cudaError_t launch_assemble(int kind, int transform, double tbx, double tby, double tbz,
-                            int nmeas, const double *comps, int comps_ld, const double *bgsens,
-                            int nbg, const double *bgval, const MagField &mf, double *raw_out,
-                            double *data_out, cudaStream_t st) {
-  k_assemble<<<cdiv(nmeas, 128), 128, 0, st>>>(kind, transform, tbx, tby, tbz, nmeas, comps,
-                                                comps_ld, bgsens, nbg, bgval, mf, raw_out,
-                                                data_out);
+                            int nmeas, const double *rows, const double *bgsens, int nbg,
+                            const double *bgval, double *raw_out, double *data_out,
+                            cudaStream_t st) {
+  J3G_DISPATCH(kind, (k_assemble<kind_raw(K)><<<cdiv(nmeas, 128), 128, 0, st>>>(
+                         transform, tbx, tby, tbz, nmeas, rows, bgsens, nbg, bgval, raw_out,
+                         data_out)));
   return cudaGetLastError();
 }
 
 cudaError_t launch_backproject(int kind, int transform, double tbx, double tby, double tbz,
                                int nmeas, const double *misfit, const double *raw,
                                double *w_raw, cudaStream_t st) {
-  k_backproject<<<cdiv(nmeas, 128), 128, 0, st>>>(kind, transform, tbx, tby, tbz, nmeas, misfit,
-                                                  raw, w_raw);
+  J3G_DISPATCH(kind, (k_backproject<kind_raw(K)><<<cdiv(nmeas, 128), 128, 0, st>>>(
+                         transform, tbx, tby, tbz, nmeas, misfit, raw, w_raw)));
   return cudaGetLastError();
 }
 
-cudaError_t launch_comp_weights(int kind, int nmeas, const double *w_raw, const MagField &mf,
-                                double *W, cudaStream_t st) {
-  k_comp_weights<<<cdiv(nmeas, 128), 128, 0, st>>>(kind, nmeas, w_raw, mf, W);
-  return cudaGetLastError();
+cudaError_t launch_node_weights(int kind, int transform, double tbx, double tby, double tbz,
+                                int nmeas, const double *misfit, const double *raw,
+                                const MagField &mf, double *w_raw, double *W, cudaStream_t st) {
+  J3G_DISPATCH(kind, return launch_chained(k_node_weights<K>, dim3(cdiv(nmeas, 128)), 128, 0, st,
+                                           transform, tbx, tby, tbz, nmeas, misfit, raw, mf,
+                                           w_raw, W));
+  return cudaSuccess;
 }
 
-cudaError_t launch_adjoint_combine(const MeshView &m, const MeshView &nodes,
-                                   const NodePlanes *planes, int nchunk, int nblock,
-                                   const double *Gpart, double *G, double *grad, cudaStream_t st) {
-  const long long nn = nodes.nnodes();
-  const int blocks = cdiv(m.ngrid(), kThreads);
-  for (int b = 0; b < nblock; ++b) {
-    k_sum_chunks<<<cdiv(nn, kThreads), kThreads, 0, st>>>((int)nn, nchunk, nblock * nn,
-                                                           Gpart + b * nn, G + b * nn);
-    if (planes)
-      k_adjoint_combine<true><<<blocks, kThreads, 0, st>>>(m, nodes, *planes, G + b * nn,
-                                                           grad + b * m.ngrid());
-    else
-      k_adjoint_combine<false><<<blocks, kThreads, 0, st>>>(m, nodes, NodePlanes{}, G + b * nn,
-                                                            grad + b * m.ngrid());
+cudaError_t launch_adjoint_finish(const MeshView &m, const MeshView &nodes,
+                                  const NodePlanes *planes, int nblock, int nsub,
+                                  const int *first_chunk, int nchunk, long long ld, double *Gpart,
+                                  double *grad, cudaStream_t st, int *launches) {
+  // a thread of the last kernel adds up to 32 chunks one after the other; more
+  // are first added up in groups, which are then spread over the GPU
+  constexpr int kGroup = 32;
+  const long long len = nodes.nnodes() * nblock;
+  int group = 1;
+  if (nchunk > kGroup)
+    for (group = kGroup; (long long)group * group < nchunk;) group *= 2;
+  const int tiles = cdiv(m.nx, kTileX) * cdiv(m.ny, kTileY) * cdiv(m.nz, kTileZ);
+  *launches = 0;
+  for (int s0 = 0; s0 < nsub; s0 += 65535) {  // grid z
+    const int ns = nsub - s0 < 65535 ? nsub - s0 : 65535;
+    if (group > 1) {
+      const cudaError_t e = launch_chained(
+          k_sum_groups, dim3(cdiv(len, kThreads), cdiv(nchunk, group), ns), kThreads, 0, st, len,
+          first_chunk, s0, nchunk, group, Gpart);
+      if (e != cudaSuccess) return e;
+      ++*launches;
+    }
+    const dim3 grid(tiles, nblock, ns);
+    const cudaError_t e =
+        planes ? launch_chained(k_adjoint_finish<true>, grid, kThreads, 0, st, m, nodes, *planes,
+                                first_chunk, s0, nchunk, group, ld, Gpart, grad)
+               : launch_chained(k_adjoint_finish<false>, grid, kThreads, 0, st, m, nodes,
+                                NodePlanes{}, first_chunk, s0, nchunk, group, ld, Gpart, grad);
+    if (e != cudaSuccess) return e;
+    ++*launches;
   }
-  return cudaGetLastError();
+  return cudaSuccess;
 }
 
 cudaError_t launch_background_grad(int kind, int nmeas, int nbg, const double *w_raw,
                                    const double *bgsens, double *grad_bg, cudaStream_t st) {
   if (nbg == 0) return cudaSuccess;
-  k_background_grad<<<nbg, kThreads, 0, st>>>(kind, nmeas, nbg, w_raw, bgsens, grad_bg);
-  return cudaGetLastError();
+  return launch_chained(k_background_grad, dim3(nbg), kThreads, 0, st, kind, nmeas, nbg, w_raw,
+                        bgsens, grad_bg);
 }
 
 cudaError_t launch_direct_rows(int kind, const MeshView &m, const StationView &s, int s0, int ns,

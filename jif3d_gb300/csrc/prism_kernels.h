@@ -37,11 +37,11 @@ struct NodePlanes {
 
 // Forward, node formulation:  per station and component
 //   U_c(s) = scale_c * sum_nodes F_c(s, node) * rho~(node)
-// rho~ = third mixed backward difference of the zero-padded model (one model
-// block; magnetisation runs it once per block into rho_t + block * nnodes).
+// rho~ = third mixed backward difference of the zero-padded model, for each of
+// its nblock blocks.
 // nodes: the node grid, m itself or that of its planes.
 cudaError_t launch_rho_tilde(const MeshView &m, const MeshView &nodes, const NodePlanes *planes,
-                             const double *rho, double *rho_t, cudaStream_t st);
+                             int nblock, const double *rho, double *rho_t, cudaStream_t st);
 // Split of the forward's work: blocks of `cols` node columns and `kper` nodes
 // of each (nblk = column blocks x nkc pieces of the columns, at most
 // max_blocks of them where more columns per block can see to that), spb
@@ -55,10 +55,13 @@ NodeForwardPlan node_forward_plan(int nx, int ny, int nz, int nmeas, long long m
 cudaError_t launch_node_forward(int kind, const MeshView &m, const StationView &s,
                                 const double *rho_t, double *partial, const NodeForwardPlan &p,
                                 cudaStream_t st);
-// comps: [nmeas][NC_COUNT] node-component sums (scaled), unused comps zero;
-// for the vertical gradient and magnetisation the raw rows [nmeas][raw].
-cudaError_t launch_forward_reduce(int kind, int nmeas, int nblk, const double *partial,
-                                  const MagField &mf, double *comps, cudaStream_t st);
+// The stations' raw rows from their partial sums, background and transform as
+// by launch_assemble.
+cudaError_t launch_forward_finish(int kind, int transform, double t_bx, double t_by, double t_bz,
+                                  int nmeas, int nblk, const double *partial,
+                                  const double *bgsens, int nbg, const double *bgval,
+                                  const MagField &mf, double *raw_out, double *data_out,
+                                  cudaStream_t st);
 
 // Background: bgsens[s][raw][j] for each layer j (GravityBackground.cpp:24-137,
 // OMPMagneticSusceptibilityImp.cpp:31-101).
@@ -67,12 +70,12 @@ cudaError_t launch_background(int kind, const MeshView &m, const StationView &s,
                               double xw, double yw, double zw, const MagField &mf,
                               double *bgsens, cudaStream_t st);
 
-// Per station: raw = raw_from_comps(comps) (+ sum_j bgsens * bgval) and the
-// optional transform.  raw_out [nmeas][raw] (may be null), data_out [nmeas][dpm].
+// Per station: raw = rows [nmeas][raw] (+ sum_j bgsens * bgval) and the optional
+// transform.  raw_out [nmeas][raw] (may be null), data_out [nmeas][dpm].
 cudaError_t launch_assemble(int kind, int transform, double t_bx, double t_by, double t_bz,
-                            int nmeas, const double *comps, int comps_ld, const double *bgsens,
-                            int nbg, const double *bgval, const MagField &mf, double *raw_out,
-                            double *data_out, cudaStream_t st);
+                            int nmeas, const double *rows, const double *bgsens, int nbg,
+                            const double *bgval, double *raw_out, double *data_out,
+                            cudaStream_t st);
 
 // Adjoint.  w_raw [nmeas][raw] are the raw-row weights (misfit already
 // back-projected through the transform).  W [nmeas][NC_COUNT] receives the
@@ -81,8 +84,10 @@ cudaError_t launch_assemble(int kind, int transform, double t_bx, double t_by, d
 cudaError_t launch_backproject(int kind, int transform, double t_bx, double t_by, double t_bz,
                                int nmeas, const double *misfit, const double *raw,
                                double *w_raw, cudaStream_t st);
-cudaError_t launch_comp_weights(int kind, int nmeas, const double *w_raw, const MagField &mf,
-                                double *W, cudaStream_t st);
+// Both at once.
+cudaError_t launch_node_weights(int kind, int transform, double t_bx, double t_by, double t_bz,
+                                int nmeas, const double *misfit, const double *raw,
+                                const MagField &mf, double *w_raw, double *W, cudaStream_t st);
 // Gpart [nchunk][nblock][nnodes] = sum over the chunk's stations of
 // sum_q W_q * F_q, per model block.
 // chunk_start (device, nchunk + 1 values, may be null): explicit station
@@ -94,11 +99,15 @@ NodeAdjointPlan node_adjoint_plan(int nx, int ny, int nz, int nblock, int nmeas)
 cudaError_t launch_node_adjoint(int kind, const MeshView &m, const StationView &s,
                                 const double *W, const NodeAdjointPlan &p, int nchunk,
                                 const int *chunk_start, double *Gpart, cudaStream_t st);
-// grad[b * ngrid + cell] = 2 * sum_corners (-1)^shifts * sum_chunks
-// Gpart[chunk][b][node] for each model block b; G: nblock * nnodes scratch.
-cudaError_t launch_adjoint_combine(const MeshView &m, const MeshView &nodes,
-                                   const NodePlanes *planes, int nchunk, int nblock,
-                                   const double *Gpart, double *G, double *grad, cudaStream_t st);
+// grad[k * ld + b * ngrid + cell] = 2 * sum_corners (-1)^shifts * sum of
+// Gpart[chunk][b][node] over the chunks of subset k, for each model block b.
+// Subset k has the chunks first_chunk[k] to first_chunk[k + 1] - 1 (device, nsub
+// + 1 values), nchunk of them at most; null: one subset of nchunk chunks.  Gpart
+// is overwritten.  launches: kernels queued.
+cudaError_t launch_adjoint_finish(const MeshView &m, const MeshView &nodes,
+                                  const NodePlanes *planes, int nblock, int nsub,
+                                  const int *first_chunk, int nchunk, long long ld, double *Gpart,
+                                  double *grad, cudaStream_t st, int *launches);
 // grad[ngrid + j] = 2 * sum_s sum_r w_raw[s][r] * bgsens[s][r][j]
 cudaError_t launch_background_grad(int kind, int nmeas, int nbg, const double *w_raw,
                                    const double *bgsens, double *grad_bg, cudaStream_t st);

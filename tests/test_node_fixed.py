@@ -214,3 +214,55 @@ def test_planes_of_given_corners(ctx, oracle_lib, kind, apart):
                                     g.data_ptr())
     ctx.synchronize()
     assert relerr(g.sum(0).cpu().numpy(), p.lqderivative(s.model, misfit)) <= 1e-10
+
+
+# cells around the gradient's tiles of 2 x 4 x 16, station chunks below and
+# beyond the 32 that a thread adds up (and the 1024 of 32 groups)
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind,shape", [(W.SCALAR, (2, 4, 16, 31)), (W.TENSOR, (3, 5, 17, 400)),
+                                        (W.MAGNETIZATION, (1, 9, 33, 260)),
+                                        (W.SCALAR, (5, 3, 15, 5000))])
+@pytest.mark.parametrize("given", [False, True])
+def test_gradient_tiles_and_chunk_sums(ctx, kind, shape, given):
+    """The gradient of all stations and of uneven subsets of them (one empty, one
+    of one station), in one call and in a captured graph; with given corners the
+    tile's nodes are planes."""
+    import torch
+    s = _survey(kind, *shape, False)
+    n = s.stations.shape[0]
+    W.setup_context(ctx, s)
+    if given:  # an upper corner that is not the next lower one, by rounding
+        co = [s.coords(a) for a in range(3)]
+        co[2][1] = np.nextafter(co[2][1], np.inf)
+        ctx.set_mesh(*co, s.xsize, s.ysize, s.zsize)
+    J = _rows(s).reshape(n, -1, s.model.size)
+    misfit = np.random.default_rng(4).normal(size=(n, J.shape[1]))
+    cut = np.array([0, 0, 1, n // 3, n])
+    like = dict(dtype=torch.float64, device="cuda")
+    m, r = torch.tensor(s.model, **like), torch.tensor(misfit, **like)
+    g = torch.full((5, s.model.size), np.nan, **like)
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    ctx.set_stream(stream.cuda_stream)
+    try:
+        subsets = [np.arange(a, b) for a, b in zip(cut[:-1], cut[1:])]
+
+        def run():
+            ctx.subsets_lqderivative_device(subsets, m.data_ptr(), r.data_ptr(), g.data_ptr())
+            ctx.lqderivative_device(m.data_ptr(), r.data_ptr(), g[4].data_ptr())
+        run()
+        ctx.synchronize()
+        first = g.cpu().numpy()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            run()
+        g.fill_(np.nan)
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+    finally:
+        ctx.set_stream(0)
+    assert np.array_equal(first, g.cpu().numpy())
+    for k, (a, b) in enumerate(list(zip(cut[:-1], cut[1:])) + [(0, n)]):
+        ref = 2.0 * np.einsum("sr,srp->p", misfit[a:b], J[a:b])
+        assert relerr(first[k], ref) <= 1e-10 if b > a else np.all(first[k] == 0.0)
