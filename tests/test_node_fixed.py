@@ -266,3 +266,26 @@ def test_gradient_tiles_and_chunk_sums(ctx, kind, shape, given):
     for k, (a, b) in enumerate(list(zip(cut[:-1], cut[1:])) + [(0, n)]):
         ref = 2.0 * np.einsum("sr,srp->p", misfit[a:b], J[a:b])
         assert relerr(first[k], ref) <= 1e-10 if b > a else np.all(first[k] == 0.0)
+
+
+# more nodes to a column than a block takes at a time, and fewer
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", [W.TENSOR, W.MAGNETIC, W.JOINT])
+@pytest.mark.parametrize("shape", [(6, 5, 9), (3, 2, 70)])
+def test_stations_among_the_nodes(ctx, kind, shape):
+    """dz of both signs and zero along the columns, where the sum of the three
+    angles changes: stations between, on, above and below the mesh's planes, off
+    the columns and on them."""
+    s = _survey(kind, *shape, 24, False)
+    n = s.stations.shape[0]
+    z = s.coords(2)
+    s.stations[:, 2] = np.concatenate([[z[0] - 5.0, z[-1] + 5.0, z[-1], z[0], z[2]],
+                                       np.random.default_rng(8).uniform(z[0], z[-1], n - 5)])
+    s.stations[8:, 0] = s.coords(0)[np.arange(n - 8) % (shape[0] + 1)]
+    s.stations[16:, 1] = s.coords(1)[np.arange(n - 16) % (shape[1] + 1)]
+    W.setup_context(ctx, s)
+    J = _rows(s)
+    d = ctx.forward(s.model)
+    assert relerr(d, J @ s.model) <= 1e-10
+    misfit = np.random.default_rng(3).normal(size=d.size)
+    assert relerr(ctx.lqderivative(s.model, misfit), 2.0 * (misfit @ J)) <= 1e-10
