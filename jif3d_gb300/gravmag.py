@@ -25,6 +25,8 @@ products, as in FullSensitivityGravMagCalculator.
 """
 from __future__ import annotations
 
+from array import array
+
 import numpy as np
 
 from . import capi
@@ -111,13 +113,7 @@ class ThreeDModelBase:
     def _coords(origin, sizes):
         # ThreeDModelBase::CalcCoords (ModelBase/ThreeDModelBase.cpp:96-113):
         # running sum of the sizes, in order, starting at the origin
-        c = np.empty(sizes.size + 1)
-        c[0] = origin
-        s = origin
-        for i, v in enumerate(sizes):
-            s = s + v
-            c[i + 1] = s
-        return c
+        return np.add.accumulate(np.concatenate([[origin], sizes]))
 
     def GetXCoordinates(self):
         c = self._corners[0]
@@ -263,7 +259,8 @@ class GeneralData:
     """Measurement positions, data and errors (DataBase/GeneralData.h)."""
 
     def __init__(self):
-        self._x, self._y, self._z = [], [], []
+        # arrays, not lists: every Calculate looks at all positions
+        self._x, self._y, self._z = array("d"), array("d"), array("d")
         self._data, self._err = np.zeros(0), np.zeros(0)
 
     def SetDataAndErrors(self, D, E):
@@ -300,10 +297,10 @@ class GeneralData:
         return np.array(self._z)
 
     def CopyMeasurementConfiguration(self, other):
-        self._x, self._y, self._z = list(other._x), list(other._y), list(other._z)
+        self._x, self._y, self._z = other._x[:], other._y[:], other._z[:]
 
     def ClearMeasurementPoints(self):
-        self._x, self._y, self._z = [], [], []
+        self._x, self._y, self._z = array("d"), array("d"), array("d")
 
 
     # ReadNetCDF / WriteNetCDF of the data classes (Gravity/ScalarGravityData.cpp:16-38
