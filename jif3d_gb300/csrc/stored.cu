@@ -502,34 +502,50 @@ __device__ __forceinline__ uint32_t ring_slot(const float4 *ring, int b) {
                                             threadIdx.x);
 }
 
-// d[m][r] for NM models at once, J read once: a block takes kMultiRows rows, so
-// that each of them shares the models' values (512 KB a model from L2, which at
-// one row per block would be NM times the traffic of J).  A stage is half a
-// chain of the four rows.  Every sum is that of k_gemv_f32, bit for bit.
+// d[m][r] for NM models at once, J read once: G groups of kT threads take
+// kMultiRows rows each and share the models' values (512 KB a model from L2,
+// which at one row per block would be NM times the traffic of J).  A stage is a
+// quarter of a chain: a float4 of each row and of each model, all copied ahead;
+// with two groups the warps of the same columns copy half of the models each and
+// meet once a stage.  Every sum is that of k_gemv_f32, bit for bit.  7168 rows of
+// 131,072 cells, four models: 763 us with the models' values loaded when wanted
+// (their latency waited for in every stage), 687 copied ahead, 655 with two
+// groups; J alone is 563 us, and the FP64 additions of the chains 400.
 constexpr int kMultiRows = 4;
-static_assert(kRingBatch == 2 * kMultiRows, "a stage is two float4 of each row");
-template <int NM>
-__global__ void __launch_bounds__(kT, 2)
+template <int NM, int G> struct MultiRing {
+  static constexpr int kGroups = G;
+  static constexpr int kStages = G == 1 ? 3 : 4;
+  static constexpr int kSlots = G * kMultiRows + NM;  // float4 of a column quad and stage
+  static constexpr int kBytes = kStages * kSlots * kT * 16;
+};
+template <int NM, int G>
+__global__ void __launch_bounds__(G * kT, 2 / G)
     k_gemv_f32_multi(const float *__restrict__ J, long long ld, int nrows,
                      const float *__restrict__ x, double *__restrict__ out, long long ld_out) {
+  using R = MultiRing<NM, G>;
   constexpr int RB = kMultiRows;
-  extern __shared__ __align__(16) float4 ring[];  // [stage][row][half of a half][thread]
-  const int r0 = blockIdx.x * RB;
+  extern __shared__ __align__(16) float4 ring[];  // [stage][rows of all groups, then models][column]
+  const int tid = threadIdx.x % kT, g = threadIdx.x / kT;
+  const int r0 = (blockIdx.x * G + g) * RB;
   const int n4 = (int)(ld / 4);
-  const float4 *p = reinterpret_cast<const float4 *>(J) + (long long)r0 * n4 + threadIdx.x;
-  const float4 *xv = reinterpret_cast<const float4 *>(x) + threadIdx.x;
-  // whole chains (four float4 of a thread, kT apart), two stages each
-  const int nfull = n4 > 3 * kT + (int)threadIdx.x
-                        ? (n4 - 3 * kT - (int)threadIdx.x - 1) / (4 * kT) + 1 : 0;
+  const float4 *p = reinterpret_cast<const float4 *>(J) + (long long)r0 * n4 + tid;
+  const float4 *xv = reinterpret_cast<const float4 *>(x) + tid;
+  // whole chains (four float4 of a thread, kT apart), four stages each; a warp
+  // goes as far as its first lane
+  auto chains = [&](int t) { return n4 > 3 * kT + t ? (n4 - 3 * kT - t - 1) / (4 * kT) + 1 : 0; };
+  const int nfull = chains(tid), most = chains(tid & ~31);
+  auto slot = [&](int b) { return ring + (b % R::kStages) * R::kSlots * kT + tid; };
   auto fetch = [&](int b) {
-    if (b < 2 * nfull) {
-      const uint32_t dst = ring_slot(ring, b);
+    if (b < 4 * nfull) {
+      const uint32_t dst = (uint32_t)__cvta_generic_to_shared(slot(b));
 #pragma unroll
       for (int r = 0; r < RB; ++r)
+        if (r0 + r < nrows)
+          copy_async16(dst + (g * RB + r) * kT * 16, p + (long long)r * n4 + b * kT);
 #pragma unroll
-        for (int u = 0; u < 2; ++u)
-          if (r0 + r < nrows)
-            copy_async16(dst + (2 * r + u) * kT * 16, p + (long long)r * n4 + (2 * b + u) * kT);
+      for (int m = 0; m < NM; ++m)
+        if (G == 1 || m % G == g)
+          copy_async16(dst + (G * RB + m) * kT * 16, xv + (long long)m * n4 + b * kT);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
@@ -539,31 +555,31 @@ __global__ void __launch_bounds__(kT, 2)
   for (int r = 0; r < RB; ++r)
 #pragma unroll
     for (int m = 0; m < NM; ++m) accd[r][m] = 0.0, acc[r][m] = 0.0f;
-  for (int b = 0; b < kRingStages - 1; ++b) fetch(b);
+  for (int b = 0; b < R::kStages - 1; ++b) fetch(b);
 #pragma unroll 1
-  for (int b = 0; b < 2 * nfull; ++b) {
-    float4 xb[NM][2];
+  for (int b = 0; b < 4 * most; ++b) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(R::kStages - 2) : "memory");
+    // stage b is there for both warps, and both have read stage b - 1
+    if constexpr (G > 1)
+      asm volatile("bar.sync %0, %1;" ::"r"(1 + tid / 32), "n"(32 * G) : "memory");
+    fetch(b + R::kStages - 1);  // into the stage that was read last
+    if (b >= 4 * nfull) continue;
+    const float4 *a = slot(b);
+    float4 xb[NM];
 #pragma unroll
-    for (int m = 0; m < NM; ++m)
-#pragma unroll
-      for (int u = 0; u < 2; ++u) xb[m][u] = xv[(long long)m * n4 + (2 * b + u) * kT];
-    fetch(b + kRingStages - 1);  // into the stage that was read last
-    asm volatile("cp.async.wait_group %0;" ::"n"(kRingStages - 1) : "memory");
-    const float4 *a = ring + (b % kRingStages) * kRingBatch * kT + threadIdx.x;
+    for (int m = 0; m < NM; ++m) xb[m] = a[(G * RB + m) * kT];
 #pragma unroll
     for (int r = 0; r < RB; ++r) {
-      const float4 a0 = a[2 * r * kT], a1 = a[(2 * r + 1) * kT];
+      const float4 a0 = a[(g * RB + r) * kT];
 #pragma unroll
       for (int m = 0; m < NM; ++m) {
         // a chain starts with a product, as k_gemv_f32's
-        float s = b & 1 ? fmaf(a0.x, xb[m][0].x, acc[r][m]) : a0.x * xb[m][0].x;
-        s = fmaf(a0.y, xb[m][0].y, s); s = fmaf(a0.z, xb[m][0].z, s);
-        s = fmaf(a0.w, xb[m][0].w, s); s = fmaf(a1.x, xb[m][1].x, s);
-        s = fmaf(a1.y, xb[m][1].y, s); s = fmaf(a1.z, xb[m][1].z, s);
-        acc[r][m] = fmaf(a1.w, xb[m][1].w, s);
+        float s = b & 3 ? fmaf(a0.x, xb[m].x, acc[r][m]) : a0.x * xb[m].x;
+        s = fmaf(a0.y, xb[m].y, s); s = fmaf(a0.z, xb[m].z, s);
+        acc[r][m] = fmaf(a0.w, xb[m].w, s);
       }
     }
-    if (b & 1) {
+    if ((b & 3) == 3) {
 #pragma unroll
       for (int r = 0; r < RB; ++r)
 #pragma unroll
@@ -571,7 +587,7 @@ __global__ void __launch_bounds__(kT, 2)
     }
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
-  for (int i = 4 * kT * nfull; i + (int)threadIdx.x < n4; i += kT) {
+  for (int i = 4 * kT * nfull; i + tid < n4; i += kT) {
 #pragma unroll
     for (int r = 0; r < RB; ++r) {
       if (r0 + r >= nrows) break;
@@ -585,14 +601,22 @@ __global__ void __launch_bounds__(kT, 2)
       }
     }
   }
-  __shared__ double red[kT / 32];
+  // every row and model's sum over the group's warps, in warp order
+  __shared__ double red[G][RB * NM][kT / 32];
 #pragma unroll
   for (int r = 0; r < RB; ++r)
 #pragma unroll
     for (int m = 0; m < NM; ++m) {
-      const double v = block_sum_d<kT>(accd[r][m], red);
-      if (threadIdx.x == 0 && r0 + r < nrows) out[m * ld_out + r0 + r] = v;
+      const double v = warp_sum_d(accd[r][m]);
+      if (tid % 32 == 0) red[g][r * NM + m][tid / 32] = v;
     }
+  __syncthreads();
+  const int r = tid / NM, m = tid % NM;
+  if (r >= RB || r0 + r >= nrows) return;
+  double v = 0.0;
+#pragma unroll
+  for (int w = 0; w < kT / 32; ++w) v += red[g][tid][w];
+  out[m * ld_out + r0 + r] = v;
 }
 
 // part[chunk][c] = sum_{r in chunk} J[r][c] w[r]; block = 1024 columns x RC rows.
@@ -1289,16 +1313,23 @@ cudaError_t launch_gemv_f32(const float *J, long long ld, int nrows, int nmod, c
     return cudaGetLastError();
   }
   if (nmod < 1 || nmod > kStreamModels || ld / 4 > INT_MAX - 8 * kT) return cudaErrorInvalidValue;
-  auto run = [&](auto kernel) {
+  auto run = [&](auto kernel, auto ring) {
+    using R = decltype(ring);
     const cudaError_t e =
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRingBytes);
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, R::kBytes);
     if (e != cudaSuccess) return e;
-    kernel<<<cdiv(nrows, kMultiRows), kT, kRingBytes, st>>>(J, ld, nrows, x, out, ld_out);
+    kernel<<<cdiv(nrows, R::kGroups * kMultiRows), R::kGroups * kT, R::kBytes, st>>>(
+        J, ld, nrows, x, out, ld_out);
     return cudaGetLastError();
   };
-  return nmod == 2   ? run(k_gemv_f32_multi<2>)
-         : nmod == 3 ? run(k_gemv_f32_multi<3>)
-                     : run(k_gemv_f32_multi<4>);
+  // two groups to a block (4 % faster) while that leaves a block for every SM
+  if (cdiv(nrows, 2 * kMultiRows) >= 152)
+    return nmod == 2   ? run(k_gemv_f32_multi<2, 2>, MultiRing<2, 2>{})
+           : nmod == 3 ? run(k_gemv_f32_multi<3, 2>, MultiRing<3, 2>{})
+                       : run(k_gemv_f32_multi<4, 2>, MultiRing<4, 2>{});
+  return nmod == 2   ? run(k_gemv_f32_multi<2, 1>, MultiRing<2, 1>{})
+         : nmod == 3 ? run(k_gemv_f32_multi<3, 1>, MultiRing<3, 1>{})
+                     : run(k_gemv_f32_multi<4, 1>, MultiRing<4, 1>{});
 }
 
 int gemv_t_chunks(int nrows) { return cdiv(nrows, kRC); }

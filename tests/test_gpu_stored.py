@@ -600,3 +600,12 @@ def test_fp32_batches_share_a_pass(ctx, shape, nmeas):
     for n in range(2, 7):
         assert np.array_equal(ctx.batched_forward(models[:n]), np.array(one[:n]))
         assert np.array_equal(ctx.batched_lqderivative(models[:n], mis[:n]), np.array(grad[:n]))
+
+
+@pytest.mark.parametrize("shape", [(16, 16, 16), (17, 16, 16)])
+@pytest.mark.parametrize("nmeas", [173, 174, 175])
+def test_fp32_batches_two_groups(ctx, shape, nmeas):
+    """The same around the 152 blocks of eight rows from which two groups of
+    threads share a block: 1211, 1218 and 1225 rows leave the last block's groups
+    three and none, two and none, one and none."""
+    test_fp32_batches_share_a_pass(ctx, shape, nmeas)
