@@ -15,6 +15,10 @@
 //              |y| > |x|, pi - that when x is negative, the sign of y;
 //              about 20 FP64 operations; fatan2_pair gives atan2(y, x) and
 //              atan2(x, y) from one ratio and series.
+// With SPLIT the quotient and the exact differences are integer work too
+// (fp64_int.cuh), six FP64 operations fewer in the arctangent and one in the
+// logarithm: the same values (the FP64 quotient may miss the nearest double once
+// in 2^39 operands).
 // Both are within about one unit in the last place of the exact value; the
 // tables come from gen_fp64_tables.py.  Zeros are handled in the fast path of
 // fatan2 with IEEE's signed results; subnormal, infinite and NaN operands
@@ -24,6 +28,7 @@
 
 #include <cstdint>
 
+#include "fp64_int.cuh"
 #include "fp64_tables.h"
 #include "fpbits.cuh"
 
@@ -39,18 +44,24 @@ __device__ __forceinline__ double small_int_to_f64(int k) {
   return __longlong_as_double((long long)(s | ((unsigned long long)(1023 + p) << 52) | mant));
 }
 
+template <bool SPLIT = false>
 __device__ __forceinline__ double flog(double x) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(x);
   const uint32_t e = (uint32_t)(b >> 52);  // with the sign bit: positive normals are 1..0x7fe
   if (e - 1u >= 0x7feu) return log(x);
   const unsigned long long mant = b & 0xfffffffffffffull;
   const uint32_t j = (uint32_t)((mant + (1ull << 44)) >> 45);  // nearest 1/128: 0..128
-  const double m = __longlong_as_double((long long)(mant | 0x3ff0000000000000ull));
-  const double F = __longlong_as_double(
-      (long long)(((unsigned long long)(1023u + (j >> 7)) << 52) |
-                  ((unsigned long long)(j & 127u) << 45)));
   const double *row = fp64tab::kLogTable[j];
-  const double f = __dsub_rn(m, F);  // exact: m and F are within 1/256
+  double f;  // m - F, exact: they are within 1/256
+  if constexpr (SPLIT) {
+    f = int_to_double((long long)(mant - ((unsigned long long)j << 45)), 52);
+  } else {
+    const double m = __longlong_as_double((long long)(mant | 0x3ff0000000000000ull));
+    const double F = __longlong_as_double(
+        (long long)(((unsigned long long)(1023u + (j >> 7)) << 52) |
+                    ((unsigned long long)(j & 127u) << 45)));
+    f = __dsub_rn(m, F);
+  }
   const double u = __dmul_rn(f, __ldg(row));
   // log1p(u) = u + u^2 (-1/2 + u/3 - u^2/4 + u^3/5 - u^4/6 + u^5/7)
   double q = __fma_rn(u, 1.0 / 7.0, -1.0 / 6.0);
@@ -67,19 +78,28 @@ __device__ __forceinline__ double flog(double x) {
   return __dadd_rn(hi, lo);
 }
 
-// atan t for t = min(a, b) / max(a, b), a and b the magnitude bits of the
-// operands; false if the operands need CUDA's atan2 (subnormal, infinite,
-// NaN, or a ratio below 2^-1000).
-__device__ __forceinline__ bool atan_ratio(unsigned long long ay, unsigned long long ax,
-                                           double &ta) {
-  const uint32_t ey = (uint32_t)(ay >> 52), ex = (uint32_t)(ax >> 52);
-  if (!((ay == 0 || ey - 1u < 0x7feu) && (ax == 0 || ex - 1u < 0x7feu))) return false;
-  const bool swap = ay > ax;  // magnitudes compare as integers
-  const unsigned long long bnum = swap ? ax : ay, bden = swap ? ay : ax;
-  double t = 0.0;
-  if (bnum != 0) {
-    const uint32_t en = (uint32_t)(bnum >> 52), ed = (uint32_t)(bden >> 52);
-    if (ed - en > 1000u) return false;
+// t = num / den and from it the nearest breakpoint c_j = j/64 and d = t - c_j
+// (exact), num and den normal magnitudes' bits, den the larger.
+template <bool SPLIT>
+__device__ __forceinline__ void atan_reduce(unsigned long long bnum, unsigned long long bden,
+                                            int &j, double &d) {
+  const uint32_t en = (uint32_t)(bnum >> 52), ed = (uint32_t)(bden >> 52);
+  if constexpr (SPLIT) {
+    int down;
+    const unsigned long long z =
+        int_quotient((bnum & kIntFrac) | kIntOne, (bden & kIntFrac) | kIntOne, down);
+    const int e = (int)(en - ed) - down;  // t = z 2^(e - 52)
+    j = 0;
+    if (e >= -8) {  // 64 t to the nearest integer, by way of t as a float
+      const uint32_t f = (uint32_t)((z + 0xfffffffull + (z >> 29 & 1u)) >> 29);
+      const float t64 = __uint_as_float(((uint32_t)(e + 126 + 6) << 23) + f);
+      j = (int)(__float_as_uint(__fadd_rn(t64, 8388608.0f)) & 0xffu);
+    }
+    if (j == 0)
+      d = __longlong_as_double((long long)(z + ((unsigned long long)(uint32_t)(e + 1022) << 52)));
+    else
+      d = int_to_double((long long)((z << (8 + e)) - ((unsigned long long)(uint32_t)j << 54)), 60);
+  } else {
     // num and den scaled by one power of two so that den is in [1, 2)
     const long long sh = (long long)(1023 - (int)ed) << 52;
     const double num = __longlong_as_double((long long)bnum + sh);
@@ -87,14 +107,31 @@ __device__ __forceinline__ bool atan_ratio(unsigned long long ay, unsigned long 
     const double r0 = f32_to_f64(__frcp_rn(f64_to_f32_ftz(den)));
     const double r1 = __fma_rn(r0, __fma_rn(-den, r0, 1.0), r0);
     const double t0 = __dmul_rn(num, r1);
-    t = __fma_rn(__fma_rn(-den, t0, num), r1, t0);
+    const double t = __fma_rn(__fma_rn(-den, t0, num), r1, t0);
+    j = __float2int_rn(__fmul_rn(f64_to_f32_ftz(t), 64.0f));
+    const double c =
+        j == 0 ? 0.0 : __longlong_as_double(__double_as_longlong(small_int_to_f64(j)) -
+                                            (6ll << 52));
+    d = __dsub_rn(t, c);
   }
-  // nearest breakpoint c_j = j/64 and d = t - c_j (exact)
-  const int j = __float2int_rn(__fmul_rn(f64_to_f32_ftz(t), 64.0f));
-  const double c =
-      j == 0 ? 0.0 : __longlong_as_double(__double_as_longlong(small_int_to_f64(j)) -
-                                          (6ll << 52));
-  const double d = __dsub_rn(t, c);
+}
+
+// atan t for t = min(a, b) / max(a, b), a and b the magnitude bits of the
+// operands; false if the operands need CUDA's atan2 (subnormal, infinite,
+// NaN, or a ratio below 2^-1000).
+template <bool SPLIT>
+__device__ __forceinline__ bool atan_ratio(unsigned long long ay, unsigned long long ax,
+                                           double &ta) {
+  const uint32_t ey = (uint32_t)(ay >> 52), ex = (uint32_t)(ax >> 52);
+  if (!((ay == 0 || ey - 1u < 0x7feu) && (ax == 0 || ex - 1u < 0x7feu))) return false;
+  const bool swap = ay > ax;  // magnitudes compare as integers
+  const unsigned long long bnum = swap ? ax : ay, bden = swap ? ay : ax;
+  int j = 0;
+  double d = 0.0;
+  if (bnum != 0) {
+    if ((uint32_t)(bden >> 52) - (uint32_t)(bnum >> 52) > 1000u) return false;
+    atan_reduce<SPLIT>(bnum, bden, j, d);
+  }
   const double *a = fp64tab::kAtanTable[j];
   double p = __ldg(a + 9);
 #pragma unroll
@@ -112,23 +149,25 @@ __device__ __forceinline__ double atan2_octant(double ta, bool swap, unsigned lo
   return __longlong_as_double(__double_as_longlong(th) | (long long)(by & 0x8000000000000000ull));
 }
 
+template <bool SPLIT = false>
 __device__ __forceinline__ double fatan2(double y, double x) {
   const unsigned long long by = (unsigned long long)__double_as_longlong(y);
   const unsigned long long bx = (unsigned long long)__double_as_longlong(x);
   const unsigned long long ay = by & 0x7fffffffffffffffull, ax = bx & 0x7fffffffffffffffull;
   double ta;
-  if (!atan_ratio(ay, ax, ta)) return atan2(y, x);
+  if (!atan_ratio<SPLIT>(ay, ax, ta)) return atan2(y, x);
   return atan2_octant(ta, ay > ax, bx, by);
 }
 
 // fatan2(y, x) and fatan2(x, y) with one shared ratio and series: the two
 // angles need the same t = min/max (bit for bit the two separate calls).
+template <bool SPLIT = false>
 __device__ __forceinline__ void fatan2_pair(double y, double x, double &yx, double &xy) {
   const unsigned long long by = (unsigned long long)__double_as_longlong(y);
   const unsigned long long bx = (unsigned long long)__double_as_longlong(x);
   const unsigned long long ay = by & 0x7fffffffffffffffull, ax = bx & 0x7fffffffffffffffull;
   double ta;
-  if (!atan_ratio(ay, ax, ta)) {
+  if (!atan_ratio<SPLIT>(ay, ax, ta)) {
     yx = atan2(y, x);
     xy = atan2(x, y);
     return;

@@ -71,14 +71,20 @@ __device__ __forceinline__ bool lt_eps(double v) {
 // Clamp from below that keeps NaN, like std::max(v, eps).
 __device__ __forceinline__ double clamp_eps(double v) { return lt_eps(v) ? kEps : v; }
 
+__device__ __forceinline__ bool normal_positive(double v) {
+  return (uint32_t)((unsigned long long)__double_as_longlong(v) >> 52) - 1u < 0x7feu;
+}
+
 // All node terms needed by `mask` (bit c set -> component c) for one offset
 // (dx, dy, dz) = station - node.  One square root serves every component.
-template <int MASK>
+// SPLIT: the same values, the square root, the quotients and the exact
+// differences on the integer pipes.
+template <int MASK, bool SPLIT = false>
 __device__ __forceinline__ void node_terms(double dx, double dy, double dz, double *out) {
   // fused: the node terms need r to FP64 accuracy, not the reference's
   // rounding (the eight-corner path keeps that)
   const double s2 = __fma_rn(dx, dx, __fma_rn(dy, dy, mul(dz, dz)));
-  const double r = sqrt(s2);
+  const double r = SPLIT && normal_positive(s2) ? int_sqrt(s2) : sqrt(s2);
   constexpr bool need_gz = MASK & (1 << NC_GZ);
   constexpr bool need_off = MASK & ((1 << NC_XY) | (1 << NC_XZ) | (1 << NC_YZ));
   double lx = 0.0, ly = 0.0;
@@ -86,37 +92,39 @@ __device__ __forceinline__ void node_terms(double dx, double dy, double dz, doub
     // ln(dx + r) and ln(dy + r) are shared by g_z and the Uyz / Uxz terms when
     // r >= eps (then g_z's clamped r equals the raw r).
     const double rg = clamp_eps(r);
-    lx = flog(add(dx, rg));
-    ly = flog(add(dy, rg));
+    const double sx = add(dx, rg), sy = add(dy, rg);
+    lx = flog<SPLIT>(sx);
+    ly = flog<SPLIT>(sy);
     if (need_gz) {
       double a;
       if ((MASK & (1 << NC_ZZ)) && !lt_eps(r)) {
         // g_z's atan2(dz r, dx dy) and Uzz's atan2(dx dy, dz r) share their ratio
         double zz;
-        fatan2_pair(mul(dz, rg), mul(dx, dy), a, zz);
+        fatan2_pair<SPLIT>(mul(dz, rg), mul(dx, dy), a, zz);
         out[NC_ZZ] = zz;
       } else {
-        a = fatan2(mul(dz, rg), mul(dx, dy));
-        if (MASK & (1 << NC_ZZ)) out[NC_ZZ] = fatan2(mul(dx, dy), mul(dz, r));
+        a = fatan2<SPLIT>(mul(dz, rg), mul(dx, dy));
+        if (MASK & (1 << NC_ZZ)) out[NC_ZZ] = fatan2<SPLIT>(mul(dx, dy), mul(dz, r));
       }
       out[NC_GZ] = __fma_rn(dx, ly, __fma_rn(dy, lx, mul(dz, a)));
     }
     if (need_off) {
       const bool shared = !lt_eps(r);
-      const double ax = add(dx, r), ay = add(dy, r), az = add(dz, r);
+      const double ax = shared ? sx : add(dx, r), ay = shared ? sy : add(dy, r);
+      const double az = add(dz, r);
       const double log_eps = fp64tab::kLogDblEps;  // log(DBL_EPSILON)
       if (MASK & (1 << NC_YZ))
-        out[NC_YZ] = lt_eps(ax) ? log_eps : (shared ? lx : flog(ax));
+        out[NC_YZ] = lt_eps(ax) ? log_eps : (shared ? lx : flog<SPLIT>(ax));
       if (MASK & (1 << NC_XZ))
-        out[NC_XZ] = lt_eps(ay) ? log_eps : (shared ? ly : flog(ay));
+        out[NC_XZ] = lt_eps(ay) ? log_eps : (shared ? ly : flog<SPLIT>(ay));
       if (MASK & (1 << NC_XY))
-        out[NC_XY] = lt_eps(az) ? log_eps : flog(az);
+        out[NC_XY] = lt_eps(az) ? log_eps : flog<SPLIT>(az);
     }
   }
-  if (MASK & (1 << NC_XX)) out[NC_XX] = fatan2(mul(dy, dz), mul(dx, r));
-  if (MASK & (1 << NC_YY)) out[NC_YY] = fatan2(mul(dx, dz), mul(dy, r));
+  if (MASK & (1 << NC_XX)) out[NC_XX] = fatan2<SPLIT>(mul(dy, dz), mul(dx, r));
+  if (MASK & (1 << NC_YY)) out[NC_YY] = fatan2<SPLIT>(mul(dx, dz), mul(dy, r));
   constexpr bool zz_done = (MASK & (1 << NC_GZ)) != 0;  // computed with g_z above
-  if ((MASK & (1 << NC_ZZ)) && !zz_done) out[NC_ZZ] = fatan2(mul(dx, dy), mul(dz, r));
+  if ((MASK & (1 << NC_ZZ)) && !zz_done) out[NC_ZZ] = fatan2<SPLIT>(mul(dx, dy), mul(dz, r));
 }
 
 // Corner order of each component's eight-term sum, as bit triples

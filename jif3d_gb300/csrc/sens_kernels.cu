@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(kThreads)
   for (int p = 0; p < U::positions; ++p) {
     // the second position of the vertical gradient is 1 m below the first
     double v[NC_COUNT];
-    node_terms<U::mask>(dx, dy, sub(p ? add(st.z[s], 1.0) : st.z[s], m.Z[k]), v);
+    node_terms<U::mask, true>(dx, dy, sub(p ? add(st.z[s], 1.0) : st.z[s], m.Z[k]), v);
 #pragma unroll
     for (int u = 0; u < U::per; ++u)
       F[((long long)sl * U::n + p * U::per + u) * nn + n] = v[U::comp(u)];
