@@ -41,12 +41,12 @@ __device__ __forceinline__ double small_int_to_f64(int k) {
   const uint32_t a = (uint32_t)(k < 0 ? -k : k);
   const int p = 31 - __clz(a);
   const unsigned long long mant = ((unsigned long long)a << (52 - p)) & 0xfffffffffffffull;
-  return __longlong_as_double((long long)(s | ((unsigned long long)(1023 + p) << 52) | mant));
+  return bits_f64((long long)(s | ((unsigned long long)(1023 + p) << 52) | mant));
 }
 
 template <bool SPLIT = false>
 __device__ __forceinline__ double flog(double x) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  const unsigned long long b = (unsigned long long)fx_bits(x);
   const uint32_t e = (uint32_t)(b >> 52);  // with the sign bit: positive normals are 1..0x7fe
   if (e - 1u >= 0x7feu) return log(x);
   const unsigned long long mant = b & 0xfffffffffffffull;
@@ -56,8 +56,8 @@ __device__ __forceinline__ double flog(double x) {
   if constexpr (SPLIT) {
     f = int_to_double((long long)(mant - ((unsigned long long)j << 45)), 52);
   } else {
-    const double m = __longlong_as_double((long long)(mant | 0x3ff0000000000000ull));
-    const double F = __longlong_as_double(
+    const double m = bits_f64((long long)(mant | 0x3ff0000000000000ull));
+    const double F = bits_f64(
         (long long)(((unsigned long long)(1023u + (j >> 7)) << 52) |
                     ((unsigned long long)(j & 127u) << 45)));
     f = __dsub_rn(m, F);
@@ -96,21 +96,21 @@ __device__ __forceinline__ void atan_reduce(unsigned long long bnum, unsigned lo
       j = (int)(__float_as_uint(__fadd_rn(t64, 8388608.0f)) & 0xffu);
     }
     if (j == 0)
-      d = __longlong_as_double((long long)(z + ((unsigned long long)(uint32_t)(e + 1022) << 52)));
+      d = bits_f64((long long)(z + ((unsigned long long)(uint32_t)(e + 1022) << 52)));
     else
       d = int_to_double((long long)((z << (8 + e)) - ((unsigned long long)(uint32_t)j << 54)), 60);
   } else {
     // num and den scaled by one power of two so that den is in [1, 2)
     const long long sh = (long long)(1023 - (int)ed) << 52;
-    const double num = __longlong_as_double((long long)bnum + sh);
-    const double den = __longlong_as_double((long long)bden + sh);
+    const double num = bits_f64((long long)bnum + sh);
+    const double den = bits_f64((long long)bden + sh);
     const double r0 = f32_to_f64(__frcp_rn(f64_to_f32_ftz(den)));
     const double r1 = __fma_rn(r0, __fma_rn(-den, r0, 1.0), r0);
     const double t0 = __dmul_rn(num, r1);
     const double t = __fma_rn(__fma_rn(-den, t0, num), r1, t0);
     j = __float2int_rn(__fmul_rn(f64_to_f32_ftz(t), 64.0f));
     const double c =
-        j == 0 ? 0.0 : __longlong_as_double(__double_as_longlong(small_int_to_f64(j)) -
+        j == 0 ? 0.0 : bits_f64(f64_bits(small_int_to_f64(j)) -
                                             (6ll << 52));
     d = __dsub_rn(t, c);
   }
@@ -146,13 +146,13 @@ __device__ __forceinline__ double atan2_octant(double ta, bool swap, unsigned lo
                                                unsigned long long by) {
   double th = swap ? __dadd_rn(fp64tab::kPio2Hi, __fma_rn(-1.0, ta, fp64tab::kPio2Lo)) : ta;
   if (bx >> 63) th = __dadd_rn(fp64tab::kPiHi, __fma_rn(-1.0, th, fp64tab::kPiLo));
-  return __longlong_as_double(__double_as_longlong(th) | (long long)(by & 0x8000000000000000ull));
+  return fx_double(fx_bits(th) | (by & 0x8000000000000000ull));
 }
 
 template <bool SPLIT = false>
 __device__ __forceinline__ double fatan2(double y, double x) {
-  const unsigned long long by = (unsigned long long)__double_as_longlong(y);
-  const unsigned long long bx = (unsigned long long)__double_as_longlong(x);
+  const unsigned long long by = (unsigned long long)fx_bits(y);
+  const unsigned long long bx = (unsigned long long)fx_bits(x);
   const unsigned long long ay = by & 0x7fffffffffffffffull, ax = bx & 0x7fffffffffffffffull;
   double ta;
   if (!atan_ratio<SPLIT>(ay, ax, ta)) return atan2(y, x);
@@ -163,8 +163,8 @@ __device__ __forceinline__ double fatan2(double y, double x) {
 // angles need the same t = min/max (bit for bit the two separate calls).
 template <bool SPLIT = false>
 __device__ __forceinline__ void fatan2_pair(double y, double x, double &yx, double &xy) {
-  const unsigned long long by = (unsigned long long)__double_as_longlong(y);
-  const unsigned long long bx = (unsigned long long)__double_as_longlong(x);
+  const unsigned long long by = (unsigned long long)fx_bits(y);
+  const unsigned long long bx = (unsigned long long)fx_bits(x);
   const unsigned long long ay = by & 0x7fffffffffffffffull, ax = bx & 0x7fffffffffffffffull;
   double ta;
   if (!atan_ratio<SPLIT>(ay, ax, ta)) {

@@ -11,11 +11,25 @@
 
 namespace j3g {
 
+// The bits of a double and back, opaque: where the compiler sees the double
+// behind a mask of the sign bit or a comparison with zero it makes them an FP64
+// absolute value, negation or comparison, each of which takes a slot of that pipe.
+__device__ __forceinline__ long long f64_bits(double v) {
+  long long r;
+  asm("mov.b64 %0, %1;" : "=l"(r) : "d"(v));
+  return r;
+}
+__device__ __forceinline__ double bits_f64(long long v) {
+  double r;
+  asm("mov.b64 %0, %1;" : "=d"(r) : "l"(v));
+  return r;
+}
+
 // v truncated to a float (20 of its mantissa bits), for magnitude and mean
 // estimates only: |v| below the float normal range gives a signed zero,
 // beyond it the largest float; infinities and NaNs keep their class.
 __device__ __forceinline__ float approx_f32(double v) {
-  const uint32_t h = (uint32_t)((unsigned long long)__double_as_longlong(v) >> 32);
+  const uint32_t h = (uint32_t)((unsigned long long)f64_bits(v) >> 32);
   const uint32_t s = h & 0x80000000u, e = (h >> 20) & 0x7ffu, m = h & 0xfffffu;
   if (e == 0x7ffu) return __uint_as_float(s | 0x7f800000u | (m ? 0x400000u : 0u));
   if (e <= 896u) return __uint_as_float(s);
@@ -28,7 +42,7 @@ __device__ __forceinline__ float approx_f32(double v) {
 // the fp16 hi / lo split of a scaled row keeps).  Larger finite values give
 // the largest float, infinities and NaNs keep their class.
 __device__ __forceinline__ float f64_to_f32_ftz(double v) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+  const unsigned long long b = (unsigned long long)f64_bits(v);
   const uint32_t s = (uint32_t)(b >> 32) & 0x80000000u;
   const uint32_t e = (uint32_t)(b >> 52) & 0x7ffu;
   if (e == 0x7ffu)
@@ -60,17 +74,17 @@ __device__ __forceinline__ double f32_to_f64(float f) {
   const unsigned long long s = (unsigned long long)(u & 0x80000000u) << 32;
   uint32_t e = (u >> 23) & 0xffu, m = u & 0x7fffffu;
   if (e == 0xffu)
-    return __longlong_as_double((long long)(s | 0x7ff0000000000000ull |
+    return bits_f64((long long)(s | 0x7ff0000000000000ull |
                                             ((unsigned long long)m << 29)));
   if (e == 0u) {
-    if (m == 0u) return __longlong_as_double((long long)s);
+    if (m == 0u) return bits_f64((long long)s);
     const int sh = __clz(m) - 8;  // bring the leading one to bit 23
     m = (m << sh) & 0x7fffffu;
     e = 1u - (uint32_t)sh;  // biased float exponent of the normalised value
-    return __longlong_as_double(
+    return bits_f64(
         (long long)(s | ((unsigned long long)(e + 896u) << 52) | ((unsigned long long)m << 29)));
   }
-  return __longlong_as_double(
+  return bits_f64(
       (long long)(s | ((unsigned long long)(e + 896u) << 52) | ((unsigned long long)m << 29)));
 }
 
@@ -85,11 +99,11 @@ static __device__ __noinline__ double scale_pow2_mul(double d, int k) {
 // d * 2^k for a normal d whose result stays normal, by an exponent add;
 // zeros pass through; other cases (subnormal, out of range) multiply.
 __device__ __forceinline__ double scale_pow2(double d, int k) {
-  const long long b = __double_as_longlong(d);
+  const long long b = f64_bits(d);
   if ((b & 0x7fffffffffffffffLL) == 0) return d;
   const int e = (int)((b >> 52) & 0x7ff);
   if (e > 0 && e < 0x7ff && e + k > 0 && e + k < 0x7ff)
-    return __longlong_as_double(b + ((long long)k << 52));
+    return bits_f64(b + ((long long)k << 52));
   return scale_pow2_mul(d, k);
 }
 
@@ -101,7 +115,7 @@ __device__ __forceinline__ double widen_pow2(float f, int k) {
   const uint32_t u = __float_as_uint(f), e = (u >> 23) & 0xffu;
   const int eb = (int)e + 896 + k;  // biased exponent of the result
   if (e - 1u < 254u && eb > 0 && eb < 0x7ff)
-    return __longlong_as_double((long long)(((unsigned long long)(u & 0x80000000u) << 32) |
+    return bits_f64((long long)(((unsigned long long)(u & 0x80000000u) << 32) |
                                             ((unsigned long long)eb << 52) |
                                             ((unsigned long long)(u & 0x7fffffu) << 29)));
   return scale_pow2(f32_to_f64(f), k);
@@ -112,12 +126,12 @@ __device__ __forceinline__ double widen_pow2(float f, int k) {
 // and subnormal d become a signed zero, results above it a signed infinity;
 // infinities and NaNs pass through.
 __device__ __forceinline__ double scale_pow2_ftz(double d, int k) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(d);
+  const unsigned long long b = (unsigned long long)f64_bits(d);
   const unsigned long long s = b & 0x8000000000000000ull;
   const int e = (int)((b >> 52) & 0x7ff), ek = e + k;
   const unsigned long long scaled =
       ek <= 0 ? s : (ek >= 0x7ff ? (s | 0x7ff0000000000000ull) : b + ((unsigned long long)(long long)k << 52));
-  return __longlong_as_double((long long)(e == 0x7ff ? b : (e == 0 ? s : scaled)));
+  return bits_f64((long long)(e == 0x7ff ? b : (e == 0 ? s : scaled)));
 }
 
 // f * 2^k by an exponent add, branch-free: exact while the result stays a

@@ -76,8 +76,19 @@ J3G_FX uint64_t fx_shr(uint64_t v, int n) {
 J3G_FX uint32_t fx_funnel(uint32_t lo, uint32_t hi, int n) { return __funnelshift_r(lo, hi, n); }
 J3G_FX uint32_t fx_bits(float a) { return __float_as_uint(a); }
 J3G_FX float fx_float(uint32_t a) { return __uint_as_float(a); }
-J3G_FX uint64_t fx_bits(double a) { return (uint64_t)__double_as_longlong(a); }
-J3G_FX double fx_double(uint64_t a) { return __longlong_as_double((long long)a); }
+// The bits of a double and back, opaque: where the compiler sees the double
+// behind a mask or a flip of the sign bit it makes them an FP64 absolute value or
+// negation, each of which takes a slot of that pipe.
+J3G_FX uint64_t fx_bits(double a) {
+  uint64_t r;
+  asm("mov.b64 %0, %1;" : "=l"(r) : "d"(a));
+  return r;
+}
+J3G_FX double fx_double(uint64_t a) {
+  double r;
+  asm("mov.b64 %0, %1;" : "=d"(r) : "l"(a));
+  return r;
+}
 J3G_FX float fx_fmaf(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 #else
 J3G_FX uint32_t fx_mulhi(uint32_t a, uint32_t b) { return (uint32_t)((uint64_t)a * b >> 32); }

@@ -63,7 +63,7 @@ inline double sub(double a, double b) { return a - b; }
 // bound): negative values (sign bit set, -0 and -inf included) are below, a
 // NaN of either sign is not, and non-negative doubles order as their bits.
 __device__ __forceinline__ bool lt_eps(double v) {
-  const long long b = __double_as_longlong(v);
+  const long long b = (long long)fx_bits(v);
   constexpr long long kEpsBits = 0x3cb0000000000000ll;  // 2^-52
   return b < 0 ? (b & 0x7fffffffffffffffll) <= 0x7ff0000000000000ll : b < kEpsBits;
 }
@@ -72,7 +72,7 @@ __device__ __forceinline__ bool lt_eps(double v) {
 __device__ __forceinline__ double clamp_eps(double v) { return lt_eps(v) ? kEps : v; }
 
 __device__ __forceinline__ bool normal_positive(double v) {
-  return (uint32_t)((unsigned long long)__double_as_longlong(v) >> 52) - 1u < 0x7feu;
+  return (uint32_t)(fx_bits(v) >> 52) - 1u < 0x7feu;
 }
 
 // All node terms needed by `mask` (bit c set -> component c) for one offset

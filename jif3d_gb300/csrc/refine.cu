@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <cstdint>
 
+#include "fpbits.cuh"
 #include "refine.h"
 
 namespace j3g {
@@ -143,7 +144,7 @@ k_refine_project(RefineMaps m, int nmb, int nblock, int nextra, const double *__
 // 0.0 + v without the FP64 pipe: v itself, except that -0.0 becomes +0.0
 // (the first add of a sum that starts at 0.0, as CombineValues' does).
 __device__ __forceinline__ double zero_plus(double v) {
-  return (__double_as_longlong(v) << 1) == 0 ? 0.0 : v;
+  return (f64_bits(v) << 1) == 0 ? 0.0 : v;
 }
 
 // Combination: one warp per coarse (x, y) row, lanes along coarse z.  The

@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(kThreads)
       unsigned mx = 0;
 #pragma unroll
       for (int b = 0; b < R::blocks; ++b)
-        mx = max(mx, (unsigned)(__double_as_longlong(out[b * R::rows + r]) >> 32) & 0x7fffffffu);
+        mx = max(mx, (unsigned)(f64_bits(out[b * R::rows + r]) >> 32) & 0x7fffffffu);
       // a NaN (station on an edge's line) is noted, and is not the maximum
       const bool nan = mx > 0x7ff00000u;
       mx = __reduce_max_sync(0xffffffffu, nan ? 0u : mx);
@@ -190,7 +190,7 @@ __global__ void k_row_sums(MeshView m, int s0, int ns, const double *__restrict_
 #pragma unroll
     for (int b = 1; b < R::blocks; ++b) v += out[b * R::rows + r];
     const long long row = (long long)(s0 + sl) * R::rows + r;
-    rowsum[row] = rowmax[2 * row + 1] ? __longlong_as_double(0x7ff8000000000000ll) : v;
+    rowsum[row] = rowmax[2 * row + 1] ? bits_f64(0x7ff8000000000000ll) : v;
   }
 }
 
@@ -198,7 +198,7 @@ __global__ void k_row_sums(MeshView m, int s0, int ns, const double *__restrict_
 // x rounded to fp16 (to nearest, as the conversion from double): through a
 // float whose last bit collects what it cuts off.
 __device__ __forceinline__ __half round_half(double x) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  const unsigned long long b = (unsigned long long)f64_bits(x);
   const uint32_t s = (uint32_t)(b >> 32) & 0x80000000u, e = (uint32_t)(b >> 52) & 0x7ffu;
   if (e == 0x7ffu || e >= 1151u) return __double2half(x);
   const uint32_t f = e <= 896u ? 0u : (e - 896u) << 23 | (uint32_t)(b >> 29) & 0x7fffffu;

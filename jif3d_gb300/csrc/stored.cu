@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(kT) k_model_centre(const double *__restrict__ 
 // FP64 operation.  |v| below 2^-126 counts as zero; bad is set for |v| of
 // 2^128 or more (and infinities, NaNs), which the caller takes in FP64.
 __device__ __forceinline__ float centred_f32(double v, float ch, float cl, bool &bad) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+  const unsigned long long b = (unsigned long long)f64_bits(v);
   const uint32_t h = (uint32_t)(b >> 32), l = (uint32_t)b;
   const uint32_t s = h & 0x80000000u, e = (h >> 20) & 0x7ffu;
   bad |= e >= 1151u;
@@ -355,7 +355,7 @@ __global__ void __launch_bounds__(kSplitThreads) k_split_models(
   } else {
     el = INT_MIN / 2;
     for (int j = (int)threadIdx.x; j < jend; j += NT) {
-      const int be = (int)(((unsigned long long)__double_as_longlong(rp[j] - cr) >> 52) & 0x7ff);
+      const int be = (int)(((unsigned long long)f64_bits(rp[j] - cr) >> 52) & 0x7ff);
       if (be) el = max(el, be - 1022 - 14);
     }
   }
@@ -381,7 +381,7 @@ __global__ void __launch_bounds__(kSplitThreads) k_split_models(
   } else {
     // 2^-e as a double (split exponents of finite doubles stay within
     // -1100 .. 1040; beyond the normal range the scaling saturates)
-    const double inv64 = __longlong_as_double((long long)min(2046, max(1, 1023 - e)) << 52);
+    const double inv64 = bits_f64((long long)min(2046, max(1, 1023 - e)) << 52);
     for (int p = (int)threadIdx.x; 2 * p < jn; p += NT) {
       const float x0 = 2 * p < jend ? f64_to_f32_ftz((rp[2 * p] - cr) * inv64) : 0.0f;
       const float x1 = 2 * p + 1 < jend ? f64_to_f32_ftz((rp[2 * p + 1] - cr) * inv64) : 0.0f;
