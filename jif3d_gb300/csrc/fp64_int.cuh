@@ -1,12 +1,12 @@
-// fp64_int.cuh -- correctly rounded FP64 square roots and quotients on the
-// integer pipes, bit for bit what the FP64 instructions' sequences round to.
+// fp64_int.cuh -- correctly rounded FP64 square roots, quotients and sums on the
+// integer pipes, bit for bit what the FP64 instructions round to.
 //
-// The GB300 starts an FP64 instruction every 16 cycles per SM, and a square root
-// or a quotient takes five to ten of them; a kernel bound by that pipe has the
-// issue slots for the 50 integer instructions that each takes here.  (A sum or a
-// product does not pay: its 49 integer instructions cost twice its one FP64
-// instruction.)  Both go from an FP32 estimate and one Newton step of 32 bits to
-// a result within one unit, and an exact remainder decides its last bit.
+// The GB300 starts an FP64 instruction every 16 cycles per SM.  A square root or
+// a quotient takes five to ten of them and 50 integer instructions here; a sum
+// takes 65 integer instructions, about 20 cycles of the SM's integer pipe, so
+// moving a part of the sums of a kernel bound by FP64 uses both pipes.  Roots and
+// quotients go from an FP32 estimate and one Newton step of 32 bits to a result
+// within one unit, and an exact remainder decides the last bit.
 #pragma once
 #include "node_fixed.cuh"
 
@@ -26,6 +26,46 @@ J3G_FX double int_to_double(int64_t v, int scale) {
   const int n = int_clz64(a);
   const uint64_t m = (a << n) >> 11;
   return fx_double(fx_pair(fx_hi(m) + ((uint32_t)(1085 - scale - n) << 20) | neg << 31, fx_lo(m)));
+}
+
+// The operands that int_add leaves to the FP64 instruction.  Out of line: a
+// predicated FP64 instruction takes its slot of the pipe in every lane's absence.
+#ifdef __CUDACC__
+static __device__ __noinline__ double int_add_rare(double a, double b) { return __dadd_rn(a, b); }
+J3G_FX uint64_t int_shl(uint64_t v, int n) {  // zero for n of 64 and more
+  uint64_t r;
+  asm("shl.b64 %0, %1, %2;" : "=l"(r) : "l"(v), "r"(n));
+  return r;
+}
+#else
+J3G_FX double int_add_rare(double a, double b) { return a + b; }
+J3G_FX uint64_t int_shl(uint64_t v, int n) { return (uint32_t)n > 63u ? 0 : v << n; }
+#endif
+
+J3G_FX double int_neg(double a) { return fx_double(fx_bits(a) ^ 1ull << 63); }
+
+// a + b
+J3G_FX double int_add(double a, double b) {
+  const uint64_t A = fx_bits(a), B = fx_bits(b), kAbs = 0x7fffffffffffffffull;
+  const bool swap = (A & kAbs) < (B & kAbs);
+  const uint64_t x = swap ? B : A, y = swap ? A : B;
+  const uint32_t xh = fx_hi(x), yh = fx_hi(y);
+  const uint32_t ex = xh >> 20 & 0x7ffu, ey = yh >> 20 & 0x7ffu;
+  if (ey == 0 || ex - 64u >= 0x7feu - 64u) return int_add_rare(a, b);
+  // ten bits below the larger operand's last one, the rest of the smaller as a
+  // sticky bit: it is only ever set where at most one bit cancels
+  const uint64_t my = ((y & kIntFrac) | kIntOne) << 10;
+  const int d = (int)(ex - ey);
+  uint64_t s = fx_shr(my, d);
+  s |= int_shl(s, d) != my;
+  const uint64_t neg = (uint64_t)(int64_t)((int32_t)(xh ^ yh) >> 31);
+  const uint64_t m = (((x & kIntFrac) | kIntOne) << 10) + ((s ^ neg) - neg);
+  if (m == 0) return 0.0;
+  const int n = int_clz64(m);
+  const uint64_t t = m << n;
+  uint64_t r = t >> 11;
+  r += (fx_lo(t) & 0x7ffu) + (fx_lo(r) & 1u) > 0x400u;  // a carry out raises the exponent
+  return fx_double(fx_pair(fx_hi(r) + (ex - (uint32_t)n << 20) | (xh & 0x80000000u), fx_lo(r)));
 }
 
 // sqrt of a positive normal x: with X = x 4^-h in [1, 4) the 53-bit integer z

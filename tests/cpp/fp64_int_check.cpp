@@ -63,5 +63,24 @@ int main() {
     bad += fx_bits(int_to_double(v, scale)) != fx_bits(std::ldexp((double)v, -scale));
   }
   std::printf("convert %lld %lld\n", bad, kN);
+  bad = 0;
+  for (long long i = 0; i < kN; ++i) {
+    // exponents anywhere, gaps of 2 and of 35 at most; specials; cancellation
+    const int e = (int)(next() % 2046) + 1, gap = (int)(next() % (i & 1 ? 4 : 70)) - (i & 1 ? 2 : 35);
+    const int f = e + gap < 0 ? 0 : e + gap > 2047 ? 2047 : e + gap;
+    double a = fx_double((next() & 1) << 63 | (uint64_t)e << 52 | fraction());
+    double b = fx_double((next() & 1) << 63 | (uint64_t)f << 52 | fraction());
+    static const double special[] = {0.0, -0.0, INFINITY, -INFINITY, NAN, 5e-324, -2e-308, 1.7e308};
+    if (i % 16 == 0) b = special[next() % 8];
+    if (i % 16 == 1) b = fx_double(fx_bits(a) ^ 1ull << 63 ^ next() % 3);
+    if (i & 8) {
+      const double t = a;
+      a = b;
+      b = t;
+    }
+    const double got = int_add(a, b), want = a + b;
+    bad += fx_bits(got) != fx_bits(want) && !(std::isnan(got) && std::isnan(want));
+  }
+  std::printf("add %lld %lld\n", bad, kN);
   return 0;
 }

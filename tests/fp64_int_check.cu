@@ -1,6 +1,6 @@
 // Device check of fp64_int.cuh and of the functions that use it: square roots
 // against the FP64 instruction, flog, fatan2 and fatan2_pair with SPLIT against
-// themselves without.  Prints one line "name mismatches tested" per check.
+// themselves without, sums against the instruction.  Prints one line "name mismatches tested" per check.
 #include <cstdio>
 #include <cuda_runtime.h>
 
@@ -34,6 +34,14 @@ __global__ void k_check(int which, unsigned long long n, unsigned long long *bad
     } else if (which == 1) {
       const double x = i & 1 ? value(r, 1, 2046) : value(r, 1021, 4);
       nb += !same(flog<true>(x), flog<false>(x));
+    } else if (which == 3) {
+      double x = value(r, 950, 100), y = value(s, i & 1 ? 1000 : 940, i & 1 ? 3 : 130);
+      if (r >> 63) x = -x;
+      if (s >> 63) y = -y;
+      if (i % 32 == 7) y = -x;
+      if (i % 32 == 8) y = 0.0;
+      if (i % 32 == 9) y *= 0x1p-1000;
+      nb += !same(int_add(x, y), __dadd_rn(x, y)) + !same(int_add(y, int_neg(x)), __dsub_rn(y, x));
     } else {
       // ratios near 1, over the breakpoints, tiny; every quadrant; zeros
       double y = value(r, 1000, i % 3 == 0 ? 2 : 40), x = value(s, 1000, 2);
@@ -51,14 +59,14 @@ __global__ void k_check(int which, unsigned long long n, unsigned long long *bad
 }
 
 int main() {
-  const char *names[] = {"sqrt", "log", "atan2"};
+  const char *names[] = {"sqrt", "log", "atan2", "add"};
   unsigned long long *bad;
-  if (cudaMalloc(&bad, 3 * sizeof *bad) != cudaSuccess) return 1;
-  cudaMemset(bad, 0, 3 * sizeof *bad);
+  if (cudaMalloc(&bad, 4 * sizeof *bad) != cudaSuccess) return 1;
+  cudaMemset(bad, 0, 4 * sizeof *bad);
   const unsigned long long n = 1ull << 27;
-  for (int w = 0; w < 3; ++w) k_check<<<1216, 256>>>(w, n, bad + w);
-  unsigned long long h[3];
+  for (int w = 0; w < 4; ++w) k_check<<<1216, 256>>>(w, n, bad + w);
+  unsigned long long h[4];
   if (cudaMemcpy(h, bad, sizeof h, cudaMemcpyDeviceToHost) != cudaSuccess) return 1;
-  for (int w = 0; w < 3; ++w) std::printf("%s %llu %llu\n", names[w], h[w], n);
+  for (int w = 0; w < 4; ++w) std::printf("%s %llu %llu\n", names[w], h[w], n);
   return 0;
 }

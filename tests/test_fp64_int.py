@@ -1,4 +1,4 @@
-"""Square roots, quotients and conversions on the integer pipes (fp64_int.cuh):
+"""Square roots, quotients, sums and conversions on the integer pipes (fp64_int.cuh):
 on the host against the processor's FP64, and on the device, with the logarithm
 and the arctangent that use them, against their FP64 forms.  Bit for bit."""
 import os
@@ -27,11 +27,11 @@ def _run(cmd, names):
 def test_host_bit_exact(tmp_path):
     _run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-I", B.CSRC,
           os.path.join(HERE, "cpp", "fp64_int_check.cpp"), "-o", str(tmp_path / "check")],
-         ["sqrt", "quotient", "convert"])
+         ["sqrt", "quotient", "convert", "add"])
 
 
 @pytest.mark.gpu
 def test_device_bit_exact(tmp_path):
     _run([B.nvcc(), "-O3", "-std=c++17", B.ARCH, "-I", B.CSRC,
           os.path.join(HERE, "fp64_int_check.cu"), "-o", str(tmp_path / "check")],
-         ["sqrt", "log", "atan2"])
+         ["sqrt", "log", "atan2", "add"])
