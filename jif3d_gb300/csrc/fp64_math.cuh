@@ -15,9 +15,9 @@
 //              |y| > |x|, pi - that when x is negative, the sign of y;
 //              about 20 FP64 operations; fatan2_pair gives atan2(y, x) and
 //              atan2(x, y) from one ratio and series.
-// With SPLIT the quotient and the exact differences are integer work too
-// (fp64_int.cuh), six FP64 operations fewer in the arctangent and one in the
-// logarithm: the same values (the FP64 quotient may miss the nearest double once
+// With SPLIT the quotient, the exact differences and the last sums are integer
+// work too (fp64_int.cuh), ten FP64 operations fewer in the arctangent and three
+// in the logarithm: the same values (the FP64 quotient may miss the nearest double once
 // in 2^39 operands).
 // Both are within about one unit in the last place of the exact value; the
 // tables come from gen_fp64_tables.py.  Zeros are handled in the fast path of
@@ -74,6 +74,7 @@ __device__ __forceinline__ double flog(double x) {
   const double hi = __fma_rn(kd, fp64tab::kLn2Lead, __ldg(row + 1));
   double lo = __fma_rn(kd, fp64tab::kLn2Trail, __ldg(row + 2));
   lo = __fma_rn(__dmul_rn(u, u), q, lo);  // + u^2 q, rounded once
+  if constexpr (SPLIT) return int_add(hi, int_add(lo, u));
   lo = __dadd_rn(lo, u);
   return __dadd_rn(hi, lo);
 }
@@ -136,14 +137,28 @@ __device__ __forceinline__ bool atan_ratio(unsigned long long ay, unsigned long 
   double p = __ldg(a + 9);
 #pragma unroll
   for (int n = 8; n >= 2; --n) p = __fma_rn(p, d, __ldg(a + n));
-  ta = __dadd_rn(__ldg(a), __fma_rn(d, p, __ldg(a + 1)));
+  const double low = __fma_rn(d, p, __ldg(a + 1));
+  ta = SPLIT ? int_add(__ldg(a), low) : __dadd_rn(__ldg(a), low);
   return true;
+}
+
+// pi - t, out of line: predicated FP64 instructions take their slots where no
+// lane wants them, and the abscissa's sign is mostly one for a warp.
+static __device__ __noinline__ double from_pi(double t) {
+  return __dadd_rn(fp64tab::kPiHi, __fma_rn(-1.0, t, fp64tab::kPiLo));
 }
 
 // The angle of (x, y) from atan t: pi/2 - atan t when |y| > |x|, pi minus
 // that when x is negative (sign bit), with the sign of y.
+template <bool SPLIT>
 __device__ __forceinline__ double atan2_octant(double ta, bool swap, unsigned long long bx,
                                                unsigned long long by) {
+  if constexpr (SPLIT) {
+    double th = ta;
+    if (swap) th = int_add(fp64tab::kPio2Hi, int_add(fp64tab::kPio2Lo, int_neg(th)));
+    if (bx >> 63) th = from_pi(th);
+    return fx_double(fx_bits(th) | (by & 0x8000000000000000ull));
+  }
   double th = swap ? __dadd_rn(fp64tab::kPio2Hi, __fma_rn(-1.0, ta, fp64tab::kPio2Lo)) : ta;
   if (bx >> 63) th = __dadd_rn(fp64tab::kPiHi, __fma_rn(-1.0, th, fp64tab::kPiLo));
   return fx_double(fx_bits(th) | (by & 0x8000000000000000ull));
@@ -156,7 +171,7 @@ __device__ __forceinline__ double fatan2(double y, double x) {
   const unsigned long long ay = by & 0x7fffffffffffffffull, ax = bx & 0x7fffffffffffffffull;
   double ta;
   if (!atan_ratio<SPLIT>(ay, ax, ta)) return atan2(y, x);
-  return atan2_octant(ta, ay > ax, bx, by);
+  return atan2_octant<SPLIT>(ta, ay > ax, bx, by);
 }
 
 // fatan2(y, x) and fatan2(x, y) with one shared ratio and series: the two
@@ -172,8 +187,8 @@ __device__ __forceinline__ void fatan2_pair(double y, double x, double &yx, doub
     xy = atan2(x, y);
     return;
   }
-  yx = atan2_octant(ta, ay > ax, bx, by);
-  xy = atan2_octant(ta, ax > ay, by, bx);
+  yx = atan2_octant<SPLIT>(ta, ay > ax, bx, by);
+  xy = atan2_octant<SPLIT>(ta, ax > ay, by, bx);
 }
 
 }  // namespace j3g

@@ -77,8 +77,8 @@ __device__ __forceinline__ bool normal_positive(double v) {
 
 // All node terms needed by `mask` (bit c set -> component c) for one offset
 // (dx, dy, dz) = station - node.  One square root serves every component.
-// SPLIT: the same values, the square root, the quotients and the exact
-// differences on the integer pipes.
+// SPLIT: the same values, the square root, the quotients, the exact differences
+// and some of the sums on the integer pipes.
 template <int MASK, bool SPLIT = false>
 __device__ __forceinline__ void node_terms(double dx, double dy, double dz, double *out) {
   // fused: the node terms need r to FP64 accuracy, not the reference's
@@ -92,7 +92,8 @@ __device__ __forceinline__ void node_terms(double dx, double dy, double dz, doub
     // ln(dx + r) and ln(dy + r) are shared by g_z and the Uyz / Uxz terms when
     // r >= eps (then g_z's clamped r equals the raw r).
     const double rg = clamp_eps(r);
-    const double sx = add(dx, rg), sy = add(dy, rg);
+    const double sx = SPLIT ? int_add(dx, rg) : add(dx, rg);
+    const double sy = SPLIT ? int_add(dy, rg) : add(dy, rg);
     lx = flog<SPLIT>(sx);
     ly = flog<SPLIT>(sy);
     if (need_gz) {
@@ -111,7 +112,7 @@ __device__ __forceinline__ void node_terms(double dx, double dy, double dz, doub
     if (need_off) {
       const bool shared = !lt_eps(r);
       const double ax = shared ? sx : add(dx, r), ay = shared ? sy : add(dy, r);
-      const double az = add(dz, r);
+      const double az = SPLIT ? int_add(dz, r) : add(dz, r);
       const double log_eps = fp64tab::kLogDblEps;  // log(DBL_EPSILON)
       if (MASK & (1 << NC_YZ))
         out[NC_YZ] = lt_eps(ax) ? log_eps : (shared ? lx : flog<SPLIT>(ax));

@@ -219,7 +219,9 @@ __global__ void k_row_sums(MeshView m, int s0, int ns, const double *__restrict_
 __device__ __forceinline__ __half round_half(double x) {
   const unsigned long long b = (unsigned long long)f64_bits(x);
   const uint32_t s = (uint32_t)(b >> 32) & 0x80000000u, e = (uint32_t)(b >> 52) & 0x7ffu;
-  if (e == 0x7ffu || e >= 1151u) return __double2half(x);
+  if (e >= 1151u)  // infinities, NaNs, beyond the range of floats
+    return __ushort_as_half(e == 0x7ffu && (b & 0xfffffffffffffull)
+                                ? (unsigned short)0x7fff : (unsigned short)(s >> 16 | 0x7c00u));
   const uint32_t f = e <= 896u ? 0u : (e - 896u) << 23 | (uint32_t)(b >> 29) & 0x7fffffu;
   return __float2half_rn(__uint_as_float(s | f | ((b & 0x1fffffffull) != 0 && f ? 1u : 0u)));
 }
