@@ -51,7 +51,6 @@ J3G_FX double int_add(double a, double b) {
   const uint64_t x = swap ? B : A, y = swap ? A : B;
   const uint32_t xh = fx_hi(x), yh = fx_hi(y);
   const uint32_t ex = xh >> 20 & 0x7ffu, ey = yh >> 20 & 0x7ffu;
-  if (ey == 0 || ex - 64u >= 0x7feu - 64u) return int_add_rare(a, b);
   // ten bits below the larger operand's last one, the rest of the smaller as a
   // sticky bit: it is only ever set where at most one bit cancels
   const uint64_t my = ((y & kIntFrac) | kIntOne) << 10;
@@ -60,8 +59,9 @@ J3G_FX double int_add(double a, double b) {
   s |= int_shl(s, d) != my;
   const uint64_t neg = (uint64_t)(int64_t)((int32_t)(xh ^ yh) >> 31);
   const uint64_t m = (((x & kIntFrac) | kIntOne) << 10) + ((s ^ neg) - neg);
-  if (m == 0) return 0.0;
-  const int n = int_clz64(m);
+  // zeros, subnormals, ends of the range, and 30 bits and more cancelled
+  if (ey == 0 || ex - 64u >= 0x7feu - 64u || fx_hi(m) == 0) return int_add_rare(a, b);
+  const int n = fx_clz(fx_hi(m));
   const uint64_t t = m << n;
   uint64_t r = t >> 11;
   r += (fx_lo(t) & 0x7ffu) + (fx_lo(r) & 1u) > 0x400u;  // a carry out raises the exponent
