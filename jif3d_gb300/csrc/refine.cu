@@ -4,7 +4,9 @@
 // so their results are bit-identical to it.
 #include <algorithm>
 #include <cstdint>
+#include <type_traits>
 
+#include "fp64_int.cuh"
 #include "fpbits.cuh"
 #include "refine.h"
 
@@ -154,13 +156,14 @@ __device__ __forceinline__ double zero_plus(double v) {
 // ModelRefiner.cpp:114-122), bit for bit.  The adds run on GB300's narrow
 // FP64 pipe, which bounds this kernel: each (row, z slot) costs one warp-wide
 // add, so KR > 0 unrolls the z run to exactly its longest length, the first
-// add of every sum (onto 0.0) is done with integer operations, and the loads
-// of RB rows, the first included, are issued before their adds.  KR = 0 runs
-// any length.  Five blocks to an SM: 128 models of 64 x 64 x 32 cells from
-// twice refined gradients 340 -> 300 us (with the first row's loads waited for
-// on their own, four blocks); the seven adds per cell alone are 240 us.
+// add of every sum (onto 0.0) and one of the second row's are done with integer
+// operations, and the loads of RB rows are issued before their adds.  KR = 0 runs
+// any length.  128 models of 64 x 64 x 32 cells from twice refined gradients 340
+// -> 207 us (1.2 GB, 180 us): 300 with the first row's loads ahead of its adds
+// too, 240 without the FP64 comparison and the predicated add that the first
+// value had cost, 220 with code of their own for it at four blocks to an SM.
 template <int KR>
-__global__ void __launch_bounds__(kThreads, 5)
+__global__ void __launch_bounds__(kThreads, 4)
 k_refine_combine(RefineMaps m, int nmb, int nblock, int nextra, const double *__restrict__ fine,
                  double *__restrict__ coarse, long long cngrid, long long fngrid) {
   constexpr int RB = KR == 0 ? 1 : (KR <= 2 ? 4 : 2);
@@ -203,7 +206,9 @@ k_refine_combine(RefineMaps m, int nmb, int nblock, int nextra, const double *__
           }
         } else if (nr > 0) {
           int i = 0, j = 0;
-          for (int r0 = 0; r0 < nr; r0 += RB) {
+          // rows r0 .. r0 + RB - 1; the first value of all starts the sum (in
+          // code of its own: a predicated add takes its slot all the same)
+          auto rows = [&](int r0, auto first) {
             double v[RB][KU];
 #pragma unroll
             for (int r = 0; r < RB; ++r) {
@@ -221,13 +226,17 @@ k_refine_combine(RefineMaps m, int nmb, int nblock, int nextra, const double *__
 #pragma unroll
                 for (int u = 0; u < KU; ++u)
                   if (u < nk) {
-                    if (r == 0 && u == 0 && r0 == 0)
+                    if (decltype(first)::value && r == 0 && u == 0)
                       sum = zero_plus(v[r][u]);
+                    else if (u == 1 && r == 1)
+                      sum = int_add(sum, v[r][u]);
                     else
                       sum += v[r][u];
                   }
               }
-          }
+          };
+          rows(0, std::true_type{});
+          for (int r0 = RB; r0 < nr; r0 += RB) rows(r0, std::false_type{});
         }
         if (ck < cn2) dst[(long long)crow * cn2 + ck] = sum;
       }

@@ -323,3 +323,33 @@ def test_cpp_refiner(oracle_lib, tmp_path):
     assert same_bits(out["coarse_grad"], ref_grad)
     assert same_bits(out["copy_grad"], ref_grad)
     assert exc
+
+
+@pytest.mark.parametrize("runs", [2, 3, 4])
+def test_combine_special_values(ctx, oracle_lib, runs):
+    """Sums with zeros of both signs, subnormals, the ends of the range,
+    infinities, NaNs and cancellation in every place, bit for bit (a NaN as a
+    NaN): one of a cell's sums is integer work and leaves these to the FP64 pipe."""
+    import torch
+    s = small_survey(W.SCALAR, seed=63, nx=5, ny=4, nz=6, bg=False, origin=(0.0, 0.0, 0.0))
+    s = dataclasses.replace(s, xsize=np.full(5, 12.0), ysize=np.full(4, 12.0),
+                            zsize=np.full(6, 12.0), model=np.zeros(120))
+    f = refine(s, [np.arange(0.0, 61.0, 6.0), np.arange(0.0, 49.0, 6.0),
+                   np.arange(0.0, 73.0, 12.0 / runs)])
+    fine_setup(ctx, s, f)
+    rng = np.random.default_rng(64)
+    special = np.array([0.0, -0.0, 5e-324, -2e-308, 1.7e308, -1.7e308, np.inf, -np.inf, np.nan,
+                        1.0, -1.0, 1.0 + 2.0 ** -52, 2.0 ** 53, -2.0 ** 53])
+    G = rng.normal(size=(6, f.ngrid))
+    for i in range(1, 6):  # more and more of them
+        take = rng.random(f.ngrid) < 0.1 * i
+        G[i, take] = rng.choice(special[:6] if i < 3 else special, take.sum())
+    dG, dOut = torch.tensor(G, device="cuda"), torch.zeros((6, 120), dtype=torch.float64,
+                                                           device="cuda")
+    ctx.refine_combine_device(6, dG.data_ptr(), dOut.data_ptr())
+    ctx.synchronize()
+    for i in range(6):
+        out, ref = dOut[i].cpu().numpy(), oracle_combine(oracle_lib, s, f, G[i], 1, 0)
+        nan = np.isnan(ref)
+        assert np.array_equal(np.isnan(out), nan)
+        assert same_bits(np.where(nan, 0.0, out), np.where(nan, 0.0, ref))
