@@ -356,9 +356,12 @@ J3G_FX FxAngle fx_atan(uint64_t n1, int s, uint64_t D, float t, float idy, const
 
 // atan2 from the angle of the magnitudes: `own` the sign of the abscissa's
 // offset, neg the sign of the ordinate.  Zero angles come from zero offsets.
+// CONVERT: by the conversion instruction.
+template <bool CONVERT = false>
 J3G_FX double fx_quadrant(uint64_t v, int scale, uint64_t v61, uint32_t own, uint32_t neg) {
   const uint64_t w = own ? nodetab::kPiS61 - v61 : v;
-  const double d = fx_to_double(w, own ? 61 : scale, neg);
+  const double d = CONVERT ? fx_convert((int64_t)w, own ? 61 : scale, neg)
+                           : fx_to_double(w, own ? 61 : scale, neg);
   return fx_hi(w) == 0 ? fx_double((uint64_t)neg << 63) : d;
 }
 
@@ -399,6 +402,9 @@ J3G_FX bool fx_node(const FxColumn &c, const FxAxis &z, const FxTables &T, doubl
     l = l < kFxLogEps || (c.axial && z.neg) ? kFxLogEps : l;
     out[4] = fx_convert(l, 57, 0);
   }
+  // without g_z and Uzz the FP64 pipe has room for the angles' conversions
+  // (total-field anomaly 8.79 -> 8.65 ms; with them joint 8.22 -> 8.36)
+  constexpr bool kConvert = !need_gz && !ZZ;
   const uint64_t R4 = r.R << 2;
   uint64_t az = 0;  // the angle of z, scale 2^61
   if constexpr (need_xx || need_yy) {
@@ -417,7 +423,7 @@ J3G_FX bool fx_node(const FxColumn &c, const FxAxis &z, const FxTables &T, doubl
     const FxAngle aM = fx_atan(n2, eM - c.ehi + e0, D2, fr * c.fhi * fx_rcp(fM), imM * r.ys, T);
     const uint64_t am = c.axial ? 0 : nodetab::kPio2S61 - ah.v61 - aM.v61;  // the complement
     az = zbig ? aM.v61 : am;
-    const double Fh = fx_quadrant(ah.v, ah.scale, ah.v61, c.neghi, c.neglo ^ z.neg);
+    const double Fh = fx_quadrant<kConvert>(ah.v, ah.scale, ah.v61, c.neghi, c.neglo ^ z.neg);
     double Fl;
     if constexpr (ZZ) {
       const uint32_t negM = zbig ? z.neg : c.neglo, negm = zbig ? c.neglo : z.neg;
@@ -427,8 +433,8 @@ J3G_FX bool fx_node(const FxColumn &c, const FxAxis &z, const FxTables &T, doubl
       Fl = zbig ? Fm : FM;
       out[3] = zbig ? FM : Fm;
     } else {
-      Fl = fx_quadrant(zbig ? am : aM.v, zbig ? 61 : aM.scale, zbig ? am : aM.v61, c.neglo,
-                       c.neghi ^ z.neg);
+      Fl = fx_quadrant<kConvert>(zbig ? am : aM.v, zbig ? 61 : aM.scale, zbig ? am : aM.v61,
+                                 c.neglo, c.neghi ^ z.neg);
     }
     out[1] = c.yhi ? Fl : Fh;
     out[2] = c.yhi ? Fh : Fl;
