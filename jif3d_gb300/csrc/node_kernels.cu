@@ -179,12 +179,13 @@ __global__ void __launch_bounds__(kNodeThreads, kNodeResident)
 }
 
 // Adjoint: block x covers blockDim columns and kper nodes of each, block y a
-// chunk of stations, staged kAdjStage at a time; the sums of a thread's nodes
+// chunk of stations from chunk0 on, staged kAdjStage at a time; the sums of a thread's nodes
 // are in shared memory, so that the node loop need not be unrolled.
 template <int KIND>
 __global__ void __launch_bounds__(kNodeThreads, kNodeResident)
     k_node_adjoint(MeshView m, StationView st, const double *__restrict__ W, int kper, int nkc,
-                   int spc, const int *__restrict__ chunk_start, double *__restrict__ Gpart) {
+                   int spc, const int *__restrict__ chunk_start, int chunk0,
+                   double *__restrict__ Gpart) {
   using T = KindTraits<KIND>;
   constexpr int MASK = T::mask;
   constexpr int NCMP = T::ncomp;
@@ -219,7 +220,7 @@ __global__ void __launch_bounds__(kNodeThreads, kNodeResident)
   const double X = m.X[i], Y = m.Y[j];
   // stations of this chunk: spc apiece, or the ranges of chunk_start (chunks
   // that never straddle a station subset)
-  const int chunk = blockIdx.y;
+  const int chunk = chunk0 + blockIdx.y;
   const int s0 = chunk_start ? chunk_start[chunk] : chunk * spc;
   const int s1 = chunk_start ? chunk_start[chunk + 1] : min(st.n, s0 + spc);
   for (int k = 0; k < nk; ++k)
@@ -368,16 +369,22 @@ NodeForwardPlan node_forward_plan(int nx, int ny, int nz, int nmeas, long long m
 }
 
 template <int KIND>
-static cudaError_t adjoint_launch(dim3 grid, int threads, size_t smem, cudaStream_t st, const MeshView &m,
-                           const StationView &s, const double *W, const NodeAdjointPlan &p,
-                           const int *chunk_start, double *Gpart) {
+static cudaError_t adjoint_launch(int blocks, int nchunk, size_t smem, cudaStream_t st,
+                                  const MeshView &m, const StationView &s, const double *W,
+                                  const NodeAdjointPlan &p, const int *chunk_start,
+                                  double *Gpart) {
   if (smem > 16384) {  // three model blocks: beyond 48 KB with the tables, by opt-in
     const cudaError_t e = cudaFuncSetAttribute(
         k_node_adjoint<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  return launch_chained(k_node_adjoint<KIND>, grid, threads, smem, st, m, s, W, p.kper, p.nkc,
-                        p.spc, chunk_start, Gpart);
+  for (int c0 = 0; c0 < nchunk; c0 += 65535) {  // grid y
+    const dim3 grid(blocks, std::min(65535, nchunk - c0));
+    const cudaError_t e = launch_chained(k_node_adjoint<KIND>, grid, p.threads, smem, st, m, s, W,
+                                         p.kper, p.nkc, p.spc, chunk_start, c0, Gpart);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 #define J3G_NODE_DISPATCH(kind, ...)                                             \
@@ -454,9 +461,8 @@ cudaError_t launch_node_adjoint(int kind, const MeshView &m, const StationView &
                                 const double *W, const NodeAdjointPlan &p, int nchunk,
                                 const int *chunk_start, double *Gpart, cudaStream_t st) {
   const int ncb = cdiv((long long)(m.nx + 1) * (m.ny + 1), p.threads);
-  const dim3 grid(ncb * p.nkc, nchunk);
   const size_t smem = sizeof(double) * (size_t)kind_nblock(kind) * p.kper * p.threads;
-  J3G_NODE_DISPATCH(kind, return adjoint_launch<K>(grid, p.threads, smem, st, m, s, W, p,
+  J3G_NODE_DISPATCH(kind, return adjoint_launch<K>(ncb * p.nkc, nchunk, smem, st, m, s, W, p,
                                                    chunk_start, Gpart));
   return cudaGetLastError();
 }

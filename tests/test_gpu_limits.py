@@ -104,3 +104,30 @@ def test_stored_adjoint_more_cells_than_grid_y(ctx):
         assert relerr(ctx.batched_lqderivative(s.model[None, :], mis[None, :])[0], g64) <= TOL
     finally:
         ctx.drop_sensitivity()
+
+
+def test_fp64_adjoint_more_chunks_than_grid_y(ctx):
+    """1.1 million stations: more chunks of 16 in the node adjoint than 65535;
+    and 70000 subsets of them, more than grid z, with gradients of their own."""
+    import torch
+    s = small_survey(W.SCALAR, seed=303, nx=3, ny=3, nz=2, nmeas=1000, bg=False)
+    copies = 1100
+    W.setup_context(ctx, s)
+    mis1 = np.random.default_rng(9).normal(size=1000)
+    g1 = ctx.lqderivative(s.model, mis1)
+    one = np.array([ctx.lqderivative(s.model, np.where(np.arange(1000) == i, mis1, 0.0))
+                    for i in range(3)])
+    big = tiled(s, copies)
+    W.setup_context(ctx, big)
+    assert relerr(ctx.lqderivative(big.model, np.tile(mis1, copies)), copies * g1) <= TOL64
+    n = 70000
+    subsets = [np.array([i % 3]) for i in range(n)]
+    like = dict(dtype=torch.float64, device="cuda")
+    m, r = torch.tensor(s.model, **like), torch.tensor(np.tile(mis1[:3], n // 3 + 1)[:n], **like)
+    g = torch.zeros(n, s.nparm, **like)
+    W.setup_context(ctx, s)
+    torch.cuda.synchronize()
+    ctx.subsets_lqderivative_device(subsets, m.data_ptr(), r.data_ptr(), g.data_ptr())
+    ctx.synchronize()
+    for i in range(3):
+        assert relerr(g[i::3].cpu().numpy(), np.broadcast_to(one[i], g[i::3].shape)) <= TOL64
