@@ -204,6 +204,8 @@ k_refine_combine(RefineMaps m, int nmb, int nblock, int nextra, const double *__
             }
             if (++j == nj) j = 0, ++i;
           }
+        } else if (KR == 1 && nr == 1) {  // a copy: 128 cells 2.24 us, not 2.40
+          if (nk > 0) sum = zero_plus(row00[k0]);
         } else if (nr > 0) {
           int i = 0, j = 0;
           // rows r0 .. r0 + RB - 1; the first value of all starts the sum (in
