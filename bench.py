@@ -58,14 +58,14 @@ SIGMA_GZ, SIGMA_U = 1e-8, 1e-9
 # denominator beside the library's own measured FMA rate.
 FP64_NOMINAL_GFLOPS = 1250.0
 
-# FP64 flops per joint node evaluation (an FMA counts 2): 21 add/mul + sqrt +
-# 3 flog + 2 fatan2 + 1 fatan2_pair + 7 accumulation FMA, with the FP64
-# instruction weights of the device functions counted by ncu on
-# microkernels of each function (sqrt 13, flog 21, fatan2 36, fatan2_pair 42);
-# the node kernels' own counters give 223 (forward) and 214 (adjoint).
+# FP64 flops per joint node evaluation in FP64 instructions (an FMA counts 2):
+# 21 add/mul + sqrt + 3 flog + 2 fatan2 + 1 fatan2_pair + 7 accumulation FMA,
+# with the weights of the device functions counted by ncu on microkernels of
+# each function (sqrt 13, flog 21, fatan2 36, fatan2_pair 42).  The node kernels
+# evaluate the terms in 64-bit fixed point on the integer pipes, so these rates
+# are FP64-equivalent ones, several times the FP64 pipe's, not a utilisation.
 FP64_FLOP_PER_JOINT_NODE = 225.0
-# FP64 flops per node evaluation of the other kinds, counted by ncu
-# (DFMA = 2, DADD, DMUL) on the node kernels, mean of forward and adjoint
+# the same of the other kinds, mean of forward and adjoint
 FP64_FLOP_PER_NODE = {1: 110.0, 2: 210.0, 3: 208.0, 4: FP64_FLOP_PER_JOINT_NODE}
 
 
@@ -411,9 +411,10 @@ def measure_fp64_configs(stream, flush, local, cpu):
     FTG on 96 x 96 x 48 (2500 stations), and the total-field anomaly on
     128 x 128 x 64 over all 32 uneven station subsets (74,753 stations in one
     subsets forward and one subsets adjoint call; no warm-up, one call each,
-    ~40 s).  FP64 roofline: node evaluations x FP64 flops per node of the
-    kind / time, against the library's measured FP64 FMA rate and against the
-    nominal rate.  Beside each, the oracle's OpenMP forward and LQDerivative
+    a few seconds).  fp64_gflops: node evaluations x the FP64 flops that a node
+    of the kind takes in FP64 instructions / time, beside the library's measured
+    FP64 FMA rate and the nominal one (above them: most of it is integer work).
+    Beside each, the oracle's OpenMP forward and LQDerivative
     on the host cores (all stations of the g_z survey, 64 seeded stations of
     the others)."""
     import torch
@@ -481,7 +482,8 @@ def measure_fp64_configs(stream, flush, local, cpu):
                                f"uses the nominal {FP64_NOMINAL_GFLOPS:.0f} GFLOP/s")
     out["how"] = ("forward and adjoint of one model, each timed on its own; fp64_frac counts "
                   "node evaluations only (the background, reductions and assembly are in the "
-                  "time)")
+                  "time), in FP64-equivalent flops: the kernels evaluate most of a node in "
+                  "fixed point, so it is above 1")
     return out
 
 
@@ -907,6 +909,8 @@ def run_plain(args, rank, world, local):
         "roofline": {"bound": "fp64", "achieved": achieved, "peak": peak, "unit": "GFLOP/s",
                      "frac": achieved / peak, "traffic": None,
                      "kernel": "k_node_forward<JOINT> / k_node_adjoint<JOINT>",
+                     "achieved_in": "FP64-equivalent flops (the node terms are evaluated in "
+                                    "fixed point on the integer pipes)",
                      "peak_source": "measured FP64 FMA probe (MEASURED_PEAKS.json has no FP64 "
                                     "entry)"},
         "clocks": clk,

@@ -5,10 +5,12 @@
 // Work is split into node columns (fixed x and y): a thread takes one column
 // and walks its nodes, so that dx, dy and dx^2 + dy^2 are formed once per
 // column and station and the z offsets once per block and station (in shared
-// memory), instead of once per node.  The terms come from node_fixed.cuh.
+// memory), instead of once per node.  The terms come from node_fixed.cuh; its
+// tables are copied to shared memory, where random lookups cost a few bank
+// conflicts (through L1 up to a cycle per lane).
 //
 // Measured (forward + adjoint of one model): joint g_z + FTG, 64 x 64 x 32
-// cells, 1024 stations 8.4 ms, from 77.1 ms with the terms on the FP64 pipe;
+// cells, 1024 stations 8.2 ms, from 77.1 ms with the terms on the FP64 pipe;
 // g_z on 12 x 10 x 6 cells, 16 stations 13.7 us from 41 us.  A joint node takes
 // about 750 instructions; the schedulers issue in 68 % of the cycles, with the
 // integer, multiply-add and FP64 pipes 55 to 65 % busy each.
@@ -25,8 +27,6 @@ constexpr int kMaxColumn = 64;  // z offsets of a forward block held at a time
 constexpr int kAdjNodes = 8;    // nodes of a column per adjoint thread
 constexpr int kAdjStage = 16;   // stations staged at a time
 
-// The tables of node_fixed.cuh are copied to shared memory: random lookups
-// there cost a few bank conflicts, through L1 up to a cycle per lane.
 // rho~ of a node: the signed sum of the cells that it is a corner of, zero
 // outside, (-1)^(number of axes along which it is the upper corner), in the
 // column order of the forward: [k][column].  PLANES: the node planes of an axis
@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(kNodeThreads)
 // difference of its nodes).  What counts is where the constant changes along the
 // column, which is where dz changes its sign: those nodes add the change.  Two
 // FP64 operations of 13 less per node (the FP64 pipe was 81 % busy and led):
-// joint 8.74 -> 8.38 ms with g_z's dz multiplied in fixed point.
+// joint 8.74 -> 8.36 ms with g_z's dz multiplied in fixed point.
 template <int KIND>
 constexpr bool kLaplace = KIND == KIND_TENSOR || KIND == KIND_MAGNETIC || KIND == KIND_JOINT;
 

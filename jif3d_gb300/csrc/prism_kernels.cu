@@ -1,7 +1,9 @@
-// prism_kernels.cu -- FP64 matrix-free prism kernels for sm_103a.
+// prism_kernels.cu -- the matrix-free prism path around the node sums: background
+// layers, the ends of the forward and the adjoint, eight-corner rows.
 //
 // Work is organised around mesh NODES (see prism_math.cuh): for a station s
-// every node n carries the corner terms F_c(s, n).  Three uses:
+// every node n carries the corner terms F_c(s, n).  Three uses, the first two
+// summed in node_kernels.cu and the third in sens_kernels.cu:
 //   forward   U_c(s) = scale_c * sum_n F_c(s, n) * rho~(n)          (summation by parts)
 //   adjoint   G(n)   = sum_s sum_c W_c(s) F_c(s, n),  grad(cell) = 2 * D3[G](cell)
 //   J rows    T_c(s, cell) = eight-node sum in the reference's order

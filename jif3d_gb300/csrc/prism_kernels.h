@@ -1,4 +1,4 @@
-// prism_kernels.h -- launchers of the FP64 prism kernels (internal interface
+// prism_kernels.h -- launchers of the prism kernels (internal interface
 // between the C-ABI layer and the kernels; no CUDA types leak past capi.cu).
 #pragma once
 #include <cuda_runtime.h>

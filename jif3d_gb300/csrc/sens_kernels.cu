@@ -10,19 +10,22 @@
 //                  corners of the mesh
 //   k_split_tiles  FP64 rows -> hi + lo in the tiled layout and, through shared
 //                  memory, its transpose, in one pass
-// The terms stay in FP64 (node_terms) and the sums in the reference's order,
-// both bound by the FP64 pipe: the pair keeps 22 bits of entries whose own
-// FP64 rounding reaches 1e-8 in the far field, so that terms rounded in any
-// other way, better ones too, would move its last bits.
+// The terms keep their FP64 bits (node_terms) and the sums the reference's order:
+// the pair keeps 22 bits of entries whose own FP64 rounding reaches 1e-8 in the
+// far field, so that terms rounded in any other way, better ones too, would move
+// its last bits.  What of it integer arithmetic can do with the same bits is done
+// there (fp64_int.cuh), beside the FP64 pipe that bounds the two first kernels.
 //
 // Measured (joint g_z + FTG, 64 x 64 x 32 cells, 1024 stations, fp16 pair):
-// node terms 36 ms and cell rows 16 ms, both at the FP64 pipe's rate; the split
-// with its transpose 4.4 ms for 15 GB of traffic, from 20.6 ms as a split that
-// read the FP64 rows three times and two transposes.
+// node terms 21.5 ms (36 with FP64 instructions alone; FP64 pipe 84 % busy), cell
+// rows 10.9 ms (16; FP64 and integer pipes 78 %), the split with its transpose
+// 4.1 ms for 15 GB of traffic, from 20.6 ms as a split that read the FP64 rows
+// three times and two transposes.
 #include <cuda_fp16.h>
 
 #include <algorithm>
 
+#include "fp64_int.cuh"
 #include "fpbits.cuh"
 #include "prism_math.cuh"
 #include "prism_kernels.h"
