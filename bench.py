@@ -411,7 +411,7 @@ def measure_fp64_configs(stream, flush, local, cpu):
     FTG on 96 x 96 x 48 (2500 stations), and the total-field anomaly on
     128 x 128 x 64 over all 32 uneven station subsets (74,753 stations in one
     subsets forward and one subsets adjoint call; no warm-up, one call each,
-    a few seconds).  fp64_gflops: node evaluations x the FP64 flops that a node
+    4 s).  fp64_gflops: node evaluations x the FP64 flops that a node
     of the kind takes in FP64 instructions / time, beside the library's measured
     FP64 FMA rate and the nominal one (above them: most of it is integer work).
     Beside each, the oracle's OpenMP forward and LQDerivative
