@@ -157,12 +157,12 @@ __device__ __forceinline__ double zero_plus(double v) {
 // FP64 pipe, which bounds this kernel: each (row, z slot) costs one warp-wide
 // add, so KR > 0 unrolls the z run to exactly its longest length, the first
 // add of every sum (onto 0.0) and one of the second row's are done with integer
-// operations, and the loads of RB rows are issued before their adds.  KR = 0 runs
-// any length.  128 models of 64 x 64 x 32 cells from twice refined gradients 340
+// operations (with MORE two of every second row's, for runs of four), and the
+// loads of RB rows are issued before their adds.  KR = 0 runs any length.  128 models of 64 x 64 x 32 cells from twice refined gradients 340
 // -> 207 us (1.2 GB, 180 us): 300 with the first row's loads ahead of its adds
 // too, 240 without the FP64 comparison and the predicated add that the first
 // value had cost, 220 with code of their own for it at four blocks to an SM.
-template <int KR>
+template <int KR, bool MORE = false>
 __global__ void __launch_bounds__(kThreads, 4)
 k_refine_combine(RefineMaps m, int nmb, int nblock, int nextra, const double *__restrict__ fine,
                  double *__restrict__ coarse, long long cngrid, long long fngrid) {
@@ -230,7 +230,7 @@ k_refine_combine(RefineMaps m, int nmb, int nblock, int nextra, const double *__
                   if (u < nk) {
                     if (decltype(first)::value && r == 0 && u == 0)
                       sum = zero_plus(v[r][u]);
-                    else if (u == 1 && r == 1)
+                    else if (r == 1 && (u == 1 || (MORE && u == 3)))
                       sum = int_add(sum, v[r][u]);
                     else
                       sum += v[r][u];
@@ -298,8 +298,10 @@ cudaError_t launch_refine_combine(const RefineMaps &m, int nmodels, int nblock, 
     k_refine_combine<3><<<grid, kThreads, 0, st>>>(m, nmb, nblock, nextra, fine, coarse, cngrid,
                                                    fngrid);
   else if (zr <= 4)
-    k_refine_combine<4><<<grid, kThreads, 0, st>>>(m, nmb, nblock, nextra, fine, coarse, cngrid,
-                                                   fngrid);
+    // two integer sums of eight where there are two warps for every SM and more:
+    // 64 x 64 x 32 cells, 8 models 123 -> 110 us; a few hundred cells 8.1, not 8.6
+    (cngrid * nmb >= 152 * 64 ? k_refine_combine<4, true> : k_refine_combine<4, false>)
+        <<<grid, kThreads, 0, st>>>(m, nmb, nblock, nextra, fine, coarse, cngrid, fngrid);
   else
     k_refine_combine<0><<<grid, kThreads, 0, st>>>(m, nmb, nblock, nextra, fine, coarse, cngrid,
                                                    fngrid);

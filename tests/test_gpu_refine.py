@@ -325,8 +325,9 @@ def test_cpp_refiner(oracle_lib, tmp_path):
     assert exc
 
 
-@pytest.mark.parametrize("runs", [2, 3, 4])
-def test_combine_special_values(ctx, oracle_lib, runs):
+# 120 cells a model; from 152 x 64 on, runs of four take two integer sums
+@pytest.mark.parametrize("runs,nmodels", [(2, 6), (3, 6), (4, 6), (4, 81), (4, 82)])
+def test_combine_special_values(ctx, oracle_lib, runs, nmodels):
     """Sums with zeros of both signs, subnormals, the ends of the range,
     infinities, NaNs and cancellation in every place, bit for bit (a NaN as a
     NaN): one of a cell's sums is integer work and leaves these to the FP64 pipe."""
@@ -344,11 +345,12 @@ def test_combine_special_values(ctx, oracle_lib, runs):
     for i in range(1, 6):  # more and more of them
         take = rng.random(f.ngrid) < 0.1 * i
         G[i, take] = rng.choice(special[:6] if i < 3 else special, take.sum())
-    dG, dOut = torch.tensor(G, device="cuda"), torch.zeros((6, 120), dtype=torch.float64,
+    G = np.tile(G, (nmodels // 6 + 1, 1))[:nmodels]
+    dG, dOut = torch.tensor(G, device="cuda"), torch.zeros((nmodels, 120), dtype=torch.float64,
                                                            device="cuda")
-    ctx.refine_combine_device(6, dG.data_ptr(), dOut.data_ptr())
+    ctx.refine_combine_device(nmodels, dG.data_ptr(), dOut.data_ptr())
     ctx.synchronize()
-    for i in range(6):
+    for i in range(nmodels):
         out, ref = dOut[i].cpu().numpy(), oracle_combine(oracle_lib, s, f, G[i], 1, 0)
         nan = np.isnan(ref)
         assert np.array_equal(np.isnan(out), nan)
