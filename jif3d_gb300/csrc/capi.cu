@@ -712,11 +712,11 @@ int build_stored(j3g_context *c, int storage) {
     J3G_TRY(ensure(c, c->JTlo, bjt));
     J3G_TRY(ensure(c, c->rowscale, sizeof(float) * (size_t)R));
     J3G_TRY(ensure(c, c->Jrowsum, sizeof(double) * (size_t)R));
-    J3G_TRY(ensure(c, c->rowmax, 2 * sizeof(unsigned) * (size_t)R));
+    J3G_TRY(ensure(c, c->rowmax, sizeof(unsigned) * (size_t)R));
     J3G_TRY(ensure(c, c->rows, sizeof(double) * (size_t)chunk * NS * K));
     J3G_TRY(ensure(c, c->gerr, sizeof(int)));
     J3G_CUDA(c, cudaMemsetAsync(c->gerr.p, 0, sizeof(int), c->stream));
-    J3G_CUDA(c, cudaMemsetAsync(c->rowmax.p, 0, 2 * sizeof(unsigned) * (size_t)R, c->stream));
+    J3G_CUDA(c, cudaMemsetAsync(c->rowmax.p, 0, sizeof(unsigned) * (size_t)R, c->stream));
     const StoredPair p{c->Jhi.p, c->Jlo.p, c->JThi.p, c->JTlo.p, ldK, ldR,
                        ptr<float>(c->rowscale), ptr<double>(c->Jrowsum)};
     J3G_LAUNCH(c, launch_zero_padding(p, R, K, c->stream));

@@ -133,8 +133,8 @@ cudaError_t launch_stored_rows32(int kind, const MeshView &m, const StationView 
 // or as the fp16 pair (stored.h): row = scale * (hi + lo) with a power-of-two
 // scale, max|hi| in (2^13, 2^14], hi / lo with ld columns and the transpose thi /
 // tlo with ldt columns, both tiled, and the FP64 row sums J 1.  rows: scratch of
-// ns * stored rows * K doubles; rowmax: two zeroed words per row of the whole
-// matrix (largest high word, any NaN).  Columns beyond K are written as zero, the
+// ns * stored rows * K doubles; rowmax: a zeroed word per row of the whole matrix
+// (the largest high word).  Columns beyond K are written as zero, the
 // rest of the padding by launch_zero_padding.
 struct StoredPair {
   void *hi, *lo, *thi, *tlo;
