@@ -1930,9 +1930,12 @@ int j3g_set_refinement(j3g_context *c, int cnx, int cny, int cnz, const double *
     c->rm.fn[a] = fn[a];
     c->cn[a] = cn[a];
   }
-  c->rm.zrun_max = 0;
-  for (int k = 0; k < cnz; ++k)
-    c->rm.zrun_max = std::max(c->rm.zrun_max, h[off[2][2] + k] - h[off[2][1] + k]);
+  int longest[3] = {0, 0, 0};  // runs of refined cells of one coarse cell
+  for (int a = 0; a < 3; ++a)
+    for (int k = 0; k < cn[a]; ++k)
+      longest[a] = std::max(longest[a], h[off[a][2] + k] - h[off[a][1] + k]);
+  c->rm.zrun_max = longest[2];
+  c->rm.one_row = longest[0] <= 1 && longest[1] <= 1;
   c->refine_covers_all = all;
   c->refine_set = true;
   return J3G_OK;

@@ -162,11 +162,11 @@ __device__ __forceinline__ double zero_plus(double v) {
 // -> 207 us (1.2 GB, 180 us): 300 with the first row's loads ahead of its adds
 // too, 240 without the FP64 comparison and the predicated add that the first
 // value had cost, 220 with code of their own for it at four blocks to an SM.
-template <int KR, bool MORE = false>
+template <int KR, bool MORE = false, bool ONE_ROW = false>
 __global__ void __launch_bounds__(kThreads, 4)
 k_refine_combine(RefineMaps m, int nmb, int nblock, int nextra, const double *__restrict__ fine,
                  double *__restrict__ coarse, long long cngrid, long long fngrid) {
-  constexpr int RB = KR == 0 ? 1 : (KR <= 2 ? 4 : 2);
+  constexpr int RB = KR == 0 || ONE_ROW ? 1 : (KR <= 2 ? 4 : 2);
   constexpr int KU = KR == 0 ? 1 : KR;
   const long long ldc = nblock * cngrid + nextra, ldf = nblock * fngrid + nextra;
   const int lane = threadIdx.x & 31;
@@ -204,8 +204,24 @@ k_refine_combine(RefineMaps m, int nmb, int nblock, int nextra, const double *__
             }
             if (++j == nj) j = 0, ++i;
           }
-        } else if (KR == 1 && nr == 1) {  // a copy: 128 cells 2.24 us, not 2.40
-          if (nk > 0) sum = zero_plus(row00[k0]);
+        } else if (KR == 1) {
+          // one value a row: the first on its own, then four at a time (put into
+          // one phase with them as below, 41 -> 65 us for 32 models of 32 x 32 x 16
+          // cells from 4 x 4 rows each)
+          if (nr > 0 && nk > 0) sum = zero_plus(row00[k0]);
+          int i = nj == 1 ? 1 : 0, j = nj == 1 ? 0 : 1;
+          for (int r0 = 1; r0 < nr; r0 += RB) {
+            double v[RB];
+#pragma unroll
+            for (int r = 0; r < RB; ++r)
+              if (r0 + r < nr) {
+                if (nk > 0) v[r] = row00[i * rstride + (long long)j * fn2 + k0];
+                if (++j == nj) j = 0, ++i;
+              }
+#pragma unroll
+            for (int r = 0; r < RB; ++r)
+              if (r0 + r < nr && nk > 0) sum += v[r];
+          }
         } else if (nr > 0) {
           int i = 0, j = 0;
           // rows r0 .. r0 + RB - 1; the first value of all starts the sum (in
@@ -287,24 +303,26 @@ cudaError_t launch_refine_combine(const RefineMaps &m, int nmodels, int nblock, 
   if (nmb <= 0) return cudaSuccess;
   const long long crows = (long long)m.cn[0] * m.cn[1];
   const dim3 grid = grid_for((crows + kThreads / 32 - 1) / (kThreads / 32), nmb);
+  auto run = [&](auto kernel) {
+    kernel<<<grid, kThreads, 0, st>>>(m, nmb, nblock, nextra, fine, coarse, cngrid, fngrid);
+  };
   const int zr = m.zrun_max;
+  // one refined row to a coarse one: the slots of the other rows' predicated adds
+  // would count (32 x 32 x 16 cells from runs of two, 64 models 17 us, not 26)
   if (zr <= 1)
-    k_refine_combine<1><<<grid, kThreads, 0, st>>>(m, nmb, nblock, nextra, fine, coarse, cngrid,
-                                                   fngrid);
+    run(k_refine_combine<1>);
   else if (zr <= 2)
-    k_refine_combine<2><<<grid, kThreads, 0, st>>>(m, nmb, nblock, nextra, fine, coarse, cngrid,
-                                                   fngrid);
+    m.one_row ? run(k_refine_combine<2, false, true>) : run(k_refine_combine<2>);
   else if (zr <= 3)
-    k_refine_combine<3><<<grid, kThreads, 0, st>>>(m, nmb, nblock, nextra, fine, coarse, cngrid,
-                                                   fngrid);
+    m.one_row ? run(k_refine_combine<3, false, true>) : run(k_refine_combine<3>);
   else if (zr <= 4)
     // two integer sums of eight where there are two warps for every SM and more:
     // 64 x 64 x 32 cells, 8 models 123 -> 110 us; a few hundred cells 8.1, not 8.6
-    (cngrid * nmb >= 152 * 64 ? k_refine_combine<4, true> : k_refine_combine<4, false>)
-        <<<grid, kThreads, 0, st>>>(m, nmb, nblock, nextra, fine, coarse, cngrid, fngrid);
+    m.one_row                  ? run(k_refine_combine<4, false, true>)
+    : cngrid * nmb >= 152 * 64 ? run(k_refine_combine<4, true>)
+                               : run(k_refine_combine<4>);
   else
-    k_refine_combine<0><<<grid, kThreads, 0, st>>>(m, nmb, nblock, nextra, fine, coarse, cngrid,
-                                                   fngrid);
+    run(k_refine_combine<0>);
   return cudaGetLastError();
 }
 

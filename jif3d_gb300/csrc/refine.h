@@ -32,6 +32,7 @@ struct RefineMaps {
   int cn[3];            // coarse cells per axis
   int fn[3];            // refined cells per axis
   int zrun_max;         // longest z run of refined cells of one coarse cell
+  bool one_row;         // no coarse cell has more than one refined x or y cell
 };
 
 // ProjectValues (:124-168) for nmodels models of nblock cell blocks followed

@@ -326,8 +326,9 @@ def test_cpp_refiner(oracle_lib, tmp_path):
 
 
 # 120 cells a model; from 152 x 64 on, runs of four take two integer sums
-@pytest.mark.parametrize("runs,nmodels", [(2, 6), (3, 6), (4, 6), (4, 81), (4, 82)])
-def test_combine_special_values(ctx, oracle_lib, runs, nmodels):
+@pytest.mark.parametrize("across", [1, 2])  # refined cells along x and y of a coarse one
+@pytest.mark.parametrize("runs,nmodels", [(1, 6), (2, 6), (3, 6), (4, 6), (4, 81), (4, 82)])
+def test_combine_special_values(ctx, oracle_lib, runs, nmodels, across):
     """Sums with zeros of both signs, subnormals, the ends of the range,
     infinities, NaNs and cancellation in every place, bit for bit (a NaN as a
     NaN): one of a cell's sums is integer work and leaves these to the FP64 pipe."""
@@ -335,7 +336,7 @@ def test_combine_special_values(ctx, oracle_lib, runs, nmodels):
     s = small_survey(W.SCALAR, seed=63, nx=5, ny=4, nz=6, bg=False, origin=(0.0, 0.0, 0.0))
     s = dataclasses.replace(s, xsize=np.full(5, 12.0), ysize=np.full(4, 12.0),
                             zsize=np.full(6, 12.0), model=np.zeros(120))
-    f = refine(s, [np.arange(0.0, 61.0, 6.0), np.arange(0.0, 49.0, 6.0),
+    f = refine(s, [np.arange(0.0, 61.0, 12.0 / across), np.arange(0.0, 49.0, 12.0 / across),
                    np.arange(0.0, 73.0, 12.0 / runs)])
     fine_setup(ctx, s, f)
     rng = np.random.default_rng(64)
