@@ -559,31 +559,34 @@ __global__ void __launch_bounds__(G * kT, 2 / G)
 #pragma unroll 1
   for (int b = 0; b < 4 * most; ++b) {
     asm volatile("cp.async.wait_group %0;" ::"n"(R::kStages - 2) : "memory");
-    // stage b is there for both warps, and both have read stage b - 1
+    // stage b is there for both warps, and both have read stage b - 1.  The form
+    // that counts single threads: where the matrix's width leaves the lanes of a
+    // warp different numbers of chains, they need not arrive together
     if constexpr (G > 1)
-      asm volatile("bar.sync %0, %1;" ::"r"(1 + tid / 32), "n"(32 * G) : "memory");
+      asm volatile("barrier.cta.sync %0, %1;" ::"r"(1 + tid / 32), "n"(32 * G) : "memory");
     fetch(b + R::kStages - 1);  // into the stage that was read last
-    if (b >= 4 * nfull) continue;
-    const float4 *a = slot(b);
-    float4 xb[NM];
+    if (b < 4 * nfull) {
+      const float4 *a = slot(b);
+      float4 xb[NM];
 #pragma unroll
-    for (int m = 0; m < NM; ++m) xb[m] = a[(G * RB + m) * kT];
+      for (int m = 0; m < NM; ++m) xb[m] = a[(G * RB + m) * kT];
 #pragma unroll
-    for (int r = 0; r < RB; ++r) {
-      const float4 a0 = a[(g * RB + r) * kT];
+      for (int r = 0; r < RB; ++r) {
+        const float4 a0 = a[(g * RB + r) * kT];
 #pragma unroll
-      for (int m = 0; m < NM; ++m) {
-        // a chain starts with a product, as k_gemv_f32's
-        float s = b & 3 ? fmaf(a0.x, xb[m].x, acc[r][m]) : a0.x * xb[m].x;
-        s = fmaf(a0.y, xb[m].y, s); s = fmaf(a0.z, xb[m].z, s);
-        acc[r][m] = fmaf(a0.w, xb[m].w, s);
+        for (int m = 0; m < NM; ++m) {
+          // a chain starts with a product, as k_gemv_f32's
+          float s = b & 3 ? fmaf(a0.x, xb[m].x, acc[r][m]) : a0.x * xb[m].x;
+          s = fmaf(a0.y, xb[m].y, s); s = fmaf(a0.z, xb[m].z, s);
+          acc[r][m] = fmaf(a0.w, xb[m].w, s);
+        }
       }
-    }
-    if ((b & 3) == 3) {
+      if ((b & 3) == 3) {
 #pragma unroll
-      for (int r = 0; r < RB; ++r)
+        for (int r = 0; r < RB; ++r)
 #pragma unroll
-        for (int m = 0; m < NM; ++m) accd[r][m] += widen_f32(acc[r][m]);
+          for (int m = 0; m < NM; ++m) accd[r][m] += widen_f32(acc[r][m]);
+      }
     }
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");

@@ -609,3 +609,13 @@ def test_fp32_batches_two_groups(ctx, shape, nmeas):
     threads share a block: 1211, 1218 and 1225 rows leave the last block's groups
     three and none, two and none, one and none."""
     test_fp32_batches_share_a_pass(ctx, shape, nmeas)
+
+
+# 3136, 4032 and 7232 padded columns: float4 columns that end in the middle of a
+# warp within the last chain, so that half of its lanes have a chain more
+@pytest.mark.parametrize("shape", [(16, 14, 14), (18, 16, 14), (16, 15, 30)])
+@pytest.mark.parametrize("nmeas", [5, 173, 175])
+def test_fp32_batches_uneven_warps(ctx, shape, nmeas):
+    """The same where the lanes of a warp go through different numbers of whole
+    chains, with one group of threads to a block and with two."""
+    test_fp32_batches_share_a_pass(ctx, shape, nmeas)
