@@ -5,7 +5,7 @@ mpmath.
 * Logarithm -- for m in [1, 2) and j = floor((m - 1) 512): a 32-bit
   multiplier G_j = round(2^32 / (1 + (j + 1/2) / 512)), so that m G_j 2^-32 - 1
   is below 2^-9.99 in magnitude, and -log(G_j 2^-32) at scale 2^57.
-* Arctangent -- atan(j/512) at scale 2^61, j = 0..512.
+* Arctangent -- atan(j/1024) at scale 2^63, j = 0..1024.
 
 Run:  python jif3d_gb300/csrc/gen_node_tables.py   (rewrites node_tables.h)
 """
@@ -15,14 +15,14 @@ import mpmath as mp
 
 mp.mp.dps = 60
 HERE = os.path.dirname(os.path.abspath(__file__))
-LOG_N, ATAN_N, LOG_BIAS = 512, 512, 128
+LOG_N, ATAN_N, LOG_BIAS = 512, 1024, 128
 
 
 def main():
     ln2 = int(mp.floor(mp.log(2) * 2 ** 89))  # scale 2^57, 32 further bits
     G = [int(mp.nint(2 ** 32 / (1 + (mp.mpf(j) + 0.5) / LOG_N))) for j in range(LOG_N)]
     L = [int(mp.nint(-mp.log(mp.mpf(g) / 2 ** 32) * 2 ** 57)) for g in G]
-    A = [int(mp.nint(mp.atan(mp.mpf(j) / ATAN_N) * 2 ** 61)) for j in range(ATAN_N + 1)]
+    A = [int(mp.nint(mp.atan(mp.mpf(j) / ATAN_N) * 2 ** 63)) for j in range(ATAN_N + 1)]
 
     def rows(v, width, suffix):
         out = []
@@ -32,7 +32,7 @@ def main():
     lines = [
         "// node_tables.h -- generated by gen_node_tables.py; do not edit.",
         "// Tables of the fixed-point logarithm (multipliers G_j at scale 2^32 and",
-        "// -log G_j at scale 2^57) and arctangent (atan(j/512) at scale 2^61).",
+        "// -log G_j at scale 2^57) and arctangent (atan(j/1024) at scale 2^63).",
         "#pragma once",
         "#include <cstdint>",
         "",

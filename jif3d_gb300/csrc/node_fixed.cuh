@@ -20,9 +20,14 @@
 //             atan(bc / ar), atan(ac / br), atan(ab / cr) add up to pi/2 (the
 //             corner's solid angle), so the two smaller ones, both <= pi/4,
 //             are evaluated and the third is their complement.
-//             atan(N/D) = atan(j/512) + atan(d), d = (N - jD/512) / (D + jN/512),
-//             |d| <= 2^-10, by two digits of long division with a Newton
-//             reciprocal, atan d = d - d^3/3 + d^5/5
+//             atan(N/D) = atan(j/1024) + atan(d), d = (N - jD/1024) / (D + jN/1024),
+//             |d| <= 2^-11, by two digits of long division with a Newton
+//             reciprocal, atan d = d - d^3/3 + d^5/5; small angles keep a scale of
+//             their own, so that each has at least 53 bits.  (With 512 steps at
+//             scale 2^61 angles below 2^-9 were up to 13 units off in the last
+//             place, four on average, the cubic term's 32 bits being worth 2^-51 of
+//             them; 1024 steps at 2^63 and the term's shift after its product leave
+//             less than FP64's own error, for 4 KB more of tables.)
 //
 // Mantissas have their top bit at 2^62, so that the cross products of a 64 x 64
 // bit multiplication add up without a carry (three multiply-adds).
@@ -316,41 +321,43 @@ struct FxAngle {
 // atan(N / D) <= pi/4 for N = n1 2^-s, s >= 0, n1 in [2^60, 2^64) or 0, D in
 // [2^58, 2^61); t = N / D and idy = 2^88 / D as floats.
 J3G_FX FxAngle fx_atan(uint64_t n1, int s, uint64_t D, float t, float idy, const FxTables &T) {
-  // ratios below 2^-11 (j = 0) are scaled by 2^x into [2^-11, 2^-10), so that
+  // ratios below 2^-12 (j = 0) are scaled by 2^x into [2^-12, 2^-11), so that
   // small angles keep their leading bits
-  const int x = fx_max(116 - (int)(fx_bits(t) >> 23), 0);
+  const int x = fx_max(115 - (int)(fx_bits(t) >> 23), 0);
   s -= x;  // below 32
-  // N with 32 bits below its unit: (nh:nl:nx), and 2^9 N modulo 2^64
+  // N with 32 bits below its unit: (nh:nl:nx), and 2^10 N modulo 2^64
   const uint32_t nh = fx_hi(n1) >> (s & 31), nl = fx_funnel(fx_lo(n1), fx_hi(n1), s);
   const uint32_t nx = fx_funnel(0, fx_lo(n1), s);
-  const uint64_t n9 = fx_pair(fx_funnel(nl, nh, 23), fx_funnel(nx, nl, 23));
-  const uint64_t n7 = fx_pair(nh >> 7, fx_funnel(nl, nh, 7));
-  const float jf = fx_fmaf(t, 512.0f, 8388608.0f);  // the nearest integer in its low bits
+  const uint64_t n10 = fx_pair(fx_funnel(nl, nh, 22), fx_funnel(nx, nl, 22));
+  const uint64_t n8 = fx_pair(nh >> 8, fx_funnel(nl, nh, 8));
+  const float jf = fx_fmaf(t, 1024.0f, 8388608.0f);  // the nearest integer in its low bits
   uint32_t j = fx_bits(jf) - 0x4b000000u;
-  j = j < 512u ? j : 512u;
-  const int64_t num = (int64_t)(n9 - (uint64_t)j * D);             // |num| <= D / 2
-  const uint64_t den = D + ((uint64_t)j * n7 >> 2);                // below 2^62
-  const float ct = (jf - 8388608.0f) * (1.0f / 512.0f);
+  j = j < 1024u ? j : 1024u;
+  const int64_t num = (int64_t)(n10 - (uint64_t)j * D);            // |num| <= D / 2
+  const uint64_t den = D + ((uint64_t)j * n8 >> 2);                // below 2^62
+  const float ct = (jf - 8388608.0f) * (1.0f / 1024.0f);
   const int32_t y0 = (int32_t)fx_f2u(idy * fx_rcp(fx_fmaf(ct, t, 1.0f)));  // 2^88 / den
   const int64_t d = (int64_t)((1ull << 58) - (uint64_t)(uint32_t)(den >> 30) * (uint32_t)y0);
   const int32_t y = y0 + (int32_t)((int64_t)y0 * (int32_t)(d >> 10) >> 48);
   const int32_t q0 = fx_mulhi_s((int32_t)(num >> 30), y);  // 2^26 num / den
   const int64_t rem = (int64_t)(((uint64_t)num << 26) - (uint64_t)(int64_t)q0 * den);
-  // 2^56 rem / den, then 2^61 num / den = 2^70 d (scaled by 2^x)
+  // 2^56 rem / den, then 2^61 num / den = 2^71 d (scaled by 2^x)
   const int64_t q1 =
       (int64_t)(int32_t)(rem >> 32) * y + fx_mulhi(fx_lo((uint64_t)rem), (uint32_t)y);
   const int64_t q = (int64_t)((uint64_t)(int64_t)q0 << 35) + (q1 >> 21);
-  // d - d^3/3 + d^5/5 with d = 2^-9 dh 2^-31
-  const int32_t dh = (int32_t)(q >> 30);
-  const uint32_t d2 = (uint32_t)((uint64_t)((int64_t)dh * dh) >> 29);  // 2^33 (2^9 d)^2
-  const uint32_t c5 = fx_mulhi(d2, 858993459u) >> fx_min(19 + 2 * x, 31);
-  const uint32_t c = fx_mulhi(d2, 1431655765u - c5) >> fx_min(2 * x, 31);
-  const int64_t cube = (int64_t)dh * (int32_t)c;  // 2^91 (d^3/3 - d^5/5)
-  const int64_t small = q - (cube >> 21);         // scale 2^70 (2^x)
+  // d - d^3/3 + d^5/5 with d = 2^-10 dh 2^-31
+  const int32_t dh = (int32_t)((q + (1 << 29)) >> 30);  // to nearest: its error counts thrice
+  const uint32_t d2 = (uint32_t)((uint64_t)((int64_t)dh * dh) >> 29);  // 2^33 (2^10 d)^2
+  const uint32_t c5 = fx_mulhi(d2, 858993459u) >> fx_min(20 + 2 * x, 31);
+  const uint32_t c = fx_mulhi(d2, 2863311531u - c5);  // 2^54 d^2 (1/3 - d^2/5)
+  const int64_t cube = (int64_t)dh * (int32_t)c;      // 2^95 (d^3/3 - d^5/5), 2^x thrice
+  const int64_t small = q - (cube >> fx_min(24 + 2 * x, 63));  // scale 2^71 (2^x)
   FxAngle r;
-  r.v61 = T.atan[j] + (uint64_t)(x ? (int64_t)fx_shr((uint64_t)small, 9 + x) : small >> 9);
-  r.v = j ? r.v61 : (uint64_t)small;
-  r.scale = j ? 61 : 70 + x;
+  const uint64_t v63 =
+      T.atan[j] + (uint64_t)(x ? (int64_t)fx_shr((uint64_t)small, 8 + x) : small >> 8);
+  r.v61 = v63 >> 2;
+  r.v = j ? v63 : (uint64_t)small;
+  r.scale = j ? 63 : 71 + x;
   return r;
 }
 

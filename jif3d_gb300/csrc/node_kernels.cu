@@ -432,7 +432,7 @@ NodeAdjointPlan node_adjoint_plan(int nx, int ny, int nz, int nblock, int nmeas)
   // fewer blocks than four rounds: the split with the least of
   // (rounds + 0.9) * time of a block, as for the forward
   const int resident = std::min<long long>(
-      kNodeResident, (227 << 10) / ((25 << 10) + 8LL * nblock * p.kper * p.threads));
+      kNodeResident, (227 << 10) / ((29 << 10) + 8LL * nblock * p.kper * p.threads));
   if ((double)ncb * p.nkc * cdiv(nmeas, p.spc) < 4.0 * 152 * resident) {
     double best = 0.0;
     for (int spc : {16, 8, 6, 4, 3, 2, 1})
@@ -440,7 +440,7 @@ NodeAdjointPlan node_adjoint_plan(int nx, int ny, int nz, int nblock, int nmeas)
         const int kper = cdiv(nz1, n), nkc = cdiv(nz1, kper);
         if (kper > kAdjNodes) continue;
         const int fit = std::min<long long>(
-            kNodeResident, (227 << 10) / ((25 << 10) + 8LL * nblock * kper * p.threads));
+            kNodeResident, (227 << 10) / ((29 << 10) + 8LL * nblock * kper * p.threads));
         const double rounds = (double)ncb * nkc * cdiv(nmeas, spc) / (152.0 * fit);
         const double cost = (rounds + 0.9) * (6.0 + spc * (1.5 + kper));
         if (best != 0.0 && cost >= best) continue;
