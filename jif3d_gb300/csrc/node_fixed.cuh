@@ -363,33 +363,18 @@ J3G_FX FxAngle fx_atan(uint64_t n1, int s, uint64_t D, float t, float idy, const
 
 // atan2 from the angle of the magnitudes: `own` the sign of the abscissa's
 // offset, neg the sign of the ordinate.  Zero angles come from zero offsets.
-// CONVERT: by the conversion instruction.
-template <bool CONVERT = false>
 J3G_FX double fx_quadrant(uint64_t v, int scale, uint64_t v61, uint32_t own, uint32_t neg) {
   const uint64_t w = own ? nodetab::kPiS61 - v61 : v;
-  const double d = CONVERT ? fx_convert((int64_t)w, own ? 61 : scale, neg)
-                           : fx_to_double(w, own ? 61 : scale, neg);
+  const double d = fx_to_double(w, own ? 61 : scale, neg);
   return fx_hi(w) == 0 ? fx_double((uint64_t)neg << 63) : d;
-}
-
-// The sum of the three angles of a node whose dz has the sign negz: with s the
-// sign of dx dy dz and n negative offsets s pi (1/2 - n), as each atan2 is s
-// times its principal angle, less s pi where its abscissa is negative, and those
-// add up to pi / 2.  Above and below a column (dx = dy = 0) only Uzz's is not 0.
-J3G_FX double fx_angle_sum(const FxColumn &c, uint32_t negz) {
-  constexpr double kPi = 3.141592653589793238462643383279502884;
-  const double half = 0.5 - (double)(c.negx + c.negy + negz);
-  if (c.axial) return negz ? kPi : 0.0;
-  return (c.negx ^ c.negy ^ negz ? -kPi : kPi) * half;
 }
 
 // The node terms of MASK (component bits as node_terms) for the offsets of
 // column c and z.  In place of the g_z term out[0] is its angle atan2(dz r, dx dy)
 // (TIMES_DZ: times dz) and out[5], out[6] are ln(dy + r), ln(dx + r): g_z is
 // dx out[5] + dy out[6] + dz out[0], which the kernels fold into their weights
-// or sums.  Without ZZ out[3] is left out: it is fx_angle_sum less out[1] and
-// out[2].  False where the offsets are left to node_terms.
-template <int MASK, bool ZZ = true, bool TIMES_DZ = false>
+// or sums.  False where the offsets are left to node_terms.
+template <int MASK, bool TIMES_DZ = false>
 J3G_FX bool fx_node(const FxColumn &c, const FxAxis &z, const FxTables &T, double *out) {
   constexpr bool need_gz = (MASK & 1) != 0;
   constexpr bool need_xx = (MASK & 2) != 0, need_yy = (MASK & 4) != 0, need_zz = (MASK & 8) != 0;
@@ -409,9 +394,6 @@ J3G_FX bool fx_node(const FxColumn &c, const FxAxis &z, const FxTables &T, doubl
     l = l < kFxLogEps || (c.axial && z.neg) ? kFxLogEps : l;
     out[4] = fx_convert(l, 57, 0);
   }
-  // without g_z and Uzz the FP64 pipe has room for the angles' conversions
-  // (total-field anomaly 8.79 -> 8.65 ms; with them joint 8.22 -> 8.36)
-  constexpr bool kConvert = !need_gz && !ZZ;
   const uint64_t R4 = r.R << 2;
   uint64_t az = 0;  // the angle of z, scale 2^61
   if constexpr (need_xx || need_yy) {
@@ -430,19 +412,16 @@ J3G_FX bool fx_node(const FxColumn &c, const FxAxis &z, const FxTables &T, doubl
     const FxAngle aM = fx_atan(n2, eM - c.ehi + e0, D2, fr * c.fhi * fx_rcp(fM), imM * r.ys, T);
     const uint64_t am = c.axial ? 0 : nodetab::kPio2S61 - ah.v61 - aM.v61;  // the complement
     az = zbig ? aM.v61 : am;
-    const double Fh = fx_quadrant<kConvert>(ah.v, ah.scale, ah.v61, c.neghi, c.neglo ^ z.neg);
-    double Fl;
-    if constexpr (ZZ) {
-      const uint32_t negM = zbig ? z.neg : c.neglo, negm = zbig ? c.neglo : z.neg;
-      const double FM = fx_quadrant(aM.v, aM.scale, aM.v61, negM, c.neghi ^ negm);
-      const double Fm =
-          fx_convert((int64_t)(negm ? nodetab::kPiS61 - am : am), 61, c.neghi ^ negM);
-      Fl = zbig ? Fm : FM;
-      out[3] = zbig ? FM : Fm;
-    } else {
-      Fl = fx_quadrant<kConvert>(zbig ? am : aM.v, zbig ? 61 : aM.scale, zbig ? am : aM.v61,
-                                 c.neglo, c.neghi ^ z.neg);
-    }
+    // every angle from its own bits: Uzz as a constant less Uxx and Uyy would save
+    // a conversion, but keeps none of a small angle's leading bits (stations below
+    // the mesh) and adds up two roundings elsewhere
+    const uint32_t negM = zbig ? z.neg : c.neglo, negm = zbig ? c.neglo : z.neg;
+    const double Fh = fx_quadrant(ah.v, ah.scale, ah.v61, c.neghi, c.neglo ^ z.neg);
+    const double FM = fx_quadrant(aM.v, aM.scale, aM.v61, negM, c.neghi ^ negm);
+    const double Fm =
+        fx_convert((int64_t)(negm ? nodetab::kPiS61 - am : am), 61, c.neghi ^ negM);
+    const double Fl = zbig ? Fm : FM;
+    out[3] = zbig ? FM : Fm;
     out[1] = c.yhi ? Fl : Fh;
     out[2] = c.yhi ? Fh : Fl;
   } else if constexpr (need_zz || need_gz) {

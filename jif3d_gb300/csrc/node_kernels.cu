@@ -10,7 +10,7 @@
 // conflicts (through L1 up to a cycle per lane).
 //
 // Measured (forward + adjoint of one model): joint g_z + FTG, 64 x 64 x 32
-// cells, 1024 stations 8.2 ms, from 77.1 ms with the terms on the FP64 pipe;
+// cells, 1024 stations 8.6 ms, from 77.1 ms with the terms on the FP64 pipe;
 // g_z on 12 x 10 x 6 cells, 16 stations 13.7 us from 41 us.  A joint node takes
 // about 750 instructions; the schedulers issue in 68 % of the cycles, with the
 // integer, multiply-add and FP64 pipes 55 to 65 % busy each.
@@ -59,18 +59,6 @@ __global__ void __launch_bounds__(kNodeThreads)
   rt[n] = v;
 }
 
-// Uzz without its own angle (kinds with all three on one model block).  The three
-// angles of a node add up to a multiple of pi / 2 that only the offsets' signs
-// decide, so the sums of Uzz are those of Uxx and Uyy, negated, and of that
-// constant; and a constant along a column adds nothing to the data (the model
-// differences of a column add up to zero) nor to the gradient (a cell takes the
-// difference of its nodes).  What counts is where the constant changes along the
-// column, which is where dz changes its sign: those nodes add the change.  Two
-// FP64 operations of 13 less per node (the FP64 pipe was 81 % busy and led):
-// joint 8.74 -> 8.36 ms with g_z's dz multiplied in fixed point.
-template <int KIND>
-constexpr bool kLaplace = KIND == KIND_TENSOR || KIND == KIND_MAGNETIC || KIND == KIND_JOINT;
-
 // Forward partial sums: block x covers cols columns and kper nodes of each,
 // block y spb stations; partial[x][station][component].
 template <int KIND>
@@ -83,7 +71,6 @@ __global__ void __launch_bounds__(kNodeThreads, kNodeResident)
   constexpr int NZ = T::twin ? 2 : 1;
   // component 0 is g_z: dx ln(dy + r) + dy ln(dx + r) + dz atan2(dz r, dx dy)
   constexpr bool kGz = (MASK & (1 << NC_GZ)) != 0;
-  constexpr int kZz = kLaplace<KIND> ? NC_ZZ - T::comp(0) : 0;  // after Uxx and Uyy
   __shared__ FxTables tab;
   __shared__ ZOffset zo[NZ][kMaxColumn];
   __shared__ double red[NCMP][kNodeThreads];
@@ -113,8 +100,6 @@ __global__ void __launch_bounds__(kNodeThreads, kNodeResident)
         if constexpr (T::twin) zo[NZ - 1][k] = z_offset(add(mz, 1.0), Z);
       }
       __syncthreads();
-      // the sign of dz at the columns' first node (kLaplace)
-      const uint32_t ref = kLaplace<KIND> && mz < m.Z[0];
       for (int col = c0 + tid; col < c1; col += nt) {
         const int i = col / ny1, j = col - i * ny1;
         const double dx = sub(mx, m.X[i]), dy = sub(my, m.Y[j]);
@@ -130,23 +115,17 @@ __global__ void __launch_bounds__(kNodeThreads, kNodeResident)
           for (int p = 0; p < NZ; ++p) {
             const ZOffset &z = zo[p][k];
             double F[NC_COUNT];
-            if (fx_node<MASK, !kLaplace<KIND>, kGz>(c, z.a, tab, F)) {
+            if (fx_node<MASK, kGz>(c, z.a, tab, F)) {
               if constexpr (kGz) {
                 slx = fma(F[NC_YZ], w[0], slx);
                 sly = fma(F[NC_XZ], w[0], sly);
               }
-              if constexpr (kLaplace<KIND>)
-                if (z.a.neg != ref)
-                  acc[kZz] = fma(fx_angle_sum(c, z.a.neg) - fx_angle_sum(c, ref), w[0], acc[kZz]);
 #pragma unroll
               for (int q = 0; q < NCMP; ++q)
-                if (T::at(q) == p && !(kGz && (T::comp(q) == NC_XZ || T::comp(q) == NC_YZ)) &&
-                    !(kLaplace<KIND> && T::comp(q) == NC_ZZ))
+                if (T::at(q) == p && !(kGz && (T::comp(q) == NC_XZ || T::comp(q) == NC_YZ)))
                   acc[q] = fma(F[T::comp(q)], w[T::block(q)], acc[q]);
             } else {
               node_terms<MASK>(dx, dy, z.d, F);
-              if constexpr (kLaplace<KIND>)
-                F[NC_ZZ] += F[NC_XX] + F[NC_YY] - fx_angle_sum(c, ref);
 #pragma unroll
               for (int q = 0; q < NCMP; ++q)
                 if (T::at(q) == p) acc[q] = fma(F[T::comp(q)], w[T::block(q)], acc[q]);
@@ -162,7 +141,6 @@ __global__ void __launch_bounds__(kNodeThreads, kNodeResident)
         }
       }
     }
-    if constexpr (kLaplace<KIND>) acc[kZz] -= acc[kZz - 2] + acc[kZz - 1];
     // a warp per component sums the threads' values (13 FP64 additions a warp
     // and component instead of a shuffle tree in every warp)
 #pragma unroll
@@ -195,9 +173,7 @@ __global__ void __launch_bounds__(kNodeThreads, kNodeResident)
   constexpr int WLD = T::special ? NCMP : NC_COUNT;
   __shared__ FxTables tab;
   __shared__ ZOffset zo[NZ][kAdjStage][kAdjNodes];
-  constexpr int kZz = kLaplace<KIND> ? NC_ZZ - T::comp(0) : 0;  // after Uxx and Uyy
   __shared__ double sx[kAdjStage], sy[kAdjStage], sw[kAdjStage][NCMP];
-  __shared__ uint32_t ref[kAdjStage];  // the sign of dz at the columns' first node
   // g_z weight times dz (component 0 is g_z, see the forward)
   constexpr bool kGz = (MASK & (1 << NC_GZ)) != 0;
   __shared__ double swz[kGz ? kAdjStage : 1][kAdjNodes];
@@ -232,14 +208,10 @@ __global__ void __launch_bounds__(kNodeThreads, kNodeResident)
     for (int t = tid; t < cnt; t += nt) {
       sx[t] = st.x[base + t];
       sy[t] = st.y[base + t];
-      if constexpr (kLaplace<KIND>) ref[t] = st.z[base + t] < m.Z[0];
     }
     for (int t = tid; t < cnt * NCMP; t += nt) {
       const int s = t / NCMP, q = t - s * NCMP;
-      const double *w = W + (long long)(base + s) * WLD;
-      sw[s][q] = w[T::special ? q : T::comp(q)];
-      if constexpr (kLaplace<KIND>)
-        if (q == kZz - 2 || q == kZz - 1) sw[s][q] -= w[NC_ZZ];
+      sw[s][q] = W[(long long)(base + s) * WLD + (T::special ? q : T::comp(q))];
     }
     for (int t = tid; t < cnt * nk; t += nt) {
       const int s = t / nk, k = t - s * nk;
@@ -274,21 +246,15 @@ __global__ void __launch_bounds__(kNodeThreads, kNodeResident)
         for (int p = 0; p < NZ; ++p) {
           const ZOffset &z = zo[p][t][k];
           double F[NC_COUNT];
-          if (fx_node<MASK, !kLaplace<KIND>>(c, z.a, tab, F)) {
-            if constexpr (kLaplace<KIND>)
-              if (z.a.neg != ref[t])
-                v[0] = fma(sw[t][kZz], fx_angle_sum(c, z.a.neg) - fx_angle_sum(c, ref[t]), v[0]);
+          if (fx_node<MASK>(c, z.a, tab, F)) {
             if constexpr (kGz)
               v[0] = fma(swz[t][k], F[NC_GZ], fma(wly, F[NC_XZ], fma(wlx, F[NC_YZ], v[0])));
 #pragma unroll
             for (int q = 0; q < NCMP; ++q)
-              if (T::at(q) == p && !(kGz && (q == 0 || T::comp(q) == NC_XZ || T::comp(q) == NC_YZ)) &&
-                  !(kLaplace<KIND> && q == kZz))
+              if (T::at(q) == p && !(kGz && (q == 0 || T::comp(q) == NC_XZ || T::comp(q) == NC_YZ)))
                 v[T::block(q)] = fma(sw[t][q], F[T::comp(q)], v[T::block(q)]);
           } else {
             node_terms<MASK>(dx, dy, z.d, F);
-            if constexpr (kLaplace<KIND>)
-              F[NC_ZZ] += F[NC_XX] + F[NC_YY] - fx_angle_sum(c, ref[t]);
 #pragma unroll
             for (int q = 0; q < NCMP; ++q)
               if (T::at(q) == p)
