@@ -99,6 +99,10 @@ struct j3g_context {
   long long child_gen = -1;
   DevBuf chunks;  // chunk station ranges of a subset adjoint
   std::vector<int> chunks_h;  // the table now in chunks
+  // bytes that the adjoint's chunk sums may take, zero (one chunk at a time) for
+  // this mesh and survey where the memory for more could not be had
+  static constexpr long long kChunkRoom = 1LL << 30;
+  long long chunk_room = kChunkRoom;
   std::map<std::array<long long, 4>, GemmPlan> plans;
   GemmPlan last_plan[2];
 
@@ -490,27 +494,48 @@ int adjoint_device(j3g_context *c, const double *d_model, const double *d_misfit
                                       rawd, mag_field(c), ptr<double>(c->wraw), ptr<double>(c->W),
                                       c->stream));
     const long long nn = nodes.nnodes();
-    const NodeAdjointPlan plan =
-        node_adjoint_plan(nodes.nx, nodes.ny, nodes.nz, nblock, c->nmeas);
-    const int spc = plan.spc;
-    int nchunk = plan.nchunk;
-    // chunks of at most spc stations that never straddle a subset, and each
-    // subset's first chunk
+    const size_t chunk_bytes = sizeof(double) * (size_t)nblock * nn;
+    NodeAdjointPlan plan;
+    // chunks of at most spc stations that never straddle a subset (and the end of
+    // the last), then each subset's first chunk
     std::vector<int> table;
-    const int *d_starts = nullptr, *d_first = nullptr;
-    int most = nchunk;  // chunks of a subset
-    if (sub) {
+    int nchunk = 0, most = 0, held = 0;  // in all, of a subset, of a group of subsets
+    std::vector<int> group;  // subsets that are summed together: each group's first
+    auto lay_out = [&](long long room) {
+      plan = node_adjoint_plan(nodes.nx, nodes.ny, nodes.nz, nblock, c->nmeas, room);
+      const int fit = (int)std::max(1LL, std::min<long long>(1 << 30, room / (long long)chunk_bytes));
       std::vector<int> first;
-      most = 0;
+      table.clear();
+      group.assign(1, 0);
+      most = held = 0;
+      int begin = 0;  // the group's first chunk
       for (int k = 0; k < nsub; ++k) {
         first.push_back((int)table.size());
-        for (int a = off[k]; a < off[k + 1]; a += spc) table.push_back(a);
-        most = std::max(most, (int)table.size() - first.back());
+        for (int a = off[k]; a < off[k + 1]; a += plan.spc) table.push_back(a);
+        const int own = (int)table.size() - first.back();
+        most = std::max(most, own);
+        if ((int)table.size() - begin > fit && k > group.back()) {
+          group.push_back(k);
+          begin = first.back();
+        }
+        held = std::max(held, (int)table.size() - begin);
       }
       nchunk = (int)table.size();
       first.push_back(nchunk);
       table.push_back(c->nmeas);
       table.insert(table.end(), first.begin(), first.end());
+      group.push_back(nsub);
+    };
+    lay_out(c->chunk_room);
+    int rc = ensure(c, c->Gpart, chunk_bytes * std::max(held, 1));
+    if (rc == J3G_ERR_NOMEM && c->chunk_room > 0) {
+      c->chunk_room = 0;
+      lay_out(0);
+      rc = ensure(c, c->Gpart, chunk_bytes * std::max(held, 1));
+    }
+    J3G_TRY(rc);
+    const int *d_starts = nullptr, *d_first = nullptr;
+    if (sub) {
       // uploaded only when the subsets' chunk layout changes: a repeated call
       // on the same subsets queues kernels only (and can be graph-captured)
       if (table != c->chunks_h) {
@@ -523,16 +548,21 @@ int adjoint_device(j3g_context *c, const double *d_model, const double *d_misfit
       d_starts = ptr<int>(c->chunks);
       d_first = d_starts + nchunk + 1;
     }
-    J3G_TRY(ensure(c, c->Gpart, sizeof(double) * (size_t)std::max(nchunk, 1) * nblock * nn));
-    if (nchunk > 0) {
-      TimedScope ts(c, J3G_TIMER_NODE_ADJOINT);
-      J3G_LAUNCH(c, launch_node_adjoint(c->kind, nodes, s, ptr<double>(c->W), plan, nchunk, d_starts,
-                                        ptr<double>(c->Gpart), c->stream));
+    const int *first = table.data() + nchunk + 1;
+    for (size_t g = 0; g + 1 < group.size(); ++g) {
+      const int c0 = first[group[g]], c1 = first[group[g + 1]];
+      if (c1 > c0) {
+        TimedScope ts(c, J3G_TIMER_NODE_ADJOINT);
+        J3G_LAUNCH(c, launch_node_adjoint(c->kind, nodes, s, ptr<double>(c->W), plan, c1 - c0,
+                                          d_starts ? d_starts + c0 : nullptr,
+                                          ptr<double>(c->Gpart), c->stream));
+      }
+      int queued = 0;
+      J3G_CUDA(c, launch_adjoint_finish(m, nodes, node_planes(c), nblock, group[g], group[g + 1],
+                                        d_first, c0, most, nparm, ptr<double>(c->Gpart), d_grad,
+                                        c->stream, &queued));
+      c->launches += queued;
     }
-    int queued = 0;
-    J3G_CUDA(c, launch_adjoint_finish(m, nodes, node_planes(c), nblock, nsub, d_first, most, nparm,
-                                      ptr<double>(c->Gpart), d_grad, c->stream, &queued));
-    c->launches += queued;
   } else {
     J3G_LAUNCH(c, launch_backproject(c->kind, c->transform, tbx, tby, tbz, c->nmeas, d_misfit, rawd,
                                      ptr<double>(c->wraw), c->stream));
@@ -1277,6 +1307,7 @@ int j3g_set_mesh(j3g_context *c, int nx, int ny, int nz, const double *xc, const
   J3G_TRY(set_planes(c));
   J3G_CUDA(c, cudaStreamSynchronize(c->stream));
   c->mesh_set = true;
+  c->chunk_room = j3g_context::kChunkRoom;
   c->refine_set = false;  // the walks belong to the old mesh
   c->bg_dirty = true;
   drop_stored(c);  // the stored sensitivity belongs to the old geometry
@@ -1313,6 +1344,7 @@ int j3g_set_stations(j3g_context *c, int n, const double *x, const double *y, co
   c->hsy.swap(vy);
   c->hsz.swap(vz);
   c->stations_set = true;
+  c->chunk_room = j3g_context::kChunkRoom;
   c->bg_dirty = true;
   drop_stored(c);  // the stored sensitivity belongs to the old geometry
   ++c->gen;

@@ -381,7 +381,7 @@ cudaError_t launch_node_forward(int kind, const MeshView &m, const StationView &
                                                 rho_t, partial, p.cols, p.kper, p.nkc, p.spb));
 }
 
-NodeAdjointPlan node_adjoint_plan(int nx, int ny, int nz, int nblock, int nmeas) {
+NodeAdjointPlan node_adjoint_plan(int nx, int ny, int nz, int nblock, int nmeas, long long room) {
   NodeAdjointPlan p;
   const int ncol = (nx + 1) * (ny + 1), nz1 = nz + 1;
   p.threads = column_threads(ncol);
@@ -416,9 +416,9 @@ NodeAdjointPlan node_adjoint_plan(int nx, int ny, int nz, int nblock, int nmeas)
         p.nkc = nkc;
       }
   }
-  // the chunks' sums within 1 GB
-  const long long room = std::max(1LL, (1LL << 30) / (8LL * nblock * ncol * nz1));
-  p.spc = std::max<long long>(p.spc, (nmeas + room - 1) / room);
+  // the chunks' sums within the caller's room
+  const long long fit = std::max(1LL, room / (8LL * nblock * ncol * nz1));
+  p.spc = std::max<long long>(p.spc, (nmeas + fit - 1) / fit);
   p.nchunk = cdiv(nmeas, p.spc);
   return p;
 }

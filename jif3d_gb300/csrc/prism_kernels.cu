@@ -296,22 +296,22 @@ __global__ void __launch_bounds__(128)
 }
 
 // Chunks of the station subset blockIdx.z (all of them without a table).
-__device__ __forceinline__ int subset_chunks(const int *first_chunk, int sub, int nchunk,
-                                             int &first) {
-  first = first_chunk ? first_chunk[sub] : 0;
-  return first_chunk ? first_chunk[sub + 1] - first : nchunk;
+__device__ __forceinline__ int subset_chunks(const int *first_chunk, int sub, int chunk0,
+                                             int nchunk, int &first) {
+  first = first_chunk ? first_chunk[sub] - chunk0 : 0;
+  return first_chunk ? first_chunk[sub + 1] - first_chunk[sub] : nchunk;
 }
 
 // Groups of `group` chunks added up in place, each into its first chunk (block
 // y one group of every subset z): chunks in order, a few loads in flight.
 __global__ void __launch_bounds__(kThreads)
-    k_sum_groups(long long len, const int *__restrict__ first_chunk, int sub0, int nchunk,
-                 int group, double *__restrict__ Gpart) {
+    k_sum_groups(long long len, const int *__restrict__ first_chunk, int sub0, int chunk0,
+                 int nchunk, int group, double *__restrict__ Gpart) {
   chain_begin();
   chain_wait();
   const long long n = (long long)blockIdx.x * kThreads + threadIdx.x;
   int first;
-  const int nk = subset_chunks(first_chunk, sub0 + blockIdx.z, nchunk, first);
+  const int nk = subset_chunks(first_chunk, sub0 + blockIdx.z, chunk0, nchunk, first);
   const int c0 = blockIdx.y * group, c1 = min(nk, c0 + group);
   if (n >= len || c1 - c0 < 2) return;
   double *g = Gpart + (first + c0) * len + n;
@@ -331,7 +331,7 @@ constexpr int kTileX = 2, kTileY = 4, kTileZ = 16;  // cells of a block: 1.99 no
 template <bool PLANES>
 __global__ void __launch_bounds__(kThreads)
     k_adjoint_finish(MeshView m, MeshView nodes, NodePlanes p, const int *__restrict__ first_chunk,
-                     int sub0, int nchunk, int group, long long ld,
+                     int sub0, int chunk0, int nchunk, int group, long long ld,
                      const double *__restrict__ Gpart, double *__restrict__ grad) {
   // the cells of a tile lie on up to twice as many planes
   __shared__ double g[PLANES ? 8 * kTileX * kTileY * kTileZ
@@ -351,7 +351,7 @@ __global__ void __launch_bounds__(kThreads)
   }
   chain_wait();
   int first;
-  const int nk = subset_chunks(first_chunk, sub0 + blockIdx.z, nchunk, first);
+  const int nk = subset_chunks(first_chunk, sub0 + blockIdx.z, chunk0, nchunk, first);
   const long long all = nodes.nnodes(), len = all * gridDim.y;
   const double *part = Gpart + first * len + blockIdx.y * all;
   const int ny1 = nodes.ny + 1, nz1 = nodes.nz + 1;
@@ -579,9 +579,9 @@ cudaError_t launch_node_weights(int kind, int transform, double tbx, double tby,
 }
 
 cudaError_t launch_adjoint_finish(const MeshView &m, const MeshView &nodes,
-                                  const NodePlanes *planes, int nblock, int nsub,
-                                  const int *first_chunk, int nchunk, long long ld, double *Gpart,
-                                  double *grad, cudaStream_t st, int *launches) {
+                                  const NodePlanes *planes, int nblock, int sub0, int sub1,
+                                  const int *first_chunk, int chunk0, int nchunk, long long ld,
+                                  double *Gpart, double *grad, cudaStream_t st, int *launches) {
   // a thread of the last kernel adds up to 32 chunks one after the other; more
   // are first added up in groups, which are then spread over the GPU
   constexpr int kGroup = 32;
@@ -591,21 +591,22 @@ cudaError_t launch_adjoint_finish(const MeshView &m, const MeshView &nodes,
     for (group = kGroup; (long long)group * group < nchunk;) group *= 2;
   const int tiles = cdiv(m.nx, kTileX) * cdiv(m.ny, kTileY) * cdiv(m.nz, kTileZ);
   *launches = 0;
-  for (int s0 = 0; s0 < nsub; s0 += 65535) {  // grid z
-    const int ns = nsub - s0 < 65535 ? nsub - s0 : 65535;
+  for (int s0 = sub0; s0 < sub1; s0 += 65535) {  // grid z
+    const int ns = sub1 - s0 < 65535 ? sub1 - s0 : 65535;
     if (group > 1) {
       const cudaError_t e = launch_chained(
           k_sum_groups, dim3(cdiv(len, kThreads), cdiv(nchunk, group), ns), kThreads, 0, st, len,
-          first_chunk, s0, nchunk, group, Gpart);
+          first_chunk, s0, chunk0, nchunk, group, Gpart);
       if (e != cudaSuccess) return e;
       ++*launches;
     }
     const dim3 grid(tiles, nblock, ns);
     const cudaError_t e =
         planes ? launch_chained(k_adjoint_finish<true>, grid, kThreads, 0, st, m, nodes, *planes,
-                                first_chunk, s0, nchunk, group, ld, Gpart, grad)
+                                first_chunk, s0, chunk0, nchunk, group, ld, Gpart, grad)
                : launch_chained(k_adjoint_finish<false>, grid, kThreads, 0, st, m, nodes,
-                                NodePlanes{}, first_chunk, s0, nchunk, group, ld, Gpart, grad);
+                                NodePlanes{}, first_chunk, s0, chunk0, nchunk, group, ld, Gpart,
+                                grad);
     if (e != cudaSuccess) return e;
     ++*launches;
   }

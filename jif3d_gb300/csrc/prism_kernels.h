@@ -95,19 +95,20 @@ cudaError_t launch_node_weights(int kind, int transform, double t_bx, double t_b
 struct NodeAdjointPlan {
   int threads, kper, nkc, spc, nchunk;
 };
-NodeAdjointPlan node_adjoint_plan(int nx, int ny, int nz, int nblock, int nmeas);
+// room: bytes for the sums of all stations' chunks (one chunk at least).
+NodeAdjointPlan node_adjoint_plan(int nx, int ny, int nz, int nblock, int nmeas, long long room);
 cudaError_t launch_node_adjoint(int kind, const MeshView &m, const StationView &s,
                                 const double *W, const NodeAdjointPlan &p, int nchunk,
                                 const int *chunk_start, double *Gpart, cudaStream_t st);
 // grad[k * ld + b * ngrid + cell] = 2 * sum_corners (-1)^shifts * sum of
-// Gpart[chunk][b][node] over the chunks of subset k, for each model block b.
-// Subset k has the chunks first_chunk[k] to first_chunk[k + 1] - 1 (device, nsub
-// + 1 values), nchunk of them at most; null: one subset of nchunk chunks.  Gpart
-// is overwritten.  launches: kernels queued.
+// Gpart[chunk - chunk0][b][node] over the chunks of subset k, for each model block
+// b and the subsets sub0 to sub1 - 1.  Subset k has the chunks first_chunk[k] to
+// first_chunk[k + 1] - 1 (device), nchunk of them at most; null: one subset of nchunk
+// chunks.  Gpart is overwritten.  launches: kernels queued.
 cudaError_t launch_adjoint_finish(const MeshView &m, const MeshView &nodes,
-                                  const NodePlanes *planes, int nblock, int nsub,
-                                  const int *first_chunk, int nchunk, long long ld, double *Gpart,
-                                  double *grad, cudaStream_t st, int *launches);
+                                  const NodePlanes *planes, int nblock, int sub0, int sub1,
+                                  const int *first_chunk, int chunk0, int nchunk, long long ld,
+                                  double *Gpart, double *grad, cudaStream_t st, int *launches);
 // grad[ngrid + j] = 2 * sum_s sum_r w_raw[s][r] * bgsens[s][r][j]
 cudaError_t launch_background_grad(int kind, int nmeas, int nbg, const double *w_raw,
                                    const double *bgsens, double *grad_bg, cudaStream_t st);
