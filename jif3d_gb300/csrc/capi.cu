@@ -74,6 +74,7 @@ struct j3g_context {
   long long st_rows = 0;       // nmeas * stored rows per station
   long long st_ld = 0;         // cells padded to a multiple of 64
   long long st_ldT = 0;        // rows padded to a multiple of 64 (transposed copy)
+  int pass_models = kStreamModels;  // models per pass of the FP32 gradients
   DevBuf J32, Jhi, Jlo, JThi, JTlo, rowscale, Jrowsum, rowmax;
   DevBuf x32, sums, part, Bhi, Blo, P, wst, wrawb, rawb, gerr, mscale, mmean, swork, sexp;
 
@@ -709,6 +710,7 @@ int build_stored(j3g_context *c, int storage) {
     drop_memory(c);
     return fail(c, J3G_ERR_NOMEM, "sensitivity of " + std::to_string(need) + " bytes does not fit");
   }
+  c->pass_models = kStreamModels;
   c->st_rows = R;
   c->st_ld = ldK;
   c->st_ldT = ldR;
@@ -1095,11 +1097,18 @@ int batched_adjoint_pass(j3g_context *c, int nmod, const double *d_models,
                                         R, c->stream));
   }
   if (c->storage == J3G_STORE_FP32) {
-    J3G_TRY(ensure(c, c->part, sizeof(double) * (size_t)std::min(nmod, kStreamModels) *
-                                   gemv_t_chunks((int)R) * ldK));
-    for (int n = 0; n < nmod; n += kStreamModels) {
+    // kStreamModels models per pass over J, one where the memory that the
+    // chunks' sums of more take (a 64th of J's a model) could not be had
+    const size_t part = sizeof(double) * (size_t)gemv_t_chunks((int)R) * ldK;
+    int rc = ensure(c, c->part, part * std::min(nmod, c->pass_models));
+    if (rc == J3G_ERR_NOMEM && nmod > 1 && c->pass_models > 1) {
+      c->pass_models = 1;
+      rc = ensure(c, c->part, part);
+    }
+    J3G_TRY(rc);
+    for (int n = 0; n < nmod; n += c->pass_models) {
       J3G_LAUNCH(c, launch_gemv_t_f32(ptr<float>(c->J32), ldK, (int)R,
-                                      std::min(kStreamModels, nmod - n),
+                                      std::min(c->pass_models, nmod - n),
                                       ptr<double>(c->wst) + (size_t)n * R, R,
                                       ptr<double>(c->part), K, 2.0, d_grads + (size_t)n * np, np,
                                       c->stream));
