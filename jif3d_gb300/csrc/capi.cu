@@ -216,6 +216,12 @@ struct TimedScope {
   }
 };
 
+void free_buf(DevBuf &b) {
+  if (b.p) cudaFree(b.p);
+  b.p = nullptr;
+  b.cap = 0;
+}
+
 int ensure(j3g_context *c, DevBuf &b, size_t bytes) {
   if (bytes == 0) bytes = 8;
   if (b.cap >= bytes) return J3G_OK;
@@ -430,6 +436,16 @@ int gridded_rows_forward(j3g_context *c, const double *d_model, double *h_sens) 
   return J3G_OK;
 }
 
+// Node planes whose buffers do not fit in memory (rc from taking them): the mesh
+// goes back to eight-corner rows, a gigabyte for any mesh.
+bool planes_without_memory(j3g_context *c, int rc) {
+  if (rc != J3G_ERR_NOMEM || c->node_exact) return false;
+  c->node_path = false;
+  for (DevBuf *b : {&c->rhot, &c->partial, &c->Gpart}) free_buf(*b);
+  ++c->prod_gen;
+  return true;
+}
+
 // Forward with every buffer on the device.  raw_out (device, nmeas*raw) optional.
 int forward_device(j3g_context *c, const double *d_model, double *d_data, double *raw_out,
                    double *h_sens) {
@@ -441,8 +457,10 @@ int forward_device(j3g_context *c, const double *d_model, double *d_data, double
   const int nbg = c->nbg_active();
   const double *bgval = d_model + c->ngrid();
   const double *bgsens = nbg ? ptr<double>(c->bgsens) : nullptr;
-  if (c->ngrid() > 0 && c->node_path && !h_sens)
-    return node_forward(c, d_model, d_data, raw_out, bgsens, bgval);
+  if (c->ngrid() > 0 && c->node_path && !h_sens) {
+    const int rc = node_forward(c, d_model, d_data, raw_out, bgsens, bgval);
+    if (!planes_without_memory(c, rc)) return rc;
+  }
   // the gridded part from explicit sensitivities, or none
   if (h_sens || c->ngrid() > 0) {
     J3G_TRY(gridded_rows_forward(c, d_model, h_sens));
@@ -454,6 +472,53 @@ int forward_device(j3g_context *c, const double *d_model, double *d_data, double
                                 ptr<double>(c->rowsum), bgsens, nbg, bgval, raw_out, d_data,
                                 c->stream));
   return J3G_OK;
+}
+
+// The adjoint's station chunks: at most plan.spc stations each, never straddling a
+// subset.  table: the chunks' first stations and the end of the last, then each
+// subset's first chunk and the number of chunks.  Subsets are summed together in
+// groups (each group's first one, and the number of subsets) whose chunks fit the
+// room for their sums.
+struct AdjointChunks {
+  NodeAdjointPlan plan;
+  std::vector<int> table, group;
+  int nchunk, most;  // in all, of a subset
+};
+
+// The chunks of the subsets with the station offsets off, and memory for their sums.
+int adjoint_chunks(j3g_context *c, const std::vector<int> &off, AdjointChunks &ch) {
+  const MeshView nodes = node_view(c);
+  const int nblock = kind_nblock(c->kind), nsub = (int)off.size() - 1;
+  const size_t chunk_bytes = sizeof(double) * (size_t)nblock * nodes.nnodes();
+  auto lay_out = [&](long long room) {
+    ch.plan = node_adjoint_plan(nodes.nx, nodes.ny, nodes.nz, nblock, c->nmeas, room);
+    const int fit = (int)std::max(1LL, std::min<long long>(1 << 30, room / (long long)chunk_bytes));
+    std::vector<int> first;
+    ch.table.clear();
+    ch.group.assign(1, 0);
+    ch.most = 0;
+    int held = 1, begin = 0;  // chunks of the largest group, a group's first
+    for (int k = 0; k < nsub; ++k) {
+      first.push_back((int)ch.table.size());
+      for (int a = off[k]; a < off[k + 1]; a += ch.plan.spc) ch.table.push_back(a);
+      ch.most = std::max(ch.most, (int)ch.table.size() - first.back());
+      if ((int)ch.table.size() - begin > fit && k > ch.group.back()) {
+        ch.group.push_back(k);
+        begin = first.back();
+      }
+      held = std::max(held, (int)ch.table.size() - begin);
+    }
+    ch.nchunk = (int)ch.table.size();
+    first.push_back(ch.nchunk);
+    ch.table.push_back(c->nmeas);
+    ch.table.insert(ch.table.end(), first.begin(), first.end());
+    ch.group.push_back(nsub);
+    return ensure(c, c->Gpart, chunk_bytes * held);
+  };
+  const int rc = lay_out(c->chunk_room);
+  if (rc != J3G_ERR_NOMEM || c->chunk_room == 0) return rc;
+  c->chunk_room = 0;
+  return lay_out(0);
 }
 
 // Adjoint of all stations into d_grad, or, with sub (nsub + 1 station
@@ -488,70 +553,35 @@ int adjoint_device(j3g_context *c, const double *d_model, const double *d_misfit
   J3G_TRY(ensure(c, c->wraw, sizeof(double) * (size_t)c->nmeas * raw));
   MeshView m = mesh_view(c);
   StationView s = station_view(c);
+  AdjointChunks ch;
+  if (ngrid > 0 && c->node_path) {
+    const int rc = adjoint_chunks(c, off, ch);
+    if (!planes_without_memory(c, rc)) J3G_TRY(rc);
+  }
   if (ngrid > 0 && c->node_path) {
     const MeshView nodes = node_view(c);
     J3G_TRY(ensure(c, c->W, sizeof(double) * (size_t)c->nmeas * std::max<int>(NC_COUNT, kMaxVc)));
     J3G_LAUNCH(c, launch_node_weights(c->kind, c->transform, tbx, tby, tbz, c->nmeas, d_misfit,
                                       rawd, mag_field(c), ptr<double>(c->wraw), ptr<double>(c->W),
                                       c->stream));
-    const long long nn = nodes.nnodes();
-    const size_t chunk_bytes = sizeof(double) * (size_t)nblock * nn;
-    NodeAdjointPlan plan;
-    // chunks of at most spc stations that never straddle a subset (and the end of
-    // the last), then each subset's first chunk
-    std::vector<int> table;
-    int nchunk = 0, most = 0, held = 0;  // in all, of a subset, of a group of subsets
-    std::vector<int> group;  // subsets that are summed together: each group's first
-    auto lay_out = [&](long long room) {
-      plan = node_adjoint_plan(nodes.nx, nodes.ny, nodes.nz, nblock, c->nmeas, room);
-      const int fit = (int)std::max(1LL, std::min<long long>(1 << 30, room / (long long)chunk_bytes));
-      std::vector<int> first;
-      table.clear();
-      group.assign(1, 0);
-      most = held = 0;
-      int begin = 0;  // the group's first chunk
-      for (int k = 0; k < nsub; ++k) {
-        first.push_back((int)table.size());
-        for (int a = off[k]; a < off[k + 1]; a += plan.spc) table.push_back(a);
-        const int own = (int)table.size() - first.back();
-        most = std::max(most, own);
-        if ((int)table.size() - begin > fit && k > group.back()) {
-          group.push_back(k);
-          begin = first.back();
-        }
-        held = std::max(held, (int)table.size() - begin);
-      }
-      nchunk = (int)table.size();
-      first.push_back(nchunk);
-      table.push_back(c->nmeas);
-      table.insert(table.end(), first.begin(), first.end());
-      group.push_back(nsub);
-    };
-    lay_out(c->chunk_room);
-    int rc = ensure(c, c->Gpart, chunk_bytes * std::max(held, 1));
-    if (rc == J3G_ERR_NOMEM && c->chunk_room > 0) {
-      c->chunk_room = 0;
-      lay_out(0);
-      rc = ensure(c, c->Gpart, chunk_bytes * std::max(held, 1));
-    }
-    J3G_TRY(rc);
+    const NodeAdjointPlan &plan = ch.plan;
     const int *d_starts = nullptr, *d_first = nullptr;
     if (sub) {
       // uploaded only when the subsets' chunk layout changes: a repeated call
       // on the same subsets queues kernels only (and can be graph-captured)
-      if (table != c->chunks_h) {
-        J3G_TRY(ensure(c, c->chunks, sizeof(int) * table.size()));
-        J3G_CUDA(c, cudaMemcpyAsync(c->chunks.p, table.data(), sizeof(int) * table.size(),
+      if (ch.table != c->chunks_h) {
+        J3G_TRY(ensure(c, c->chunks, sizeof(int) * ch.table.size()));
+        J3G_CUDA(c, cudaMemcpyAsync(c->chunks.p, ch.table.data(), sizeof(int) * ch.table.size(),
                                     cudaMemcpyHostToDevice, c->stream));
         J3G_CUDA(c, cudaStreamSynchronize(c->stream));  // the host table is a local
-        c->chunks_h = table;
+        c->chunks_h = ch.table;
       }
       d_starts = ptr<int>(c->chunks);
-      d_first = d_starts + nchunk + 1;
+      d_first = d_starts + ch.nchunk + 1;
     }
-    const int *first = table.data() + nchunk + 1;
-    for (size_t g = 0; g + 1 < group.size(); ++g) {
-      const int c0 = first[group[g]], c1 = first[group[g + 1]];
+    const int *first = ch.table.data() + ch.nchunk + 1;
+    for (size_t g = 0; g + 1 < ch.group.size(); ++g) {
+      const int k0 = ch.group[g], k1 = ch.group[g + 1], c0 = first[k0], c1 = first[k1];
       if (c1 > c0) {
         TimedScope ts(c, J3G_TIMER_NODE_ADJOINT);
         J3G_LAUNCH(c, launch_node_adjoint(c->kind, nodes, s, ptr<double>(c->W), plan, c1 - c0,
@@ -559,9 +589,9 @@ int adjoint_device(j3g_context *c, const double *d_model, const double *d_misfit
                                           ptr<double>(c->Gpart), c->stream));
       }
       int queued = 0;
-      J3G_CUDA(c, launch_adjoint_finish(m, nodes, node_planes(c), nblock, group[g], group[g + 1],
-                                        d_first, c0, most, nparm, ptr<double>(c->Gpart), d_grad,
-                                        c->stream, &queued));
+      J3G_CUDA(c, launch_adjoint_finish(m, nodes, node_planes(c), nblock, k0, k1, d_first, c0,
+                                        ch.most, nparm, ptr<double>(c->Gpart), d_grad, c->stream,
+                                        &queued));
       c->launches += queued;
     }
   } else {
@@ -602,7 +632,9 @@ int adjoint_device(j3g_context *c, const double *d_model, const double *d_misfit
 // The node planes of a mesh whose corners are given one by one (NodePlanes):
 // the upper corner of cell i (corner + size, as the reference forms it) shares
 // the plane of the next cell's lower corner where the two are equal bit for bit.
-// Meshes of more than kMaxPlaneNodes plane nodes keep the eight-corner kernel.
+// Meshes of more than kMaxPlaneNodes plane nodes keep the eight-corner kernel, as
+// do those for whose plane nodes (2 GB a model block at the limit, for the model
+// differences and again for the sums of the gradient) there is no memory.
 constexpr long long kMaxPlaneNodes = 1LL << 28;
 int set_planes(j3g_context *c) {
   const int n[3] = {c->nx, c->ny, c->nz};
@@ -659,12 +691,6 @@ bool valid_kind(int k) { return k >= J3G_SCALAR && k <= J3G_MAGNETIZATION; }
 
 // ---------------------------------------------------------------------------
 // Device-resident sensitivity (the GPU side of FullSensitivityGravMagCalculator)
-
-void free_buf(DevBuf &b) {
-  if (b.p) cudaFree(b.p);
-  b.p = nullptr;
-  b.cap = 0;
-}
 
 void drop_memory(j3g_context *c) {
   for (DevBuf *b : {&c->J32, &c->Jhi, &c->Jlo, &c->JThi, &c->JTlo, &c->rowscale, &c->Jrowsum,

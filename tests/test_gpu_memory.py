@@ -112,3 +112,25 @@ def test_fp32_batch_with_little_memory():
     ctx.close()
     for g in got:
         assert np.array_equal(g, ref)
+
+
+def test_given_corners_with_little_memory(oracle_lib):
+    """142 x 142 x 142 cells, no corner shared, three model blocks: 0.55 GB of model
+    differences on the node planes and as much of chunk sums, 0.2 GB of eight-corner
+    rows for the one station where that cannot be had."""
+    n = 142
+    size = np.full(n, 20.0)
+    corner = 21.0 * np.arange(n)  # gaps of a metre
+    rng = np.random.default_rng(6)
+    s = W.Survey("gaps", size, size, size, (0.0, 0.0, 0.0), np.array([[1500.0, 1400.0, -30.0]]),
+                 W.MAGNETIZATION, rng.uniform(1, 11, 3 * n ** 3), bg_thick=np.zeros(0))
+    ctx = capi.Context(0)
+    W.setup_context(ctx, s)
+    ctx.set_mesh(corner, corner, corner, size, size, size)
+    p = oracle_lib.Problem(corner, corner, corner, size, size, size, s.stations, kind=s.kind)
+    misfit = rng.normal(size=3)
+    with _memory_left(GB * 45 // 100):
+        got = ctx.forward(s.model), ctx.lqderivative(s.model, misfit)
+    ctx.close()
+    assert relerr(got[0], p.forward(s.model)) <= 1e-10
+    assert relerr(got[1], p.lqderivative(s.model, misfit)) <= 1e-10
