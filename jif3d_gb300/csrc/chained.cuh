@@ -30,7 +30,9 @@ inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, int threads, 
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+  if (e != cudaSuccess) cudaGetLastError();  // returned here, not by the next launch's check
+  return e;
 }
 
 }  // namespace j3g
