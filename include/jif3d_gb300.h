@@ -392,9 +392,9 @@ int j3g_set_test_fault(j3g_context *ctx, int fault);
  *
  * Scratch is a fixed 16 MiB device array inside the library (held by every
  * GPU that loads the library until the process exits): the call allocates and
- * frees nothing.  It needs (nx+1)(ny+1)(nz+1) + 7*nmeas doubles plus at least
- * one block of nmeas*ncomp doubles (ncomp = 1 scalar, 6 tensor / magnetic,
- * 7 joint), all rounded up to 32 doubles, within 2^21 doubles; larger problems
+ * frees nothing.  It needs (nx+1)(ny+1)(nz+1) doubles, rounded up to 32, plus at
+ * least one block of nmeas*ncomp doubles (ncomp = 1 scalar, 6 tensor / magnetic,
+ * 7 joint) within 2^21 doubles; larger problems
  * return J3G_ERR_SCRATCH_LIMIT without touching d_data.  Every call shares
  * the array and leaves its last contents behind (each call writes all it
  * reads, nothing needs to start at zero), so calls that overlap on the GPU

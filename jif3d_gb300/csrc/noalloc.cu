@@ -83,13 +83,12 @@ extern "C" int j3g_forward_noalloc(int kind, int nx, int ny, int nz, const doubl
   if (nmeas > 0 && (!d_sx || !d_sy || !d_sz)) return J3G_ERR_ARG;
   if (nmeas == 0) return J3G_OK;
 
-  // scratch plan: rho~ (one value per node), per-station component sums,
-  // and the per-block partial sums of the node reduction
+  // scratch plan: rho~ (one value per node) and the per-block partial sums of the
+  // node reduction
   const long long nn = (long long)(nx + 1) * (ny + 1) * (nz + 1);
   const int ncomp = kind_ncomp(kind);
   const long long rho_len = round_up(nn);
-  const long long comps_len = round_up((long long)nmeas * NC_COUNT);
-  const long long left = kScratchDoubles - rho_len - comps_len;
+  const long long left = kScratchDoubles - rho_len;
   const long long per_block = (long long)nmeas * ncomp;
   if (left < per_block) return J3G_ERR_SCRATCH_LIMIT;
   const long long max_blocks = left / per_block;
@@ -103,8 +102,7 @@ extern "C" int j3g_forward_noalloc(int kind, int nx, int ny, int nz, const doubl
   int rc = scratch_for(device, st, &scratch);
   if (rc != J3G_OK) return rc;
   double *rho_t = scratch;
-  double *comps = scratch + rho_len;
-  double *partial = comps + comps_len;
+  double *partial = scratch + rho_len;
 
   MeshView m;
   m.nx = nx;
@@ -127,8 +125,8 @@ extern "C" int j3g_forward_noalloc(int kind, int nx, int ny, int nz, const doubl
   mf.factor = 1.0 / (4 * 3.141592653589793238462643383279502884 * kGravConst);
 
   // every scratch value read below is written first in the same call, so no
-  // clearing is needed: rho~ covers all nodes, the partials all (block,
-  // station, component) triples and the sums all (station, component) pairs
+  // clearing is needed: rho~ covers all nodes and the partials all (block,
+  // station, component) triples
   if (launch_rho_tilde(m, m, nullptr, 1, d_model, rho_t, st) != cudaSuccess) return J3G_ERR_CUDA;
   if (launch_node_forward(kind, m, s, rho_t, partial, plan, st) != cudaSuccess)
     return J3G_ERR_CUDA;
