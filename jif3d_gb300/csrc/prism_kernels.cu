@@ -414,9 +414,9 @@ __global__ void k_background_grad(int kind, int nmeas, int nbg, const double *__
 // raw_from_vc (BzSensBot - BzSensTop, OMPMagneticGradImp.cpp:88-99) and
 // magnetisation as factor * U_kj in row k, column block j
 // (OMPMagnetizationImp.cpp:58-68, 93-104).
-template <int KIND, class OutT = double>
+template <int KIND>
 __device__ __forceinline__ void store_cell_rows(const double *u, const MagField &mf,
-                                                long long ngrid, long long cell, OutT *rows,
+                                                long long ngrid, long long cell, double *rows,
                                                 long long ld) {
   using T = KindTraits<KIND>;
   if constexpr (KIND == KIND_MAGNETIZATION) {
@@ -424,11 +424,11 @@ __device__ __forceinline__ void store_cell_rows(const double *u, const MagField 
     for (int k = 0; k < 3; ++k)
 #pragma unroll
       for (int jb = 0; jb < 3; ++jb)
-        rows[(long long)k * ld + jb * ngrid + cell] = (OutT)mul(mf.factor, u[3 * k + jb]);
+        rows[(long long)k * ld + jb * ngrid + cell] = mul(mf.factor, u[3 * k + jb]);
   } else if constexpr (KIND == KIND_MAG_GRADIENT) {
     double raw[3];
     raw_from_vc(KIND, u, mf, raw);
-    rows[cell] = (OutT)raw[0];
+    rows[cell] = raw[0];
   } else {
     double c[NC_COUNT];
 #pragma unroll
@@ -436,7 +436,7 @@ __device__ __forceinline__ void store_cell_rows(const double *u, const MagField 
     double raw[10];
     raw_from_comps(KIND, c, mf, raw);
 #pragma unroll
-    for (int r = 0; r < T::raw; ++r) rows[(long long)r * ld + cell] = (OutT)raw[r];
+    for (int r = 0; r < T::raw; ++r) rows[(long long)r * ld + cell] = raw[r];
   }
 }
 
