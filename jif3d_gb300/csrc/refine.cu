@@ -158,10 +158,11 @@ __device__ __forceinline__ double zero_plus(double v) {
 // add, so KR > 0 unrolls the z run to exactly its longest length, the first
 // add of every sum (onto 0.0) and one of the second row's are done with integer
 // operations (with MORE two of every second row's, for runs of four), and the
-// loads of RB rows are issued before their adds.  KR = 0 runs any length.  128 models of 64 x 64 x 32 cells from twice refined gradients 340
-// -> 207 us (1.2 GB, 180 us): 300 with the first row's loads ahead of its adds
-// too, 240 without the FP64 comparison and the predicated add that the first
-// value had cost, 220 with code of their own for it at four blocks to an SM.
+// loads of RB rows are issued before their adds.  KR = 0 runs any length.  128
+// models of 64 x 64 x 32 cells from twice refined gradients 340 -> 207 us (1.2 GB,
+// 180 us): 300 with the first row's loads ahead of its adds too, 240 without the
+// FP64 comparison and the predicated add that the first value had cost, 220 with
+// code of their own for it at four blocks to an SM.
 template <int KR, bool MORE = false, bool ONE_ROW = false>
 __global__ void __launch_bounds__(kThreads, 4)
 k_refine_combine(RefineMaps m, int nmb, int nblock, int nextra, const double *__restrict__ fine,
@@ -316,11 +317,15 @@ cudaError_t launch_refine_combine(const RefineMaps &m, int nmodels, int nblock, 
   else if (zr <= 3)
     m.one_row ? run(k_refine_combine<3, false, true>) : run(k_refine_combine<3>);
   else if (zr <= 4)
-    // two integer sums of eight where there are two warps for every SM and more:
-    // 64 x 64 x 32 cells, 8 models 123 -> 110 us; a few hundred cells 8.1, not 8.6
-    m.one_row                  ? run(k_refine_combine<4, false, true>)
-    : cngrid * nmb >= 152 * 64 ? run(k_refine_combine<4, true>)
-                               : run(k_refine_combine<4>);
+    // two integer sums of eight from the warp (a coarse row of a model block) on
+    // that is the seventeenth on an SM, where the FP64 adds begin to queue: 16 rows
+    // to a coarse one, 8 x 8 coarse rows, 38 models 10.8 us (11.1 with two), 40
+    // models 13.9 (14.7 with one), 64 models 17.2 (19.3); 64 x 64 x 32 cells, 8
+    // models 110 (123); 4 rows to a coarse one the same within 2 % up to 24 warps,
+    // two rows 4 % the other way there
+    m.one_row                 ? run(k_refine_combine<4, false, true>)
+    : crows * nmb > 152 * 16  ? run(k_refine_combine<4, true>)
+                              : run(k_refine_combine<4>);
   else
     run(k_refine_combine<0>);
   return cudaGetLastError();

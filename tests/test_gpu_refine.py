@@ -356,3 +356,10 @@ def test_combine_special_values(ctx, oracle_lib, runs, nmodels, across):
         nan = np.isnan(ref)
         assert np.array_equal(np.isnan(out), nan)
         assert same_bits(np.where(nan, 0.0, out), np.where(nan, 0.0, ref))
+
+
+# 20 coarse rows a model: 2420 and 2440 warps, on both sides of the 152 x 16 from
+# which runs of four take two integer sums (the sizes of the test above are below)
+@pytest.mark.parametrize("nmodels", [121, 122])
+def test_combine_special_values_two_integer_sums(ctx, oracle_lib, nmodels):
+    test_combine_special_values(ctx, oracle_lib, 4, nmodels, 2)
