@@ -54,19 +54,20 @@ METRIC = "Mcell*station/s fwd+adjoint"
 UNIT = "Mcell*station/s"
 L2_FLUSH_BYTES = 512 << 20  # > 129 MB L2
 SIGMA_GZ, SIGMA_U = 1e-8, 1e-9
-# Nominal FP64 (non-tensor) rate of a GB300, for a second FP64 roofline
-# denominator beside the library's own measured FMA rate.
-FP64_NOMINAL_GFLOPS = 1250.0
-
 # FP64 flops per joint node evaluation in FP64 instructions (an FMA counts 2):
 # 21 add/mul + sqrt + 3 flog + 2 fatan2 + 1 fatan2_pair + 7 accumulation FMA,
 # with the weights of the device functions counted by ncu on microkernels of
 # each function (sqrt 13, flog 21, fatan2 36, fatan2_pair 42).  The node kernels
-# evaluate the terms in 64-bit fixed point on the integer pipes, so these rates
-# are FP64-equivalent ones, several times the FP64 pipe's, not a utilisation.
+# evaluate the terms in 64-bit fixed point on the integer pipes, so these give
+# FP64-equivalent rates, several times the FP64 pipe's, and no utilisation.
 FP64_FLOP_PER_JOINT_NODE = 225.0
 # the same of the other kinds, mean of forward and adjoint
 FP64_FLOP_PER_NODE = {1: 110.0, 2: 210.0, 3: 208.0, 4: FP64_FLOP_PER_JOINT_NODE}
+# What bounds the node kernels is the issue of instructions, one per scheduler and
+# cycle: warp instructions of a joint node, mean of forward (824) and adjoint (795),
+# counted by ncu (smsp__inst_executed over nodes x stations / 32)
+INSTR_PER_JOINT_NODE = 810.0
+SCHEDULERS = 152 * 4
 
 
 def parse():
@@ -411,9 +412,9 @@ def measure_fp64_configs(stream, flush, local, cpu):
     FTG on 96 x 96 x 48 (2500 stations), and the total-field anomaly on
     128 x 128 x 64 over all 32 uneven station subsets (74,753 stations in one
     subsets forward and one subsets adjoint call; no warm-up, one call each,
-    4 s).  fp64_gflops: node evaluations x the FP64 flops that a node
-    of the kind takes in FP64 instructions / time, beside the library's measured
-    FP64 FMA rate and the nominal one (above them: most of it is integer work).
+    4 s).  fp64_equivalent_gflops: node evaluations x the FP64 flops that a node
+    of the kind takes in FP64 instructions / time, and how many times the library's
+    measured FP64 FMA rate that is (no utilisation: most of it is integer work).
     Beside each, the oracle's OpenMP forward and LQDerivative
     on the host cores (all stations of the g_z survey, 64 seeded stations of
     the others)."""
@@ -463,8 +464,7 @@ def measure_fp64_configs(stream, flush, local, cpu):
              "forward_ms": t_f, "adjoint_ms": t_a,
              "value": pairs / (t * 1e-3), "forward": pairs / (t_f * 1e-3),
              "adjoint": pairs / (t_a * 1e-3), "unit": UNIT,
-             "fp64_gflops": gflops, "fp64_frac": gflops / peak,
-             "fp64_frac_of_nominal": gflops / FP64_NOMINAL_GFLOPS,
+             "fp64_equivalent_gflops": gflops, "times_fp64_pipe": gflops / peak,
              "flop_per_node": FP64_FLOP_PER_NODE[kind]}
         if full_batch:
             e["subsets"] = len(subs)
@@ -478,12 +478,11 @@ def measure_fp64_configs(stream, flush, local, cpu):
         out[s.name] = e
     out["fp64_peak_gflops"] = peak
     out["fp64_peak_source"] = ("j3g_probe_fp64: this library's FMA-chain probe kernel "
-                               "(no FP64 figure in MEASURED_PEAKS.json); fp64_frac_of_nominal "
-                               f"uses the nominal {FP64_NOMINAL_GFLOPS:.0f} GFLOP/s")
-    out["how"] = ("forward and adjoint of one model, each timed on its own; fp64_frac counts "
-                  "node evaluations only (the background, reductions and assembly are in the "
-                  "time), in FP64-equivalent flops: the kernels evaluate most of a node in "
-                  "fixed point, so it is above 1")
+                               "(no FP64 figure in MEASURED_PEAKS.json)")
+    out["how"] = ("forward and adjoint of one model, each timed on its own; "
+                  "fp64_equivalent_gflops counts node evaluations only (the background, "
+                  "reductions and assembly are in the time), at the FP64 flops that a node would "
+                  "take in FP64 instructions: the kernels evaluate most of it in fixed point")
     return out
 
 
@@ -893,10 +892,11 @@ def run_plain(args, rank, world, local):
     e2e = {"value": units * world * args.steps / e2e_s / 1e6, "unit": UNIT,
            "h2d_bytes_per_step": 8 * (2 * s.nparm + misfit_h.size),
            "d2h_bytes_per_step": 8 * (dh.size + gh.size)}
-    peak = ctx.probe_fp64()
     nodes = (s.shape[0] + 1) * (s.shape[1] + 1) * (s.shape[2] + 1)
     node_ms = (nf_ms + na_ms) / max(1, nf_n + na_n)
-    achieved = nodes * n * FP64_FLOP_PER_JOINT_NODE / (node_ms * 1e-3) / 1e9
+    per_s = nodes * n / (node_ms * 1e-3)
+    achieved = per_s / 32 * INSTR_PER_JOINT_NODE / 1e9
+    peak = SCHEDULERS * clk["sm_mhz"] * 1e-3 if clk["sm_mhz"] else None
     ctx.close()
     return {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
@@ -906,13 +906,13 @@ def run_plain(args, rank, world, local):
                    "models": 1, "l2": "flushed between timed steps (512 MiB write)",
                    "parallelism": f"replicas{world}"},
         "e2e": e2e, "gpu_launches": launches,
-        "roofline": {"bound": "fp64", "achieved": achieved, "peak": peak, "unit": "GFLOP/s",
-                     "frac": achieved / peak, "traffic": None,
+        "roofline": {"bound": "issue", "achieved": achieved, "peak": peak,
+                     "unit": "G warp instructions/s",
+                     "frac": achieved / peak if peak else None, "traffic": None,
                      "kernel": "k_node_forward<JOINT> / k_node_adjoint<JOINT>",
-                     "achieved_in": "FP64-equivalent flops (the node terms are evaluated in "
-                                    "fixed point on the integer pipes)",
-                     "peak_source": "measured FP64 FMA probe (MEASURED_PEAKS.json has no FP64 "
-                                    "entry)"},
+                     "fp64_equivalent_gflops": per_s * FP64_FLOP_PER_JOINT_NODE / 1e9,
+                     "peak_source": "one instruction per scheduler and cycle, 152 x 4 "
+                                    "schedulers, at the SM clock sampled under load"},
         "clocks": clk,
     }
 

@@ -12,8 +12,8 @@
 // Measured (forward + adjoint of one model): joint g_z + FTG, 64 x 64 x 32
 // cells, 1024 stations 8.6 ms, from 77.1 ms with the terms on the FP64 pipe;
 // g_z on 12 x 10 x 6 cells, 16 stations 13.7 us from 41 us.  A joint node takes
-// about 750 instructions; the schedulers issue in 68 % of the cycles, with the
-// integer, multiply-add and FP64 pipes 55 to 65 % busy each.
+// about 810 instructions; the schedulers issue in 67 % of the cycles, with the
+// integer, multiply-add and FP64 pipes 60 to 70 % busy each.
 #include <algorithm>
 
 #include "chained.cuh"
